@@ -127,6 +127,13 @@ bool make_layout(const fbp_dims* d, uint32_t flags, Layout* L)
         L->off_wkey = take(nw * 8);
         L->off_wpos = take(nw);
         L->off_wflag = take(nw * M);
+        const size_t spec = fft_spectra_bytes(dims_of(*L));
+        if (spec) {
+            L->off_spec = take(spec);
+            L->off_clist = take(M * C);
+            L->off_ccnt = take(M * 4);
+            L->off_tw = take(256 * 8);
+        }
     }
     if (!(flags & FBP_PLAIN_FP32) && (flags & FBP_OVERLAP_RECHECK)) {
         const uint64_t xt = M * M * S2 * S2 * 4;
@@ -141,6 +148,7 @@ bool make_layout(const fbp_dims* d, uint32_t flags, Layout* L)
             if (gb > L->nw) gb = L->nw;
             L->gbatch = gb;
             L->off_g = take(gb * per);
+            L->off_vc2 = take(gb * C * 4);              // the batch's window energies per channel
             L->off_order = take(gb * 4);                // screening order of a batch (by best label)
             L->off_perm = take(M * 4 + 8 + M * 8);      // order, then (8-aligned) non-zero channel masks
             L->off_mx = take(M * M * 4 + 2 * M * 4);   // max -X_ft per pair; max sqrt(E), max E per template
@@ -297,6 +305,7 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         if (ready.n == 0) FBP_TRY(launch_tc_update_voltage(d, w, voltage, nullptr, nullptr, 0, true, st));
     }
     if (lazy) FBP_CUDA(cudaMemsetAsync(w.base + lay.off_wflag, 0, lay.nw * lay.M, st));
+    if (!plain) FBP_TRY(launch_fft_templates(d, w, templates, st));
     if (!plain && overlap) FBP_TRY(launch_overlap_tables(d, w, templates, st));
     uint32_t nlist = d.nw, total = 0;
     api_detail::StageTimer tm;

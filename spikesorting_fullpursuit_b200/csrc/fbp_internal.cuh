@@ -107,10 +107,12 @@ struct Layout {
     // lazy exactness of the tensor-core likelihood: per-window maximum keys and
     // positive flags, and per (window, template) "row holds estimates" flags
     size_t off_wkey, off_wpos, off_wflag;
+    // transforms (corr_fft.cu): template spectra, channel lists and counts, twiddles
+    size_t off_spec, off_clist, off_ccnt, off_tw;
     // screened overlap recheck: truncated energies Et[M][S2] (f64), pair cross
     // terms XT[M][M][S2][S2] (f32), partial correlations G[gbatch][M][S2] (f32),
     // template processing order perm[M]
-    size_t off_et, off_xt, off_xtt, off_g, off_order, off_perm, off_mx, off_cand, off_bscr;
+    size_t off_et, off_xt, off_xtt, off_g, off_order, off_perm, off_mx, off_cand, off_bscr, off_vc2;
     uint64_t cand_cap;
     uint64_t gbatch;
     bool screened;
@@ -210,6 +212,13 @@ int launch_lazy_fix(const Dims& d, const Work& w, const float* V, const float* T
 int launch_tc_prepare_templates(const Dims& d, const Work& w, const float* T, cudaStream_t st);
 int launch_tc_update_voltage(const Dims& d, const Work& w, const float* V, const uint32_t* idx,
                              const uint32_t* win, uint32_t n, bool all, cudaStream_t st);
+
+// Correlations by transforms (corr_fft.cu)
+size_t fft_spectra_bytes(const Dims& d);        // 0: these sizes are not supported
+bool fft_windows_supported(const Dims& d);      // window correlations at every shift of the recheck
+int launch_fft_templates(const Dims& d, const Work& w, const float* T, cudaStream_t st);
+int launch_window_corr(const Dims& d, const Work& w, const float* V, const float* theta, const float2* Et,
+                       uint32_t k0, uint32_t kc, float* G, float* vc2, cudaStream_t st);
 
 // Screened overlap recheck (overlap_fast.cu)
 int launch_overlap_tables(const Dims& d, const Work& w, const float* T, cudaStream_t st);

@@ -19,7 +19,7 @@
 
 #include <vector>
 
-#include "fbp_internal.cuh"
+#include "fft256.cuh"
 
 namespace fbp {
 namespace {
@@ -380,7 +380,7 @@ struct ScreenShared {
 __host__ __device__ inline size_t screen_smem_bytes(uint32_t M, uint32_t S2, bool staged)
 {
     const size_t s2p = (S2 + 3) & ~3u, mp = (M + 3) & ~3u;
-    size_t b = 5 * s2p * 4 + 3 * mp * 4 + 256 * 4 + (size_t)kRowCap * 8 + (size_t)kCandCap * 12;
+    size_t b = 5 * s2p * 4 + 4 * mp * 4 + 256 * 4 + (size_t)kRowCap * 8 + (size_t)kCandCap * 12;
     b += (((size_t)S2 + 15) & ~(size_t)15) + (((size_t)M * S2 + 15) & ~(size_t)15);
     if (staged) b += (size_t)M * S2 * 8;
     return b + 64;
@@ -407,7 +407,11 @@ struct ScreenRow {
 // G_f(a) +- alpha(a), with alpha + beta = K (sqrt E_f(a) |v|_f + sqrt E_t(b) |v|_t +
 // E_f(a) + E_t(b)) the rigorous bound of |estimate - reference float value|
 // (|v|_x: the window's norm over template x's non-zero channels)
-// (K carries slack for the few float operations of this regrouping).  Phase B
+// (K carries slack for the few float operations of this regrouping).  Partial
+// correlations made by transforms (vc2 given: the windows' energies per channel)
+// are off by at most (64 + 3 n_x) u |T_x| |z|_x instead, z the pair of windows
+// transformed together (fft256.cuh): that is added once per template, and K keeps
+// the reference's own rounding only.  Phase B
 // bounds every row from shared-memory maxima (each component at least the
 // item's, same monotone float order) and keeps the rows that can reach the
 // window's seed; a quick lower bound from the best row of each warp prunes
@@ -422,7 +426,8 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
     const uint32_t* __restrict__ flag, DevStatus* status, const uint32_t* __restrict__ best_lab,
     const uint32_t* __restrict__ best_idx, const float* __restrict__ best_lik, unsigned long long* keys,
     const float* __restrict__ mx, unsigned long long* gcand, uint32_t gcand_cap,
-    const unsigned long long* __restrict__ chmask, float* bscratch, const uint32_t* __restrict__ order)
+    const unsigned long long* __restrict__ chmask, float* bscratch, const uint32_t* __restrict__ order,
+    const float* __restrict__ vc2)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ ScreenShared sh;
@@ -446,8 +451,9 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
     float* gmaxu = reinterpret_cast<float*>(alist + s2p);       // [M] max_b Bu[t][b]
     float* nx = gmaxu + mp;                                     // [M] max -X_ft over items
     float* nvt = nx + mp;                                       // [M] window norm over template t's channels
-    float* vc2 = nvt + mp;                                      // [C <= 256] window energy per channel
-    float* rowmax = vc2 + 256;                                  // [kRowCap]
+    float* mft = nvt + mp;                                      // [M] bound of the transforms' rounding
+    float* ve = mft + mp;                                       // [C <= 256] window energy per channel
+    float* rowmax = ve + 256;                                   // [kRowCap]
     uint32_t* rows = reinterpret_cast<uint32_t*>(rowmax + kRowCap);   // [kRowCap]
     uint32_t* cand = rows + kRowCap;                            // [kCandCap][3]
     uint8_t* fa = reinterpret_cast<uint8_t*>(cand + 3 * kCandCap);   // [S2] bit0 in bounds, bit1 L_f > 0
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
     uint32_t lbits = 0;
     while ((1u << lbits) < d.WG) ++lbits;
     const float u = 1.0f / 16777216.0f;
-    const float K = 1.01f * 1.05f * u * 2.0f * ((float)d.C * W + d.C + W + 24);
+    const float K = 1.01f * 1.05f * u * (vc2 ? 1.0f : 2.0f) * ((float)d.C * W + d.C + W + 32);
     const uint32_t nflag = status->n_flag;
     unsigned long long exact_n = 0, item_n = 0;
     for (uint32_t jo = blockIdx.x; jo < kcount; jo += gridDim.x) {
@@ -480,7 +486,10 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
         // per template, the norm of the window over that template's channels: a
         // template's products touch no other channel, so its part of the bound
         // (Cauchy-Schwarz over its support) needs no more
-        for (uint32_t c = warp; c < d.C; c += nwarps) {
+        const uint32_t kp = kk ^ 1u;   // the window transformed together with this one
+        const bool pair = vc2 != nullptr && kp < kcount && k0 + kp < nflag;
+        for (uint32_t c = threadIdx.x; vc2 != nullptr && c < d.C; c += blockDim.x) ve[c] = vc2[(size_t)kk * d.C + c];
+        for (uint32_t c = warp; vc2 == nullptr && c < d.C; c += nwarps) {
             float e2 = 0.f;
             for (uint32_t j = lane; j < W; j += 32) {
                 const float v = V[(uint64_t)c * d.N + p + j];
@@ -488,7 +497,7 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
             }
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, off);
-            if (lane == 0) vc2[c] = e2;
+            if (lane == 0) ve[c] = e2;
         }
         for (uint32_t x = threadIdx.x; x < S2; x += blockDim.x) {
             const uint64_t xp = (uint64_t)x + p;
@@ -505,17 +514,24 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
         __syncthreads();
         for (uint32_t t = threadIdx.x; t < M; t += blockDim.x) {
             const unsigned long long mt = chmask[t];   // all ones above 64 channels
-            float e2 = 0.f;
+            float e2 = 0.f, z2 = 0.f;
+            uint32_t n = 0;
             for (uint32_t c = 0; c < d.C; ++c)
-                if (c >= 64 || ((mt >> c) & 1ull)) e2 += vc2[c];
+                if (c >= 64 || ((mt >> c) & 1ull)) {
+                    e2 += ve[c];
+                    if (pair) z2 += vc2[(size_t)kp * d.C + c];
+                    ++n;
+                }
             nvt[t] = sqrtf(e2) * 1.001f;
+            mft[t] = vc2 == nullptr ? 0.f
+                                    : 1.05f * u * (kFftTerms + 3.f * n) * mx[(size_t)M * M + t] * sqrtf(e2 + z2) * 1.001f;
         }
         __syncthreads();
         const float nvf = nvt[f];
         float ma2 = -INFINITY;
         for (uint32_t x = threadIdx.x; x < S2; x += blockDim.x) {
             const float2 ea = Etab[(uint64_t)f * S2 + x];
-            const float al = K * fmaf(nvf, ea.y, ea.x);
+            const float al = fmaf(K, fmaf(nvf, ea.y, ea.x), mft[f]);
             const float g = Gk[(uint64_t)f * S2 + x];
             const uint8_t fl = fa[x];
             const float au = (fl & 1) ? g + al : -INFINITY, alo = (fl & 1) ? g - al : -INFINITY;
@@ -531,7 +547,7 @@ __global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
             const uint64_t xp = (uint64_t)x + p;
             const bool inb = xp >= S && xp < (uint64_t)d.N - W + S;
             const float2 eb = Etab[e];
-            const float be = K * fmaf(nvt[t], eb.y, eb.x);
+            const float be = fmaf(K, fmaf(nvt[t], eb.y, eb.x), mft[t]);
             const float g = Gk[e];
             Bu[e] = inb ? g + be : -INFINITY;
             Bl[e] = inb ? g - be : -INFINITY;
@@ -881,6 +897,14 @@ __global__ void __launch_bounds__(256) score_kernel(Dims d, const float* __restr
 
 }  // namespace
 
+// Whether a call's partial correlations are made by transforms: wherever they
+// apply (W + S <= 256 and the channels' spectra fit shared memory), unless the
+// caller asked for a template group of the direct kernel.  Measured against it,
+// per pursuit: 16 channels x 40 templates, 300 s 31.8 -> 6.0 ms; 64 x 200, 20 s
+// 38.8 -> 11.3 ms; 11 x 27 without zero channels, 43 s 2.3 -> 0.8 ms; 4 x 5, 5 s
+// 0.16 -> 0.08 ms.
+static bool window_corr_by_fft(const Dims& d) { return fft_windows_supported(d) && tuning().pc_group == 0; }
+
 struct PcConfig {
     int Q = 0;
     size_t smem = 0;
@@ -969,7 +993,9 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
     const PcConfig pc = pc_config();
     const int Q = pc.Q;
     const size_t smem_a = pc.smem;
-    if (Q == 0) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
+    const bool fft = window_corr_by_fft(d);
+    if (Q == 0 && !fft) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
+    float* vc2 = fft ? w.at<float>(L.off_vc2) : nullptr;
     const uint32_t pc_threads = 32u * std::min<uint32_t>((S2 + 15) / 16, kPcMaxWarps);
     const bool bstaged = (uint64_t)d.M * S2 * 8 <= kBStage;
     const size_t smem_b = screen_smem_bytes(d.M, S2, bstaged);
@@ -983,9 +1009,13 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
     const unsigned long long* chm = reinterpret_cast<const unsigned long long*>(perm + ((d.M + 1) & ~1u));
     for (uint32_t k0 = 0; k0 < nflag_max; k0 += (uint32_t)L.gbatch) {
         const uint32_t kc = (uint32_t)((nflag_max - k0) < L.gbatch ? (nflag_max - k0) : L.gbatch);
-        count_launch(3);
-        {
+        count_launch(2);
+        if (fft) {
         KScope ks(&fbp_chunk_stats::ms_partial_corr, st);
+        FBP_TRY(launch_window_corr(d, w, V, theta, Et, k0, kc, G, vc2, st));
+        } else {
+        KScope ks(&fbp_chunk_stats::ms_partial_corr, st);
+        count_launch();
         // persistent over the windows: as many CTAs as fit resident, split over the template groups
 #define FBP_PC(QQ)                                                                                            \
     case QQ: {                                                                                                \
@@ -1018,7 +1048,7 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
         screen_kernel<<<gb, kScrThreads, smem_b, st>>>(d, V, T, w.L(), theta, Et, XT, w.at<float>(L.off_xtt), G, k0, kc,
                                                        w.flag(), w.status(), w.best_lab(), w.best_idx(), w.best_lik(),
                                                        w.keys(), w.at<float>(L.off_mx), gcand, (uint32_t)L.cand_cap, chm,
-                                                       bstaged ? nullptr : w.at<float>(L.off_bscr), order);
+                                                       bstaged ? nullptr : w.at<float>(L.off_bscr), order, vc2);
         }
         KScope ks(&fbp_chunk_stats::ms_score, st);
         score_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, w.flag(), k0, w.best_lab(), w.best_idx(), gcand,

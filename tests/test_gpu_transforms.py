@@ -1,0 +1,54 @@
+"""Pursuits whose correlations are made by 256-point transforms, at the sizes where the
+transform kernels can go wrong, against the oracle: indices, labels, order and clips equal."""
+import copy
+
+import numpy as np
+import pytest
+
+import oracle
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from spikesorting_fullpursuit_b200 import binary_pursuit, synth  # noqa: E402
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+# (channels, units, sampling rate, clip window in samples before / after, shift range or None for W - 1)
+CASES = {
+    "one_channel_one_unit": (1, 1, 40000, 40, 60, None),
+    "odd_channels_and_units": (5, 9, 30000, 30, 45, None),
+    "half_shift": (7, 11, 30000, 30, 45, 37),
+    "no_shift": (3, 4, 30000, 30, 45, 0),
+    "shift_beyond_window": (3, 4, 20000, 10, 25, 50),
+    "longest_window": (4, 5, 40000, 50, 77, None),
+    "window_past_the_transform": (4, 5, 40000, 50, 78, None),
+    "short_window": (4, 6, 20000, 8, 11, None),
+    "seventeen_units": (16, 17, 30000, 20, 30, None),
+    "many_channels": (33, 8, 30000, 20, 30, None),
+    "more_channels_than_a_mask": (70, 4, 30000, 20, 30, None),
+}
+
+
+@pytest.mark.parametrize("recheck", [True, False])
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_pursuit_matches_oracle(case, recheck):
+    C, M, fs, before, after, S = CASES[case]
+    clip = (-(before + 0.25) / fs, (after - 0.25) / fs)
+    V, si, sm, _ = synth.make_recording(17 * len(case) + C, n_chans=C, fs=fs, duration_s=0.25, n_units=M,
+                                        rate_model=("uniform", 20.0, 60.0), overlap_frac=0.3, clip_width=clip)
+    W = si["n_samples_per_chan"]
+    si["get_adjusted_clips"] = True
+    si["do_overlap_recheck"] = recheck
+    S = W - 1 if S is None else S
+    want = oracle.binary_pursuit(V, np.float32, si, copy.deepcopy(sm), n_max_shift_inds=S,
+                                 global_mem_size=183 * 1024 ** 3)
+    got = binary_pursuit(V, np.float32, si, copy.deepcopy(sm), n_max_shift_inds=S, verbose=False)
+    assert len(want[0]) > 0
+    for g, w in zip(got, want):
+        assert np.array_equal(np.asarray(g), np.asarray(w)), (case, W, S)
