@@ -59,7 +59,7 @@ typedef struct fbp_chunk_stats {
     uint32_t n_spikes;       /* spikes written */
     uint64_t listed;         /* windows whose likelihood was (re)computed, summed over passes */
     uint64_t flagged;        /* windows given to the overlap recheck, summed over passes */
-    uint64_t fixups;         /* likelihood samples recomputed exactly after the tensor-core product
+    uint64_t fixups;         /* likelihood samples recomputed exactly after the fast likelihood
                                 (4 per queued run of consecutive samples) */
     uint64_t pair_exact;     /* overlap items whose pair likelihood was computed exactly */
     float ms_likelihood;     /* device time per stage, summed over passes (0 unless timing) */
@@ -69,7 +69,7 @@ typedef struct fbp_chunk_stats {
     float ms_residual;
     float ms_total;
     /* device time per kernel family, summed over passes (0 unless timing) */
-    float ms_lik_tc;         /* tensor-core likelihood */
+    float ms_lik_tc;         /* fast likelihood (by transforms, or on the tensor cores) */
     float ms_fixup;          /* exact recomputation of queued likelihood samples */
     float ms_lik_exact;      /* plain FP32 likelihood */
     float ms_partial_corr;   /* partial correlations of the screened recheck */
@@ -90,8 +90,11 @@ typedef struct fbp_chunk_stats {
 #define FBP_TIMING 0x4u
 
 /* Launch shapes of the tensor-core likelihood and of the screened recheck's
- * partial correlations; 0 leaves a choice to the library.  Values the sizes do
- * not allow (shared memory, TMEM) fall back to the library's choice. */
+ * direct partial correlations; 0 leaves a choice to the library, which makes both
+ * by transforms where the sizes allow (template_len <= 128, the channels' spectra
+ * fit shared memory): a value of lik_* asks for the tensor-core kernel instead,
+ * pc_group for the direct one.  Values the sizes do not allow (shared memory,
+ * TMEM) fall back to the library's choice. */
 typedef struct fbp_tuning {
     uint32_t lik_tiles;    /* 128-sample tiles per likelihood CTA: 1 to 4 */
     uint32_t lik_group;    /* (tap, channel pair) steps of templates per staged copy */

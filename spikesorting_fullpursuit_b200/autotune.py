@@ -1,13 +1,14 @@
 """Launch-shape autotuner for the pursuit, cached per chunk shape and device.
 
-The library picks its launch shapes from the sizes alone (include/fbp.h,
-fbp_tuning): 128-sample tiles per tensor-core likelihood CTA, template steps
-per staged copy, staged copies in flight, and templates per
-partial-correlation CTA.  ``tune`` measures candidates on the caller's own
-data -- a leading slice of the voltage with the real templates -- and keeps
-the fastest: first the likelihood shapes, by the likelihood kernel's device
-time within whole pursuits of the slice (the pass-by-pass window lists of a
-real pursuit), then the partial-correlation group, by whole pursuits.  Results are cached in a JSON file
+The library picks its kernels and launch shapes from the sizes alone
+(include/fbp.h, fbp_tuning): correlations by transforms where they apply; a
+caller's values ask for the tensor-core likelihood (128-sample tiles per CTA,
+template steps per staged copy, staged copies in flight) and the direct partial
+correlations (templates per CTA) instead.  ``tune`` measures the library's choice
+and these candidates on the caller's own data -- a leading slice of the voltage
+with the real templates -- and keeps the fastest: first the likelihood, by its
+stage's device time within whole pursuits of the slice (the pass-by-pass window
+lists of a real pursuit), then the partial-correlation group, by whole pursuits.  Results are cached in a JSON file
 (``FBP_TUNE_CACHE``, else ~/.cache/spikesorting_fullpursuit_b200/tuning.json)
 keyed by (channels, templates, window, shift, device name), so each shape is
 measured once.  Launch shapes change speed only: every candidate gives the
@@ -86,10 +87,12 @@ def _time(torch, fn, reps=3):
 
 
 def lik_candidates(M):
-    """Likelihood launch shapes to measure: the persistent kernel (lik_tiles 0)
-    with 1 to 4 epilogue warpgroups, then per-CTA tile counts."""
+    """Likelihood launch shapes to measure: the library's choice, the persistent
+    tensor-core kernel (lik_tiles 0) with 1 to 4 epilogue warpgroups, then per-CTA
+    tile counts."""
     Np = (M + 15) // 16 * 16
-    out = [{"lik_tiles": 0, "lik_epi": e, "lik_stages": st, "lik_group": 0, "pc_group": 0}
+    out = [dict.fromkeys(FIELDS, 0)]
+    out += [{"lik_tiles": 0, "lik_epi": e, "lik_stages": st, "lik_group": 0, "pc_group": 0}
            for e in (2, 3, 1, 4) for st in (0, 4)]
     tiles = tuple(k for k in (2, 4, 1) if k * Np <= 512)
     for lt in tiles:
@@ -150,7 +153,7 @@ def tune(voltage, templates, bias, theta, W, S, overlap=True, sample_s=None, sam
     try:
         for cand in lik_candidates(M):
             apply(cand)
-            ms = min(run_pursuit(True).ms_lik_tc for _ in range(2))
+            ms = min(run_pursuit(True).ms_likelihood for _ in range(2))
             if best_ms is None or ms < best_ms:
                 best, best_ms = dict(cand), ms
         if overlap:

@@ -6,6 +6,7 @@
 // and back every pass and compacts window lists with np.nonzero
 // (binary_pursuit_parallel.py:966-979, 1210-1251); here the lists are compacted
 // on the device and the host reads one 48-byte status word per pass.
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -133,6 +134,8 @@ bool make_layout(const fbp_dims* d, uint32_t flags, Layout* L)
             L->off_clist = take(M * C);
             L->off_ccnt = take(M * 4);
             L->off_tw = take(256 * 8);
+            L->off_lbnd = take(M * 8);
+            L->off_units = take(nw * 8);
         }
     }
     if (!(flags & FBP_PLAIN_FP32) && (flags & FBP_OVERLAP_RECHECK)) {
@@ -274,10 +277,11 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
     const bool plain = (flags & FBP_PLAIN_FP32) != 0;
     const bool overlap = (flags & FBP_OVERLAP_RECHECK) != 0;
     const bool timing = (flags & 0x4u) != 0;
-    const bool use_tc = !plain && tc_supported(dims_of(lay));
-    // tensor-core likelihood with lazy exactness: estimates kept where no
-    // decision needs the exact value (see lik_tc.cu)
-    const bool lazy = use_tc;
+    // fast likelihood (transforms, or tensor cores) with lazy exactness: estimates
+    // kept where no decision needs the exact value (see corr_fft.cu, lik_tc.cu)
+    const bool use_fft = !plain && fft_likelihood_chosen(dims_of(lay));
+    const bool use_tc = !plain && !use_fft && tc_supported(dims_of(lay));
+    const bool lazy = use_fft || use_tc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     fbp_chunk_stats local{};
     fbp_chunk_stats& S = stats ? *stats : local;
@@ -300,12 +304,12 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
     FBP_CUDA(cudaMemsetAsync(w.base + lay.off_best_lik, 0, lay.off_list - lay.off_best_lik, st));
     FBP_CUDA(cudaMemsetAsync(w.status(), 0, sizeof(DevStatus), st));
     FBP_TRY(launch_iota(w.list(), d.nw, st));
+    if (!plain) FBP_TRY(launch_fft_templates(d, w, templates, st));
     if (use_tc) {
         FBP_TRY(launch_tc_prepare_templates(d, w, templates, st));
         if (ready.n == 0) FBP_TRY(launch_tc_update_voltage(d, w, voltage, nullptr, nullptr, 0, true, st));
     }
     if (lazy) FBP_CUDA(cudaMemsetAsync(w.base + lay.off_wflag, 0, lay.nw * lay.M, st));
-    if (!plain) FBP_TRY(launch_fft_templates(d, w, templates, st));
     if (!plain && overlap) FBP_TRY(launch_overlap_tables(d, w, templates, st));
     uint32_t nlist = d.nw, total = 0;
     api_detail::StageTimer tm;
@@ -322,26 +326,36 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         FBP_CUDA(cudaMemsetAsync(&w.status()->chain_overflow, 0, 8, st));
         tm.start(timing, st, &S.ms_likelihood);
         if (pass == 1 && ready.n > 0) {
-            // first pass behind the upload: each arrived range is packed and the
-            // tiles whose strips it completes are pursued
+            // first pass behind the upload: of each arrived range, the spans (or
+            // tiles, their voltage packed first) it completes are pursued
             const uint64_t R8 = use_tc ? tc_tile_rows(d) : 0, ntile = (lay.N + 127) / 128;
-            uint64_t packed = 0, tdone = 0;
+            const uint64_t span = use_fft ? fft_span(d) : 0, halo = lay.W - 1;
+            uint64_t packed = 0, done = 0;
             for (uint32_t k = 0; k < ready.n; ++k) {
                 FBP_TRY(wait_ready(ready, k, st));
-                if (!use_tc) continue;
                 const bool last = k + 1 == ready.n;
-                const uint64_t r1 = last ? lay.vq_rows : ready.upto[k];
-                FBP_TRY(launch_tc_pack_range(d, w, voltage, packed, r1, st));
-                packed = r1;
-                const uint64_t tready = last ? ntile : (r1 >= R8 ? (r1 - R8) / 128 + 1 : 0);
-                if (tready > tdone) {
+                uint64_t upto = 0;
+                if (use_fft) {
+                    upto = last ? (lay.N + span - 1) / span
+                                : (ready.upto[k] >= halo ? (ready.upto[k] - halo) / span : 0);
+                    if (upto > done)
+                        FBP_TRY(launch_likelihood_fft(d, w, voltage, templates, bias, w.list(), nlist, w.L(), st,
+                                                      done, upto - done));
+                } else if (use_tc) {
+                    const uint64_t r1 = last ? lay.vq_rows : ready.upto[k];
+                    FBP_TRY(launch_tc_pack_range(d, w, voltage, packed, r1, st));
+                    packed = r1;
+                    upto = last ? ntile : (r1 >= R8 ? (r1 - R8) / 128 + 1 : 0);
                     uint64_t nfix = 0;
-                    FBP_TRY(launch_likelihood_tc(d, w, voltage, templates, bias, w.list(), nlist, w.L(), lazy, st,
-                                                 &nfix, tdone, tready - tdone));
-                    tdone = tready;
+                    if (upto > done)
+                        FBP_TRY(launch_likelihood_tc(d, w, voltage, templates, bias, w.list(), nlist, w.L(), lazy, st,
+                                                     &nfix, done, upto - done));
                 }
+                done = std::max(done, upto);
             }
-            if (!use_tc) FBP_TRY(launch_likelihood_exact(d, voltage, templates, bias, w.list(), nlist, w.L(), st));
+            if (!lazy) FBP_TRY(launch_likelihood_exact(d, voltage, templates, bias, w.list(), nlist, w.L(), st));
+        } else if (use_fft) {
+            FBP_TRY(launch_likelihood_fft(d, w, voltage, templates, bias, w.list(), nlist, w.L(), st));
         } else if (use_tc) {
             uint64_t nfix = 0;
             FBP_TRY(launch_likelihood_tc(d, w, voltage, templates, bias, w.list(), nlist, w.L(), lazy, st, &nfix));

@@ -84,6 +84,7 @@ struct DevStatus {
     uint32_t chain_overflow;// a prune/reassign chain was longer than the walk limit
     uint32_t error;         // nonzero: a kernel detected an inconsistent state
     uint32_t n_fix;         // runs of 4 likelihood samples queued for exact recomputation
+    uint32_t n_units;       // spans of listed windows the transform likelihood takes this pass
     uint32_t n_pair_exact;  // overlap items recomputed exactly
     uint32_t n_conf;        // spikes of this pass overlapping an earlier one
     unsigned long long pair_items;  // items evaluated by the overlap recheck
@@ -108,7 +109,7 @@ struct Layout {
     // positive flags, and per (window, template) "row holds estimates" flags
     size_t off_wkey, off_wpos, off_wflag;
     // transforms (corr_fft.cu): template spectra, channel lists and counts, twiddles
-    size_t off_spec, off_clist, off_ccnt, off_tw;
+    size_t off_spec, off_clist, off_ccnt, off_tw, off_lbnd, off_units;
     // screened overlap recheck: truncated energies Et[M][S2] (f64), pair cross
     // terms XT[M][M][S2][S2] (f32), partial correlations G[gbatch][M][S2] (f32),
     // template processing order perm[M]
@@ -203,6 +204,8 @@ int launch_likelihood_tc(const Dims& d, const Work& w, const float* V, const flo
 // Vq rows [r0, r1) from the voltage; the voltage rows a whole-chunk tile's strip reads
 int launch_tc_pack_range(const Dims& d, const Work& w, const float* V, uint64_t r0, uint64_t r1, cudaStream_t st);
 uint64_t tc_tile_rows(const Dims& d);
+int launch_fixup(const Dims& d, const Work& w, const float* V, const float* T, const float* bias, float* Lk, bool lazy,
+                 cudaStream_t st);
 // Lazy exactness: per-window argmax from the window keys, and the exact
 // recomputation of estimates whose voltage the coming residual changes in
 // windows the next pass does not relist.
@@ -216,9 +219,16 @@ int launch_tc_update_voltage(const Dims& d, const Work& w, const float* V, const
 // Correlations by transforms (corr_fft.cu)
 size_t fft_spectra_bytes(const Dims& d);        // 0: these sizes are not supported
 bool fft_windows_supported(const Dims& d);      // window correlations at every shift of the recheck
+bool fft_likelihood_chosen(const Dims& d);      // the likelihood of these sizes (and the caller's tuning)
 int launch_fft_templates(const Dims& d, const Work& w, const float* T, cudaStream_t st);
 int launch_window_corr(const Dims& d, const Work& w, const float* V, const float* theta, const float2* Et,
                        uint32_t k0, uint32_t kc, float* G, float* vc2, cudaStream_t st);
+// the pursuit's likelihood (lazy exactness); nlist == d.nw: the whole chunk, spans [span0, span0 + span_count) of fft_span(d) samples
+// each; span k reads the voltage up to sample (k + 1) * fft_span(d) + W - 2
+int launch_likelihood_fft(const Dims& d, const Work& w, const float* V, const float* T, const float* bias,
+                          const uint32_t* list, uint32_t nlist, float* L, cudaStream_t st, uint64_t span0 = 0,
+                          uint64_t span_count = ~0ull);
+uint64_t fft_span(const Dims& d);
 
 // Screened overlap recheck (overlap_fast.cu)
 int launch_overlap_tables(const Dims& d, const Work& w, const float* T, cudaStream_t st);

@@ -32,9 +32,9 @@ namespace fbp {
 constexpr uint32_t kFft = 256;          // transform length
 constexpr float kFftTerms = 64.f;       // rounding of a correlation: (kFftTerms + 3 n) u, see above
 
-// Template spectra: spec[t][c][m][l] = {X(k), X(k + 16)}, k = l + 32 m, X = DFT(T[t][c]) / 256
-// (the inverse transform's scale), complex as {re, im}; only the template's non-zero
-// channels clist[t][0 .. ccnt[t]) are written.
+// Template spectra, by the template's non-zero channels clist[t][0 .. ccnt[t]):
+// spec[t][i][m][l] = {X(k), X(k + 16)}, k = l + 32 m, X = DFT(T[t][clist[t][i]]) / 256 (the
+// inverse transform's scale), complex as {re, im}.
 struct FftTables {
     const float4* spec;       // [M][C][8][16]
     const uint8_t* clist;     // [M][C]
@@ -100,20 +100,25 @@ __device__ __forceinline__ void fft16(float2 (&x)[16])
 template <int SG>
 __device__ __forceinline__ void fft256(float2 (&x)[16], float2* buf, const float2* tw, uint32_t l)
 {
-    fft16<SG>(x);
+    // one copy of the 16-point transform in the code, run twice: unrolled, the kernels
+    // outgrow the instruction cache (a third of their stalls)
+#pragma unroll 1
+    for (int step = 0;; ++step) {
+        fft16<SG>(x);
+        if (step) return;
 #pragma unroll
-    for (uint32_t r = 0; r < 16; ++r) {
-        if (r) {
-            const float2 w = tw[r * 16 + l];
-            x[r] = c_mul(x[r], w.x, SG * w.y);
+        for (uint32_t r = 0; r < 16; ++r) {
+            if (r) {
+                const float2 w = tw[r * 16 + l];
+                x[r] = c_mul(x[r], w.x, SG * w.y);
+            }
+            buf[r * 16 + (l ^ r)] = x[r];
         }
-        buf[r * 16 + (l ^ r)] = x[r];
-    }
-    __syncwarp();
+        __syncwarp();
 #pragma unroll
-    for (uint32_t i = 0; i < 16; ++i) x[i] = buf[l * 16 + (i ^ l)];
-    __syncwarp();
-    fft16<SG>(x);
+        for (uint32_t i = 0; i < 16; ++i) x[i] = buf[l * 16 + (i ^ l)];
+        __syncwarp();
+    }
 }
 
 // Forward transform of channel data x (input order) into the channel's spectrum
@@ -125,33 +130,65 @@ __device__ __forceinline__ void fft_channel(float2 (&x)[16], float4* zs, const f
     for (uint32_t m = 0; m < 8; ++m) zs[m * 16 + l] = make_float4(x[2 * m].x, x[2 * m].y, x[2 * m + 1].x, x[2 * m + 1].y);
 }
 
-// Correlation of template t with the channel spectra zs[C][8][16] of the CTA's
-// signal pair, by a half-warp: x[q] = r_A[l + 16 q] + i r_B[l + 16 q].  A half-warp
-// without a template passes valid == false (it takes part in the exchange).
-__device__ __forceinline__ void fft_correlate(const FftTables& F, uint32_t C, uint32_t t, bool valid,
-                                              const float4* zs, float2* buf, const float2* tw, uint32_t l,
+// One template of a half-warp, as far as it is fetched ahead of its use: its channel
+// count, the channels of its first 16 list entries (entry l on lane l) and the first
+// half of its first spectrum.
+struct FftAhead {
+    uint32_t cnt, cl;
+    float4 T[4];
+};
+
+__device__ __forceinline__ void fft_fetch(const FftTables& F, uint32_t C, uint32_t t, bool valid, uint32_t l, FftAhead& A)
+{
+    A.cnt = valid ? __ldg(F.ccnt + t) : 0u;
+    A.cl = valid && l < C ? F.clist[(size_t)t * C + l] : 0u;
+    const float4* sp = F.spec + (size_t)t * C * 128 + l;
+#pragma unroll
+    for (int m = 0; m < 4; ++m) A.T[m] = valid ? __ldg(sp + m * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+__device__ __forceinline__ void fft_mac4(const float4 (&T)[4], const float4* zp, float2* x)
+{
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {   // x += conj(T) Z
+        const float4 Z = zp[m * 16];
+        x[2 * m].x = fmaf(T[m].x, Z.x, fmaf(T[m].y, Z.y, x[2 * m].x));
+        x[2 * m].y = fmaf(T[m].x, Z.y, fmaf(-T[m].y, Z.x, x[2 * m].y));
+        x[2 * m + 1].x = fmaf(T[m].z, Z.z, fmaf(T[m].w, Z.w, x[2 * m + 1].x));
+        x[2 * m + 1].y = fmaf(T[m].z, Z.w, fmaf(-T[m].w, Z.z, x[2 * m + 1].y));
+    }
+}
+
+// Correlation of template t (fetched ahead in A) with the channel spectra zs[C][8][16]
+// of the CTA's signal pair, by a half-warp: x[q] = r_A[l + 16 q] + i r_B[l + 16 q].  A
+// half-warp without a template has A.cnt == 0 (it takes part in the exchange).  The
+// spectra come from L2: each half spectrum is loaded while the one before it is
+// used, and template tn's first while t is transformed.
+__device__ __forceinline__ void fft_correlate(const FftTables& F, uint32_t C, uint32_t t, FftAhead& A, uint32_t tn,
+                                              bool next, const float4* zs, float2* buf, const float2* tw, uint32_t l,
                                               float2 (&x)[16])
 {
 #pragma unroll
     for (int m = 0; m < 16; ++m) x[m] = make_float2(0.f, 0.f);
-    const uint32_t cnt = valid ? F.ccnt[t] : 0u;
-    const uint8_t* cl = F.clist + (size_t)t * C;
+    const uint32_t cnt = A.cnt, half = 0xFFFFu << (threadIdx.x & 16u);
     const float4* sp = F.spec + (size_t)t * C * 128 + l;
+    const float4* zl = zs + l;
     for (uint32_t i = 0; i < cnt; ++i) {
-        const uint32_t c = cl[i];
-        const float4* tp = sp + (size_t)c * 128;
-        const float4* zp = zs + (size_t)c * 128 + l;
+        if ((i & 15u) == 0u && i) A.cl = i + l < C ? F.clist[(size_t)t * C + i + l] : 0u;
+        const float4* zp = zl + __shfl_sync(half, A.cl, i & 15u, 16) * 128;
+        float4 B[4];
 #pragma unroll
-        for (int m = 0; m < 8; ++m) {
-            const float4 T = __ldg(tp + m * 16);
-            const float4 Z = zp[m * 16];
-            x[2 * m].x = fmaf(T.x, Z.x, fmaf(T.y, Z.y, x[2 * m].x));       // conj(T) Z
-            x[2 * m].y = fmaf(T.x, Z.y, fmaf(-T.y, Z.x, x[2 * m].y));
-            x[2 * m + 1].x = fmaf(T.z, Z.z, fmaf(T.w, Z.w, x[2 * m + 1].x));
-            x[2 * m + 1].y = fmaf(T.z, Z.w, fmaf(-T.w, Z.z, x[2 * m + 1].y));
+        for (int m = 0; m < 4; ++m) B[m] = __ldg(sp + 64 + m * 16);
+        fft_mac4(A.T, zp, x);
+        sp += 128;
+        if (i + 1 < cnt) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) A.T[m] = __ldg(sp + m * 16);
         }
+        fft_mac4(B, zp + 64, x + 8);
     }
     __syncwarp();
+    fft_fetch(F, C, next ? tn : 0u, next, l, A);
     fft256<1>(x, buf, tw, l);
 }
 

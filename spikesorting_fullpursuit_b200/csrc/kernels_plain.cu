@@ -13,7 +13,7 @@
 //   * spike output: window-list order; residual: list order for overlaps.
 #include <cub/cub.cuh>
 
-#include "fbp_internal.cuh"
+#include "lik_common.cuh"
 
 namespace fbp {
 namespace {
@@ -480,32 +480,6 @@ __global__ void __launch_bounds__(kOvThreads) overlap_plain_kernel(
 // parse_overlap_recheck_indices (binary_pursuit.cl:657-815), one thread per
 // flagged window, from the winner key.
 // ---------------------------------------------------------------------------
-// Exact likelihood of (t, s) in the reference order (compute_maximum_likelihood,
-// binary_pursuit.cl:216-252) from the current voltage, by a whole warp: each
-// lane forms the products of 32 taps at a time (each product rounds the same
-// wherever it is formed), and every lane adds them in tap order, so all lanes
-// end with the reference's sum.  Channels where the template is entirely zero
-// add 0 * v terms in the reference, which leave a nonzero sum unchanged.
-__device__ float warp_exact_lik(const Dims& d, const float* __restrict__ V, const float* __restrict__ T, float b,
-                                uint32_t t, uint32_t s, const float* __restrict__ tnorm)
-{
-    const uint32_t lane = threadIdx.x & 31;
-    float acc = b;
-    for (uint32_t c = 0; c < d.C; ++c) {
-        if (tnorm[(uint64_t)t * d.C + c] == 0.f) continue;
-        const float* tr = T + ((uint64_t)t * d.C + c) * d.W;
-        const float* vr = V + (uint64_t)c * d.N + s;
-        for (uint32_t j0 = 0; j0 < d.W; j0 += 32) {
-            const uint32_t j = j0 + lane;
-            const float p = j < d.W ? fmul(__ldg(tr + j), vr[j]) : 0.f;
-            const uint32_t n = d.W - j0 < 32u ? d.W - j0 : 32u;
-#pragma unroll 8
-            for (uint32_t k = 0; k < n; ++k) acc = fadd(acc, __shfl_sync(0xffffffffu, p, k));
-        }
-    }
-    return acc;
-}
-
 // L[t][s], made exact where the tensor-core likelihood may have left an estimate
 // (a positive value in a flagged window row; the window's voltage is unchanged
 // since it was computed, so the current voltage gives the exact value).  Called

@@ -34,7 +34,7 @@
 
 #include <algorithm>
 
-#include "fbp_internal.cuh"
+#include "lik_common.cuh"
 
 namespace fbp {
 namespace {
@@ -208,32 +208,6 @@ struct TcParams {
     uint8_t* wflag;             // [nw][M] 1: the window's row of template t holds estimates
     uint32_t wslots;            // win_slots(W): window slots per tile in shared memory
 };
-
-// Key of a positive likelihood v at (template t, sample s) of window w:
-// larger for a larger value, then for a smaller t, then for a smaller s -- the
-// order in which compute_template_maximum_likelihood (binary_pursuit.cl:395-408)
-// keeps the first maximum.  Needs W <= 1024 and t < 2^22.
-__device__ __forceinline__ unsigned long long window_key(float v, uint32_t t, uint32_t local_s)
-{
-    return ((unsigned long long)__float_as_uint(v) << 32) | (unsigned long long)(0xFFFFFFFFu - ((t << 10) | local_s));
-}
-
-// The reference's sum, skipping template channels that are entirely zero
-// (tnorm == 0): there it adds 0 * v terms, which leave a nonzero sum unchanged
-// (and a zero sum zero, up to the sign of zero, which no decision reads).
-__device__ float exact_likelihood(const Dims& d, const float* __restrict__ V, const float* __restrict__ T,
-                                  float b, uint32_t t, uint32_t s, const float* __restrict__ tnorm)
-{
-    float acc = b;
-    for (uint32_t c = 0; c < d.C; ++c) {
-        if (tnorm[(uint64_t)t * d.C + c] == 0.f) continue;
-        const float* tr = T + ((uint64_t)t * d.C + c) * d.W;
-        const float* vr = V + (uint64_t)c * d.N + s;
-        for (uint32_t j = 0; j < d.W; ++j) acc = __fadd_rn(acc, __fmul_rn(tr[j], vr[j]));
-    }
-    return acc;
-}
-
 
 // TMEM -> registers: 4 consecutive accumulator columns of the warp's 32 lanes.
 // The wait is a separate statement that names the destination registers, so no
@@ -1116,76 +1090,35 @@ __global__ void __launch_bounds__(persist_threads(NE), 1) lik_tc_persist_kernel(
     }
 }
 
-// With lazy exactness, each positive exact value also enters its window's key
-// and positive flag (after the likelihood kernel has published the CTA's own).
-__device__ __forceinline__ void note_window(const Dims& d, unsigned long long* wkey, uint8_t* wpos, float v,
-                                            uint32_t t, uint32_t s)
+// Exact recomputation of the queued runs (reference order, FP32), a warp per run.
+// An entry is (t << 40) | (mask << 32) | s0: samples s0 + k with bit k of the 4-bit
+// mask set.  The lanes form the products of 32 taps at a time (a product rounds the
+// same wherever it is formed; the next 32 taps' operands are already on their way),
+// and every lane adds them one by one in the reference's order, channel-major, taps
+// ascending, over the template's non-zero channels (the others add exact zeros).
+// The chain of additions (about 6 cycles each with its broadcast) bounds a run; one
+// thread per run, with its operands fetched four taps at a time, took 5 to 30 times
+// as long (12.2 ms per pursuit of 20 s of 64 channels x 200 templates).
+__global__ void __launch_bounds__(256) fixup_kernel(Dims d, const float* __restrict__ V, const float* __restrict__ T,
+                                                    const float* __restrict__ bias,
+                                                    const unsigned long long* __restrict__ fix, uint32_t cap,
+                                                    const DevStatus* status, float* L, unsigned long long* wkey,
+                                                    uint8_t* wpos, const float* __restrict__ tnorm)
 {
-    if (wkey == nullptr || !(v > 0.f)) return;
-    const uint32_t w = s / d.W;
-    atomicMax(&wkey[w], window_key(v, t, s - w * d.W));
-    wpos[w] = 1;
-}
-
-// Exact recomputation of the queued runs (reference order, FP32).  An entry
-// is (t << 40) | (mask << 32) | s0: samples s0 + k with bit k of the 4-bit mask
-// set.  A thread carries the four samples' sequential sums side by side: per 4
-// taps one 16-byte template load and 4 voltage loads feed 16 multiply-adds
-// (each sum still adds its products one at a time, in the reference's order).
-__global__ void fixup_kernel(Dims d, const float* __restrict__ V, const float* __restrict__ T,
-                             const float* __restrict__ Tp, const float* __restrict__ bias,
-                             const unsigned long long* __restrict__ fix, uint32_t cap, const DevStatus* status,
-                             float* L, unsigned long long* wkey, uint8_t* wpos, const float* __restrict__ tnorm)
-{
-    const uint32_t n = min(status->n_fix, cap);
-    const uint32_t W = d.W, Wp = (W + 3) & ~3u, W4 = W & ~3u;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t n = min(status->n_fix, cap), lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    for (uint32_t i = blockIdx.x * wpb + (threadIdx.x >> 5); i < n; i += gridDim.x * wpb) {
         const unsigned long long e = fix[i];
-        const uint32_t t = (uint32_t)(e >> 40), mask = (uint32_t)(e >> 32) & 0xFu, s0 = (uint32_t)e;
-        const float b = bias[t];
-        if ((uint64_t)s0 + W + 3 > d.N) {   // the run reaches the end of the chunk: one sample at a time
-            for (uint32_t k = 0; k < 4; ++k)
-                if ((mask >> k) & 1u) {
-                    const float v = exact_likelihood(d, V, T, b, t, s0 + k, tnorm);
-                    L[(uint64_t)t * d.N + s0 + k] = v;
-                    note_window(d, wkey, wpos, v, t, s0 + k);
-                }
-            continue;
-        }
-        float a0 = b, a1 = b, a2 = b, a3 = b;
-        for (uint32_t c = 0; c < d.C; ++c) {
-            if (tnorm[(uint64_t)t * d.C + c] == 0.f) continue;   // an all-zero template channel adds 0
-            const float* vr = V + (uint64_t)c * d.N + s0;
-            const float* tr = Tp + ((uint64_t)t * d.C + c) * Wp;
-            float w0 = __ldg(vr), w1 = __ldg(vr + 1), w2 = __ldg(vr + 2);   // V[s0 + j + 0..2]
-            uint32_t j = 0;
-            for (; j < W4; j += 4) {
-                const float4 t4 = __ldg(reinterpret_cast<const float4*>(tr + j));
-                const float w3 = __ldg(vr + j + 3), w4 = __ldg(vr + j + 4), w5 = __ldg(vr + j + 5),
-                            w6 = __ldg(vr + j + 6);
-                a0 = __fadd_rn(a0, __fmul_rn(t4.x, w0)); a1 = __fadd_rn(a1, __fmul_rn(t4.x, w1));
-                a2 = __fadd_rn(a2, __fmul_rn(t4.x, w2)); a3 = __fadd_rn(a3, __fmul_rn(t4.x, w3));
-                a0 = __fadd_rn(a0, __fmul_rn(t4.y, w1)); a1 = __fadd_rn(a1, __fmul_rn(t4.y, w2));
-                a2 = __fadd_rn(a2, __fmul_rn(t4.y, w3)); a3 = __fadd_rn(a3, __fmul_rn(t4.y, w4));
-                a0 = __fadd_rn(a0, __fmul_rn(t4.z, w2)); a1 = __fadd_rn(a1, __fmul_rn(t4.z, w3));
-                a2 = __fadd_rn(a2, __fmul_rn(t4.z, w4)); a3 = __fadd_rn(a3, __fmul_rn(t4.z, w5));
-                a0 = __fadd_rn(a0, __fmul_rn(t4.w, w3)); a1 = __fadd_rn(a1, __fmul_rn(t4.w, w4));
-                a2 = __fadd_rn(a2, __fmul_rn(t4.w, w5)); a3 = __fadd_rn(a3, __fmul_rn(t4.w, w6));
-                w0 = w4; w1 = w5; w2 = w6;
-            }
-            for (; j < W; ++j) {   // remaining taps; w0..w2 hold V[s0 + j + 0..2]
-                const float tv = __ldg(tr + j);
-                const float w3 = __ldg(vr + j + 3);
-                a0 = __fadd_rn(a0, __fmul_rn(tv, w0)); a1 = __fadd_rn(a1, __fmul_rn(tv, w1));
-                a2 = __fadd_rn(a2, __fmul_rn(tv, w2)); a3 = __fadd_rn(a3, __fmul_rn(tv, w3));
-                w0 = w1; w1 = w2; w2 = w3;
+        const uint32_t t = (uint32_t)(e >> 40), s0 = (uint32_t)e;
+        uint32_t mask = (uint32_t)(e >> 32) & 0xFu;
+        while (mask) {
+            const uint32_t s = s0 + __ffs(mask) - 1;
+            mask &= mask - 1;
+            const float v = warp_exact_lik(d, V, T, bias[t], t, s, tnorm);
+            if (lane == 0) {
+                L[(uint64_t)t * d.N + s] = v;
+                note_window(d, wkey, wpos, v, t, s);
             }
         }
-        float* Lr = L + (uint64_t)t * d.N + s0;
-        if (mask & 1u) { Lr[0] = a0; note_window(d, wkey, wpos, a0, t, s0); }
-        if (mask & 2u) { Lr[1] = a1; note_window(d, wkey, wpos, a1, t, s0 + 1); }
-        if (mask & 4u) { Lr[2] = a2; note_window(d, wkey, wpos, a2, t, s0 + 2); }
-        if (mask & 8u) { Lr[3] = a3; note_window(d, wkey, wpos, a3, t, s0 + 3); }
     }
 }
 
@@ -1536,6 +1469,21 @@ bool persist_config(const Dims& d, const TcConfig& c, PersistConfig* p)
     return false;
 }
 
+// Exact recomputation of the runs the likelihood kernel queued.
+int launch_fixup(const Dims& d, const Work& w, const float* V, const float* T, const float* bias, float* Lk, bool lazy,
+                 cudaStream_t st)
+{
+    const Layout& L = *w.lay;
+    count_launch();
+    KScope ks(&fbp_chunk_stats::ms_fixup, st);
+    fixup_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, bias, w.at<unsigned long long>(L.off_fix),
+                                          (uint32_t)L.n_fix_cap, w.status(), Lk,
+                                          lazy ? w.at<unsigned long long>(L.off_wkey) : nullptr,
+                                          lazy ? w.at<uint8_t>(L.off_wpos) : nullptr, w.at<float>(L.off_tnorm));
+    FBP_CUDA(cudaGetLastError());
+    return FBP_OK;
+}
+
 template <int NE>
 static int launch_persist(const PersistParams& Q, uint32_t grid, size_t smem, cudaStream_t st)
 {
@@ -1602,7 +1550,7 @@ int launch_likelihood_tc(const Dims& d, const Work& w, const float* V, const flo
     }
     FBP_CUDA(cudaMemsetAsync(&w.status()->n_fix, 0, 4, st));
     PersistConfig pc;
-    count_launch(2);
+    count_launch();
     if (lazy && persist_config(d, c, &pc)) {
         // the pursuit's passes: persistent CTAs over batches of tiles
         PersistParams Q;
@@ -1627,11 +1575,7 @@ int launch_likelihood_tc(const Dims& d, const Work& w, const float* V, const flo
         KScope ks(&fbp_chunk_stats::ms_lik_tc, st);
         lik_tc_kernel<<<grid, kThreads, c.smem, st>>>(P);
     }
-    KScope ks(&fbp_chunk_stats::ms_fixup, st);
-    fixup_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, P.Tp, bias, P.fix, P.fix_cap, w.status(), Lk, P.wkey, P.wpos,
-                                          P.tnorm);
-    FBP_CUDA(cudaGetLastError());
-    return FBP_OK;
+    return launch_fixup(d, w, V, T, bias, Lk, lazy, st);
 }
 
 }  // namespace fbp
