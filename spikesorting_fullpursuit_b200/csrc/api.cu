@@ -128,13 +128,13 @@ bool make_layout(const fbp_dims* d, uint32_t flags, Layout* L)
         L->off_wkey = take(nw * 8);
         L->off_wpos = take(nw);
         L->off_wflag = take(nw * M);
+        L->off_clist = take(M * C);
+        L->off_ccnt = take(M * 4);
+        L->off_lbnd = take(M * 8);
         const size_t spec = fft_spectra_bytes(dims_of(*L));
-        if (spec) {
+        if (spec) {   // likelihood and partial correlations by transforms
             L->off_spec = take(spec);
-            L->off_clist = take(M * C);
-            L->off_ccnt = take(M * 4);
             L->off_tw = take(256 * 8);
-            L->off_lbnd = take(M * 8);
             L->off_units = take(nw * 8);
         }
     }
@@ -151,14 +151,16 @@ bool make_layout(const fbp_dims* d, uint32_t flags, Layout* L)
             if (gb > L->nw) gb = L->nw;
             L->gbatch = gb;
             L->off_g = take(gb * per);
-            L->off_vc2 = take(gb * C * 4);              // the batch's window energies per channel
+            L->off_vc2 = take(gb * C * 4);              // the batch's window energies per channel ...
+            L->off_z2 = take(gb * C * 4);               // ... and those of the signals transformed together
             L->off_order = take(gb * 4);                // screening order of a batch (by best label)
-            L->off_perm = take(M * 4 + 8 + M * 8);      // order, then (8-aligned) non-zero channel masks
+            L->off_perm = take(M * 4);                  // template order of the direct partial correlations
             L->off_mx = take(M * M * 4 + 2 * M * 4);   // max -X_ft per pair; max sqrt(E), max E per template
+            const uint64_t xc = M * M * S2 * ((S2 + 31) / 32) * 4;
+            L->off_xc = take(xc);                       // max -X over chunks of 32 shifts, both orders
+            L->off_xct = take(xc);
             L->cand_cap = 16ull << 20;                  // exact-scoring candidates per batch
             L->off_cand = take(L->cand_cap * 8);
-            // screening tables of each persistent screen CTA when they exceed shared memory
-            L->off_bscr = (M * S2 * 8 > 96 * 1024) ? take(296 * M * S2 * 8) : 0;
         }
     }
     L->bytes = align_up(off, 256);
@@ -304,7 +306,7 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
     FBP_CUDA(cudaMemsetAsync(w.base + lay.off_best_lik, 0, lay.off_list - lay.off_best_lik, st));
     FBP_CUDA(cudaMemsetAsync(w.status(), 0, sizeof(DevStatus), st));
     FBP_TRY(launch_iota(w.list(), d.nw, st));
-    if (!plain) FBP_TRY(launch_fft_templates(d, w, templates, st));
+    if (!plain) FBP_TRY(launch_template_info(d, w, templates, st));
     if (use_tc) {
         FBP_TRY(launch_tc_prepare_templates(d, w, templates, st));
         if (ready.n == 0) FBP_TRY(launch_tc_update_voltage(d, w, voltage, nullptr, nullptr, 0, true, st));
@@ -497,6 +499,7 @@ extern "C" int fbp_likelihood(const fbp_dims* dims, int mode, const float* volta
     }
     if (mode != 0 && tc_supported(d)) {
         FBP_CUDA(cudaMemsetAsync(w.status(), 0, sizeof(DevStatus), st));
+        FBP_TRY(launch_template_info(d, w, templates, st, false));
         FBP_TRY(launch_tc_prepare_templates(d, w, templates, st));
         FBP_TRY(launch_tc_update_voltage(d, w, voltage, nullptr, nullptr, 0, true, st));
         uint64_t nfix = 0;

@@ -18,7 +18,7 @@ constexpr size_t kFftSmemMost = 222 * 1024;   // dynamic shared memory of a CTA
 constexpr size_t kSpecMost = 2ull << 30;      // bytes of template spectra
 
 // Per template, one warp: its non-zero channels, their norms (rounded up; 0 for an
-// all-zero channel), the channel mask, the taps padded to a multiple of 4 (exact
+// all-zero channel), the channel mask (all ones above 64 channels), the taps padded to a multiple of 4 (exact
 // recomputation), and the bound of the likelihood's estimate,
 //     lbnd.x sum_c |T_c| |z_c| + lbnd.y |bias|
 // (the reference's sequential sum of n W products, then the transforms, over the
@@ -56,7 +56,7 @@ __global__ void template_info_kernel(Dims d, const float* __restrict__ T, uint8_
         }
         if (lane == 0) {
             ccnt[t] = n;
-            tchm[t] = mask;
+            tchm[t] = d.C <= 64 ? mask : ~0ull;   // more than 64 channels: nothing is skipped by it
             lbnd[t] = make_float2(1.05f * u * ((float)n * d.W + 6.f + kFftTerms + 3.f * n), 1.05f * u * ((float)n * d.W + 8.f));
         }
     }
@@ -94,10 +94,27 @@ __global__ void __launch_bounds__(kFft) spectra_kernel(Dims d, const float* __re
     o[(k >> 4) & 1u] = make_float2((float)(re / kFft), (float)(im / kFft));
 }
 
+// A window's energy e on a channel is not a finite number: its samples are zeroed
+// (PART 0 the real, 1 the imaginary parts), and the energy becomes NaN if a sample is
+// not finite, infinite if only the squares overflow.  By whole half-warps.
+template <int PART>
+__device__ __forceinline__ float keep_apart(float2 (&x)[16], float e)
+{
+    if (e < INFINITY) return e;
+    bool wild = false;
+#pragma unroll
+    for (int m = 0; m < 16; ++m) {
+        float& v = PART ? x[m].y : x[m].x;
+        wild |= !(fabsf(v) < INFINITY);
+        v = 0.f;
+    }
+    return __any_sync(0xFFFFu << (threadIdx.x & 16u), wild) ? __int_as_float(0x7fffffff) : INFINITY;
+}
+
 // Partial correlations of flagged windows (see overlap_fast.cu):
 //     G[k][t][b] = X_t(b) - 0.5 Et[t][b],   X_t(b) = sum_cj T[t][c][j - (b - S)] v[c][j]
-// over the window's W samples, and the window's energy per channel, vc2[k][c].  A CTA
-// takes two windows at a time (kk = 2 u, 2 u + 1 of the batch) as one complex signal:
+// over the window's W samples, the window's energy per channel, vc2[k][c], and that of
+// the signals transformed together, z2[k][c].  A CTA takes two windows at a time (kk = 2 u, 2 u + 1 of the batch) as one complex signal:
 // the windows, zero-padded to 256, are transformed channel by channel, then each
 // half-warp correlates its templates.  A window needs W + min(S, W - 1) <= 256: a
 // shift's samples then never wrap onto another's.
@@ -110,7 +127,7 @@ __global__ void __launch_bounds__(MAXT, MINB) window_corr_kernel(
     Dims d, FftTables F, const float* __restrict__ V, const float* __restrict__ L, const float* __restrict__ theta,
     const float2* __restrict__ Et, const uint32_t* __restrict__ flag, DevStatus* status,
     const uint32_t* __restrict__ best_lab, const uint32_t* __restrict__ best_idx, uint32_t k0, uint32_t kc, float* G,
-    float* vc2)
+    float* vc2, float* z2)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const uint32_t nh = blockDim.x >> 4;
@@ -157,9 +174,16 @@ __global__ void __launch_bounds__(MAXT, MINB) window_corr_kernel(
             }
             ea = half_sum(ea);
             eb = half_sum(eb);
+            if (!(ea + eb < INFINITY)) {   // keep what is not finite, or overflows, off the other window
+                ea = keep_apart<0>(x, ea);
+                eb = keep_apart<1>(x, eb);
+            }
+            __syncwarp();
             if (on && l == 0) {
-                if (2 * u < live) vc2[(size_t)(2 * u) * d.C + c] = ea;
-                if (2 * u + 1 < live) vc2[(size_t)(2 * u + 1) * d.C + c] = eb;
+                const size_t at = (size_t)(2 * u) * d.C + c;
+                const float z = (ea < INFINITY ? ea : 0.f) + (eb < INFINITY ? eb : 0.f);
+                if (2 * u < live) { vc2[at] = ea; z2[at] = z; }
+                if (2 * u + 1 < live) { vc2[at + d.C] = eb; z2[at + d.C] = z; }
             }
             // an idle half-warp of the last channels exchanges through a spare buffer
             fft_channel(x, on ? zs + (size_t)c * 128 : reinterpret_cast<float4*>(xbuf + (size_t)h * kFft), tw, l);
@@ -531,16 +555,18 @@ static FftTables fft_tables(const Work& w)
                      w.at<float2>(L.off_tw)};
 }
 
-int launch_fft_templates(const Dims& d, const Work& w, const float* T, cudaStream_t st)
+int launch_template_info(const Dims& d, const Work& w, const float* T, cudaStream_t st, bool spectra)
 {
-    if (fft_spectra_bytes(d) == 0) return FBP_OK;
     const Layout& L = *w.lay;
-    count_launch(2);
+    count_launch();
     template_info_kernel<<<std::min<uint32_t>((d.M + 3) / 4, 148 * 8), 128, 0, st>>>(
         d, T, w.at<uint8_t>(L.off_clist), w.at<uint32_t>(L.off_ccnt), w.at<float>(L.off_tnorm),
         w.at<unsigned long long>(L.off_tchm), w.at<float>(L.off_tpad), w.at<float2>(L.off_lbnd));
-    spectra_kernel<<<d.M * d.C, kFft, 0, st>>>(d, T, w.at<uint8_t>(L.off_clist), w.at<uint32_t>(L.off_ccnt),
-                                               w.at<float4>(L.off_spec), w.at<float2>(L.off_tw));
+    if (spectra && fft_spectra_bytes(d) > 0) {
+        count_launch();
+        spectra_kernel<<<d.M * d.C, kFft, 0, st>>>(d, T, w.at<uint8_t>(L.off_clist), w.at<uint32_t>(L.off_ccnt),
+                                                   w.at<float4>(L.off_spec), w.at<float2>(L.off_tw));
+    }
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -617,7 +643,7 @@ int launch_likelihood_fft(const Dims& d, const Work& w, const float* V, const fl
 }
 
 int launch_window_corr(const Dims& d, const Work& w, const float* V, const float* theta, const float2* Et,
-                       uint32_t k0, uint32_t kc, float* G, float* vc2, cudaStream_t st)
+                       uint32_t k0, uint32_t kc, float* G, float* vc2, float* z2, cudaStream_t st)
 {
     const FftShape s = fft_shape(d.C, d.M, 0);
     const uint32_t grid = std::min<uint32_t>((kc + 1) / 2, 148u * s.per_sm);
@@ -627,7 +653,7 @@ int launch_window_corr(const Dims& d, const Work& w, const float* V, const float
     FBP_CUDA(allow_max_dyn_smem(window_corr_kernel<MAXT, MINB>));                                              \
     window_corr_kernel<MAXT, MINB><<<grid, 16 * s.nh, s.smem, st>>>(d, F, V, w.L(), theta, Et, w.flag(),       \
                                                                     w.status(), w.best_lab(), w.best_idx(),    \
-                                                                    k0, kc, G, vc2)
+                                                                    k0, kc, G, vc2, z2)
     if (s.nh <= 8) {
         FBP_WC(128, 5);
     } else if (s.nh <= 16) {

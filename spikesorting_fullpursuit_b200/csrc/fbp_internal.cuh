@@ -111,9 +111,9 @@ struct Layout {
     // transforms (corr_fft.cu): template spectra, channel lists and counts, twiddles
     size_t off_spec, off_clist, off_ccnt, off_tw, off_lbnd, off_units;
     // screened overlap recheck: truncated energies Et[M][S2] (f64), pair cross
-    // terms XT[M][M][S2][S2] (f32), partial correlations G[gbatch][M][S2] (f32),
-    // template processing order perm[M]
-    size_t off_et, off_xt, off_xtt, off_g, off_order, off_perm, off_mx, off_cand, off_bscr, off_vc2;
+    // terms XT[M][M][S2][S2] (f32) and their chunk bounds, partial correlations
+    // G[gbatch][M][S2] (f32), template processing order perm[M]
+    size_t off_et, off_xt, off_xtt, off_xc, off_xct, off_g, off_order, off_perm, off_mx, off_cand, off_vc2, off_z2;
     uint64_t cand_cap;
     uint64_t gbatch;
     bool screened;
@@ -220,9 +220,10 @@ int launch_tc_update_voltage(const Dims& d, const Work& w, const float* V, const
 size_t fft_spectra_bytes(const Dims& d);        // 0: these sizes are not supported
 bool fft_windows_supported(const Dims& d);      // window correlations at every shift of the recheck
 bool fft_likelihood_chosen(const Dims& d);      // the likelihood of these sizes (and the caller's tuning)
-int launch_fft_templates(const Dims& d, const Work& w, const float* T, cudaStream_t st);
+// non-zero channels, norms, masks and bounds of the templates, and their spectra
+int launch_template_info(const Dims& d, const Work& w, const float* T, cudaStream_t st, bool spectra = true);
 int launch_window_corr(const Dims& d, const Work& w, const float* V, const float* theta, const float2* Et,
-                       uint32_t k0, uint32_t kc, float* G, float* vc2, cudaStream_t st);
+                       uint32_t k0, uint32_t kc, float* G, float* vc2, float* z2, cudaStream_t st);
 // the pursuit's likelihood (lazy exactness); nlist == d.nw: the whole chunk, spans [span0, span0 + span_count) of fft_span(d) samples
 // each; span k reads the voltage up to sample (k + 1) * fft_span(d) + W - 2
 int launch_likelihood_fft(const Dims& d, const Work& w, const float* V, const float* T, const float* bias,

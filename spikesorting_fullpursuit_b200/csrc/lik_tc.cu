@@ -1237,28 +1237,9 @@ __global__ void voltage_repack_kernel(Dims d, const float* __restrict__ V, uint3
     }
 }
 
-// Tq[j][qp][h][n][e] = T[n][(2qp+h)*4+e][j]; Tp[t][c][j] = T[t][c][j] (zero for
-// j >= W); tnorm[t][c] = |T[t][c][:]|.
-__global__ void template_pack_kernel(Dims d, const float* __restrict__ T, uint32_t Cq, uint32_t Np, float* Tq,
-                                     float* Tp, float* tnorm, unsigned long long* tchm)
+// Tq[j][qp][h][n][e] = T[n][(2qp+h)*4+e][j].
+__global__ void template_pack_kernel(Dims d, const float* __restrict__ T, uint32_t Cq, uint32_t Np, float* Tq)
 {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < d.M; t += gridDim.x * blockDim.x) {
-        unsigned long long m = 0ull;
-        for (uint32_t c = 0; c < d.C && c < 64; ++c) {
-            const float* r = T + ((uint64_t)t * d.C + c) * d.W;
-            bool nz = false;
-            for (uint32_t j = 0; j < d.W && !nz; ++j) nz = r[j] != 0.f;
-            if (nz) m |= 1ull << c;
-        }
-        tchm[t] = m;
-    }
-    const uint32_t Wp = (d.W + 3) & ~3u;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)d.M * d.C * Wp;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t j = (uint32_t)(i % Wp);
-        const uint64_t tc = i / Wp;
-        Tp[i] = j < d.W ? T[tc * d.W + j] : 0.f;
-    }
     const uint64_t total = (uint64_t)d.W * Cq * Np * 4;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t e = i % 4;
@@ -1267,12 +1248,6 @@ __global__ void template_pack_kernel(Dims d, const float* __restrict__ T, uint32
         const uint32_t j = (uint32_t)(i / 4 / Np / Cq);
         const uint32_t c = qh * 4 + e;
         Tq[i] = (n < d.M && c < d.C) ? T[((uint64_t)n * d.C + c) * d.W + j] : 0.f;
-    }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < d.M * d.C; i += gridDim.x * blockDim.x) {
-        const float* r = T + (uint64_t)i * d.W;
-        double a = 0.0;
-        for (uint32_t j = 0; j < d.W; ++j) a += (double)r[j] * r[j];
-        tnorm[i] = (float)(sqrt(a) * (1.0 + 1e-6));
     }
 }
 
@@ -1383,8 +1358,7 @@ int launch_tc_prepare_templates(const Dims& d, const Work& w, const float* T, cu
     if (!tc_config(d, &c)) return FBP_OK;
     const Layout& L = *w.lay;
     count_launch();
-    template_pack_kernel<<<256, 256, 0, st>>>(d, T, c.Cq, c.Np, w.at<float>(L.off_tt_hi), w.at<float>(L.off_tpad),
-                                              w.at<float>(L.off_tnorm), w.at<unsigned long long>(L.off_tchm));
+    template_pack_kernel<<<256, 256, 0, st>>>(d, T, c.Cq, c.Np, w.at<float>(L.off_tt_hi));
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }

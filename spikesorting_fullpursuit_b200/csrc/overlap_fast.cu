@@ -9,14 +9,12 @@
 //     X_ft     = sum_cj F_a[c,j] T_b[c,j]
 // G is a partial correlation of every template with the window (computed per
 // window), X_ft depends only on the template pair and the two shifts (a table
-// built once per call).  |v_ref - estimate| is bounded rigorously by a
-// function of truncated template energies and the window's norm (see
-// est_bound in screen_kernel).  Only items whose interval can reach the best lower bound (and
-// the window's seed likelihood) are scored exactly in the reference's float
-// order; the winner key -- value, then work-group, then tree slot -- is
-// therefore the reference's.
-#include <cub/cub.cuh>
-
+// built once per call).  |v_ref - estimate| is bounded rigorously by a margin
+// per window and template pair (pair_margin).  Only items whose interval can
+// reach the best lower bound (and the window's seed likelihood) are scored
+// exactly in the reference's float order; the winner key -- value, then
+// work-group, then tree slot -- is therefore the reference's.
+#include <algorithm>
 #include <vector>
 
 #include "fft256.cuh"
@@ -28,117 +26,168 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
 
-// Truncated energy of template t at shift x: sum over the template samples u
-// that land inside the window, u in [S-x, S-x+W) and [0, W).  Stored as
-// (E, sqrt(E)), each rounded up, for the screening bound and the partial
-// correlations.
-__global__ void energy_table_kernel(Dims d, const float* __restrict__ T, float2* Et)
+// Truncated energies of template t (one CTA): E(x) = sum over the template samples
+// u that land inside the window at shift x, u in [S-x, S-x+W) and [0, W), as
+// (E, sqrt(E)), each rounded up (partial correlations), and their maxima over the
+// shifts, maxs[t] = sqrt(E), maxs[M + t] = E (screening bound).
+__global__ void __launch_bounds__(128) energy_table_kernel(Dims d, const float* __restrict__ T, float2* Et, float* maxs)
 {
-    const uint32_t S2 = 2 * d.S + 1;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < d.M * S2; i += gridDim.x * blockDim.x) {
-        const uint32_t t = i / S2, x = i % S2;
-        const int lo = max(0, (int)d.S - (int)x), hi = min((int)d.W, (int)d.S - (int)x + (int)d.W);
+    extern __shared__ double cum[];   // [W + 1] running energy over the taps
+    __shared__ int s_me, s_ms;
+    const uint32_t t = blockIdx.x, S2 = 2 * d.S + 1, W = d.W;
+    if (threadIdx.x == 0) { cum[0] = 0.0; s_me = 0; s_ms = 0; }
+    for (uint32_t u = threadIdx.x; u < W; u += blockDim.x) {
         double e = 0.0;
         for (uint32_t c = 0; c < d.C; ++c) {
-            const float* r = T + ((uint64_t)t * d.C + c) * d.W;
-            for (int u = lo; u < hi; ++u) e += (double)r[u] * (double)r[u];
+            const double v = T[((uint64_t)t * d.C + c) * W + u];
+            e = fma(v, v, e);
         }
-        Et[i] = make_float2(__double2float_ru(e * (1.0 + 1e-12)), __double2float_ru(sqrt(e) * (1.0 + 1e-12)));
+        cum[u + 1] = e;
     }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (uint32_t u = 1; u <= W; ++u) cum[u] += cum[u - 1];
+    __syncthreads();
+    float me = 0.f, ms = 0.f;
+    for (uint32_t x = threadIdx.x; x < S2; x += blockDim.x) {
+        const int lo = max(0, (int)d.S - (int)x), hi = min((int)W, (int)d.S - (int)x + (int)W);
+        // the difference of two running sums is off by at most 2 W 2^-53 of the whole energy
+        const double e = hi > lo ? (cum[hi] - cum[lo]) * (1.0 + 1e-12) + cum[W] * 1e-12 : 0.0;
+        const float ef = __double2float_ru(e), es = __double2float_ru(sqrt(e) * (1.0 + 1e-12));
+        Et[(uint64_t)t * S2 + x] = make_float2(ef, es);
+        me = fmaxf(me, ef);
+        ms = fmaxf(ms, es);
+    }
+    atomicMax(&s_me, __float_as_int(me));   // both >= 0
+    atomicMax(&s_ms, __float_as_int(ms));
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        maxs[t] = __int_as_float(s_ms);
+        maxs[d.M + t] = __int_as_float(s_me);
+    }
+}
+
+// largest value of the warp's lanes, NaN ignored
+__device__ __forceinline__ float warp_max(float v)
+{
+    float r;
+    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
 }
 
 // Pair cross terms X_ft(a, b) for |a-b| <= W, one CTA per (f, t), stored as
 // XT[f][t][a][b] and transposed as XTT[f][t][b][a]: products
 // P_delta[u] = sum_c F[c,u] T[c,u+delta] in double, prefix sums over u, then
-// X_ft(a, b) = Q_delta[hi] - Q_delta[lo] with delta = a-b.
-constexpr int kLagChunk = 16;
+// X_ft(a, b) = Q_delta[hi] - Q_delta[lo] with delta = a-b.  Pairs without a shared
+// channel have X == 0: their table is never read and stays unwritten.  Also the
+// bounds over whole chunks of 32 shifts, XC[f][a][t][ch] = max over b of the chunk,
+// |a-b| <= W, of -X_ft(a, b) (-inf if there is none) and XCT[f][t][b][ch] over a, and
+// max -X (at least 0) per pair.  32 lags at a time: a lag is a lane, so that a warp
+// writes 32 consecutive shifts of a row (with the row index on the lanes every 4-byte
+// store was a sector of its own: 64 channels x 200 templates about 12 ms of a call).
+constexpr int kCrossThreads = 256;
 
-__global__ void __launch_bounds__(256) cross_table_kernel(Dims d, const float* __restrict__ T, float* XT, float* XTT,
-                                                          float* max_negx)
+__global__ void __launch_bounds__(kCrossThreads) cross_table_kernel(Dims d, const float* __restrict__ T,
+                                                                    const unsigned long long* __restrict__ chmask,
+                                                                    int lags, float* XT, float* XTT, float* XC,
+                                                                    float* XCT, float* max_negx)
 {
-    typedef cub::BlockReduce<float, 256> RF;
-    __shared__ typename RF::TempStorage rtmp;
-    float mneg = 0.f;
     extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ int s_neg;
     const uint32_t f = blockIdx.x / d.M, t = blockIdx.x % d.M;
-    const uint32_t S2 = 2 * d.S + 1, W = d.W, C = d.C;
+    const uint32_t S2 = 2 * d.S + 1, W = d.W, C = d.C, nch = (S2 + 31) / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = kCrossThreads / 32;
+    const unsigned long long both = chmask[f] & chmask[t];   // all ones above 64 channels
+    if (both == 0ull) {
+        if (threadIdx.x == 0) max_negx[blockIdx.x] = 0.f;
+        return;
+    }
+    const uint32_t pitch = (W + 1) | 1u;   // odd: the lags of a warp read different banks
     float* Fs = reinterpret_cast<float*>(smraw);
     float* Ts = Fs + C * W;
-    double* Q = reinterpret_cast<double*>(Ts + C * W);  // [kLagChunk][W+1]; 8*C*W bytes in, aligned
+    double* Q = reinterpret_cast<double*>(Ts + C * W);  // [lags <= 32][pitch]; 8*C*W bytes in, aligned
+    if (threadIdx.x == 0) s_neg = 0;
     for (uint32_t e = threadIdx.x; e < C * W; e += blockDim.x) {
         Fs[e] = T[(uint64_t)f * C * W + e];
         Ts[e] = T[(uint64_t)t * C * W + e];
     }
     __syncthreads();
+    float* xt = XT + (uint64_t)blockIdx.x * S2 * S2;
+    float* xtt = XTT + (uint64_t)blockIdx.x * S2 * S2;
     const int dmax = (int)min(W, 2 * d.S);
-    for (int d0 = -dmax; d0 <= dmax; d0 += kLagChunk) {
-        for (uint32_t e = threadIdx.x; e < kLagChunk * W; e += blockDim.x) {
-            const int li = e / W, u = e % W, delta = d0 + li;
-            double acc = 0.0;
-            if (delta <= dmax && u + delta >= 0 && u + delta < (int)W)
-                for (uint32_t c = 0; c < C; ++c) acc += (double)Fs[c * W + u] * (double)Ts[c * W + u + delta];
-            Q[li * (W + 1) + u + 1] = acc;
+    for (int d0 = -dmax; d0 <= dmax; d0 += lags) {
+        for (int li = warp; li < lags; li += nwarps) {
+            const int delta = d0 + li;
+            double* q = Q + li * pitch;
+            double run = 0.0;   // prefix sums of a lag by a warp, 32 taps at a time
+            if (lane == 0) q[0] = 0.0;
+            for (uint32_t u0 = 0; u0 < W; u0 += 32) {
+                const int u = (int)(u0 + lane);
+                double acc = 0.0;
+                if (u < (int)W && u + delta >= 0 && u + delta < (int)W && delta <= dmax) {
+                    if (C <= 64)
+                        for (unsigned long long m = both; m; m &= m - 1) {
+                            const uint32_t c = __ffsll((long long)m) - 1;
+                            acc = fma((double)Fs[c * W + u], (double)Ts[c * W + u + delta], acc);
+                        }
+                    else
+                        for (uint32_t c = 0; c < C; ++c)
+                            acc = fma((double)Fs[c * W + u], (double)Ts[c * W + u + delta], acc);
+                }
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const double o = __shfl_up_sync(0xffffffffu, acc, off);
+                    if ((int)lane >= off) acc += o;
+                }
+                acc += run;
+                if (u < (int)W) q[u + 1] = acc;
+                run = __shfl_sync(0xffffffffu, acc, 31);
+            }
         }
         __syncthreads();
-        if (threadIdx.x < kLagChunk) {
-            double* q = Q + threadIdx.x * (W + 1);
-            q[0] = 0.0;
-            for (uint32_t u = 1; u <= W; ++u) q[u] += q[u - 1];
-        }
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < kLagChunk * S2; e += blockDim.x) {
-            const int li = e / S2, a = e % S2, delta = d0 + li;
+        const int delta = (int)lane < lags ? d0 + (int)lane : dmax + 1;
+        for (int a = (int)warp; a < (int)S2; a += nwarps) {   // row a: shifts b = a - delta
             const int b = a - delta;
             if (delta > dmax || b < 0 || b >= (int)S2) continue;
             const int lo = max(max(0, -delta), (int)d.S - a);
             const int hi = min(min((int)W, (int)W - delta), (int)d.S - a + (int)W);
-            const double v = hi > lo ? Q[li * (W + 1) + hi] - Q[li * (W + 1) + lo] : 0.0;
-            const float xv = (float)v;
-            XT[(((uint64_t)f * d.M + t) * S2 + a) * S2 + b] = xv;
-            XTT[(((uint64_t)f * d.M + t) * S2 + b) * S2 + a] = xv;
-            mneg = fmaxf(mneg, -xv);
+            xt[(uint64_t)a * S2 + b] = hi > lo ? (float)(Q[lane * pitch + hi] - Q[lane * pitch + lo]) : 0.f;
+        }
+        for (int b = (int)warp; b < (int)S2; b += nwarps) {   // row b of the transposed table: a = b + delta
+            const int a = b + delta;
+            if (delta > dmax || a < 0 || a >= (int)S2) continue;
+            const int lo = max(max(0, -delta), (int)d.S - a);
+            const int hi = min(min((int)W, (int)W - delta), (int)d.S - a + (int)W);
+            xtt[(uint64_t)b * S2 + a] = hi > lo ? (float)(Q[lane * pitch + hi] - Q[lane * pitch + lo]) : 0.f;
         }
         __syncthreads();
     }
-    const float m = RF(rtmp).Reduce(mneg, cub::Max());
-    if (threadIdx.x == 0) max_negx[blockIdx.x] = m;
-}
-
-// Per template: max over shifts of sqrt(E) and of E (bounds for whole rows).
-__global__ void energy_max_kernel(Dims d, const float2* __restrict__ Et, float* maxs)
-{
-    const uint32_t S2 = 2 * d.S + 1;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < d.M; t += gridDim.x * blockDim.x) {
-        float ms = 0.f, me = 0.f;
-        for (uint32_t x = 0; x < S2; ++x) {
-            ms = fmaxf(ms, Et[(uint64_t)t * S2 + x].y);
-            me = fmaxf(me, Et[(uint64_t)t * S2 + x].x);
+    float neg = 0.f;
+    for (uint32_t e = warp; e < 2 * S2; e += nwarps) {
+        const uint32_t y = e >> 1;
+        const float* row = ((e & 1u) ? xtt : xt) + (uint64_t)y * S2;
+        float* out = (e & 1u) ? XCT + ((uint64_t)blockIdx.x * S2 + y) * nch
+                              : XC + (((uint64_t)f * S2 + y) * d.M + t) * nch;
+        for (uint32_t ch = 0; ch < nch; ++ch) {
+            const uint32_t x = ch * 32 + lane;
+            const bool in = x < S2 && x + W >= y && x <= y + W;
+            const float m = warp_max(in ? -row[x] : -INFINITY);
+            if (lane == 0) out[ch] = m;
+            neg = fmaxf(neg, m);
         }
-        maxs[t] = ms;
-        maxs[d.M + t] = me;
     }
+    if (lane == 0) atomicMax(&s_neg, __float_as_int(neg));
+    __syncthreads();
+    if (threadIdx.x == 0) max_negx[blockIdx.x] = __int_as_float(s_neg);
 }
 
-// Template processing order for the partial correlations: sorted by the
-// first non-zero channel so groups of neighbouring templates share channels.
-__global__ void template_order_kernel(Dims d, const float* __restrict__ T, uint32_t* perm,
-                                      unsigned long long* chmask)
+// Template processing order of the direct partial correlations: sorted by the first
+// non-zero channel so groups of neighbouring templates share channels.
+__global__ void template_order_kernel(Dims d, const uint8_t* __restrict__ clist, const uint32_t* __restrict__ ccnt,
+                                      uint32_t* perm)
 {
     extern __shared__ uint32_t key[];
-    for (uint32_t t = threadIdx.x; t < d.M; t += blockDim.x) {
-        uint32_t first = d.C;
-        unsigned long long m = 0ull;
-        for (uint32_t c = 0; c < d.C; ++c) {
-            bool nz = false;
-            for (uint32_t j = 0; j < d.W && !nz; ++j) nz = T[((uint64_t)t * d.C + c) * d.W + j] != 0.f;
-            if (nz) {
-                if (first == d.C) first = c;
-                m |= c < 64 ? (1ull << c) : 0ull;
-            }
-        }
-        key[t] = first;
-        chmask[t] = d.C <= 64 ? m : ~0ull;   // more than 64 channels: no skipping
-    }
+    for (uint32_t t = threadIdx.x; t < d.M; t += blockDim.x) key[t] = ccnt[t] ? clist[(size_t)t * d.C] : d.C;
     __syncthreads();
     if (threadIdx.x == 0) {
         for (uint32_t t = 0; t < d.M; ++t) perm[t] = t;
@@ -352,6 +401,13 @@ __device__ float pair_exact_g(const Dims& d, const float* __restrict__ T, const 
     return acc;
 }
 
+// the same, out of line
+__device__ __noinline__ float pair_exact_call(const Dims d, const float* T, const float* V, uint32_t f, uint32_t t,
+                                              uint32_t p, uint32_t a, uint32_t b, unsigned long long chans)
+{
+    return pair_exact_g(d, T, V, f, t, p, a, b, chans);
+}
+
 __device__ __forceinline__ uint32_t item_priority(uint64_t r, uint32_t WG, uint32_t lbits)
 {
     const uint32_t g = (uint32_t)(r / WG), l = (uint32_t)(r % WG);
@@ -359,470 +415,484 @@ __device__ __forceinline__ uint32_t item_priority(uint64_t r, uint32_t WG, uint3
     return g * WG + br;
 }
 
-constexpr int kScrThreads = 384;
-constexpr int kRowCap = 2048;   // surviving rows kept in shared memory
-constexpr int kCandCap = 256;   // candidates buffered in shared memory per window (more go straight to the global list)
-constexpr int kScanQ = 8;       // items per lane of a row chunk (32 * kScanQ shifts)
-constexpr uint32_t kBStage = 96 * 1024;   // per-window item tables staged in shared memory up to this size
-constexpr uint32_t kScreenGrid = 148 * 2;  // persistent CTAs (two per SM); also sizes the unstaged table scratch
+constexpr int kScrThreads = 128;
+constexpr uint32_t kChunkCap = 512;    // chunks of 32 items kept in shared memory
+constexpr uint32_t kRowCap = 768;      // rows (t, b) kept in shared memory
+constexpr uint32_t kQueue = 64;        // chunks a warp keeps for evaluation
+constexpr int kScrPerSm = 8;
+
+struct ScreenArgs {
+    Dims d;
+    const float* V;
+    const float* T;
+    const float* L;
+    const float* theta;
+    const float* XT;
+    const float* XTT;
+    const float* XC;
+    const float* XCT;
+    const float* mx;        // [M][M] max -X, then [M] max sqrt(E), [M] max E
+    const float* G;
+    const float* vc2;       // [kc][C] window energies per channel, or null: from the voltage (direct correlations)
+    const float* z2;        // [kc][C] energies of the signal pair transformed together
+    uint32_t k0, kc;
+    const uint32_t* flag;
+    DevStatus* status;
+    const uint32_t* best_lab;
+    const uint32_t* best_idx;
+    const float* best_lik;
+    unsigned long long* keys;
+    unsigned long long* gcand;
+    uint32_t cand_cap;
+    const unsigned long long* chmask;
+    const uint32_t* order;
+};
 
 struct ScreenShared {
-    float lb;
-    float maxau2;
+    int lb;              // largest lower bound, float bits (0: none above 0)
+    uint32_t nA, top;    // shifts in A+, the place in alist of the largest G_f
+    uint32_t nrows, nchunks, full;
     unsigned long long best;
-    uint32_t nA;
-    uint32_t nrows;
-    uint32_t ncand;
-    uint32_t gfull;   // the global candidate list ran out of room for this window
 };
 
-// Shared-memory bytes of screen_kernel for these sizes (tables staged or not).
-__host__ __device__ inline size_t screen_smem_bytes(uint32_t M, uint32_t S2, bool staged)
+__host__ __device__ inline uint32_t scr_chunks(uint32_t S2) { return (S2 + 31) / 32; }
+
+// Shared-memory bytes of screen_kernel.
+__host__ __device__ inline size_t screen_smem_bytes(uint32_t M, uint32_t S2, uint32_t C)
 {
-    const size_t s2p = (S2 + 3) & ~3u, mp = (M + 3) & ~3u;
-    size_t b = 5 * s2p * 4 + 4 * mp * 4 + 256 * 4 + (size_t)kRowCap * 8 + (size_t)kCandCap * 12;
-    b += (((size_t)S2 + 15) & ~(size_t)15) + (((size_t)M * S2 + 15) & ~(size_t)15);
-    if (staged) b += (size_t)M * S2 * 8;
-    return b + 64;
+    const size_t nch = scr_chunks(S2);
+    return (nch * 32 * 2 + (size_t)M * nch * 2 + (size_t)M * 4 + nch + C * 2 + kChunkCap * 3 + kRowCap * 2 +
+            kQueue * 2 * (kScrThreads / 32)) * 4 + 16;
 }
 
-// One row of items seen from the lanes of a warp: the row's fixed part (uf,
-// lf), the per-item parts (ua[x], la[x]) and the cross terms xr[x] for x in
-// [lo, hi).  Item bounds: UB = (uf + ua[x]) - X, LB = (lf + la[x]) - X.
-struct ScreenRow {
-    float uf, lf;
-    const float* ua;
-    const float* la;
-    const float* xr;   // null: the templates share no channel, X == 0
-    int lo, hi;
-    uint32_t t, y;
-    bool fixed_a;
+// Bound of |estimate - reference float value| of every item (a, t, b) of a window
+// with best template f, u = 2^-24, over the templates' whole energies E (at least any
+// truncated one):
+//     u 1.06 [ (U (W + 1) + W + 48) (A_f + A_t) + B_f + B_t ],
+//     A_x = sqrt E_x |v|_x + E_x,  |v|_x the window's norm over template x's channels.
+// The first part: the reference adds U (W + 1) terms one at a time, U the channels
+// where f or t is not zero (elsewhere it adds exact zeros), W of each channel's
+// energy, and the estimate's own few operations; |s v| <= |f v| + |t v|,
+// s^2 <= 2 f^2 + 2 t^2.  B_x: the partial correlations -- by transforms
+// (64 + 3 n_x) sqrt E_x |z|_x (fft256.cuh, z the pair of windows transformed
+// together), directly n_x W sqrt E_x |v|_x.  An infinite margin (the window's energy
+// overflows) keeps every item, NaN (a sample is not finite: so are the reference's
+// values) none.
+struct MarginPart {
+    float a, b;   // A_x, B_x
 };
 
+__device__ __forceinline__ MarginPart margin_part(const ScreenArgs& P, uint32_t t, const float* ve, const float* ze)
+{
+    const Dims& d = P.d;
+    float v2 = 0.f, z2 = 0.f;
+    uint32_t n = 0;
+    const unsigned long long m = P.chmask[t];
+    for (uint32_t c = 0; c < d.C; ++c)
+        if (d.C > 64 || ((m >> c) & 1ull)) {
+            v2 += ve[c];
+            z2 += ze[c];
+            ++n;
+        }
+    const float se = P.mx[(size_t)d.M * d.M + t], e = P.mx[(size_t)d.M * d.M + d.M + t];
+    const float nv = se > 0.f ? sqrtf(v2) * 1.001f : 0.f, nz = se > 0.f ? sqrtf(z2) * 1.001f : 0.f;
+    MarginPart r;
+    r.a = fmaf(se, nv, e);
+    r.b = P.vc2 ? (kFftTerms + 3.f * n) * se * nz : (float)n * d.W * se * nv;
+    return r;
+}
+
+__device__ __forceinline__ float pair_margin(const Dims& d, MarginPart f, MarginPart t, uint32_t U)
+{
+    return 1.06f / 16777216.f * (((float)U * (d.W + 1) + d.W + 48.f) * (f.a + t.a) + f.b + t.b);
+}
+
 // Screening of one flagged window per CTA.
-//   rows, kind 1: (a in A+, t) -- a fixed, the lanes run over b (cross table XT[f][t][a][:]);
-//   rows, kind 2: (t, b) with L_t(b) > 0 -- b fixed, the lanes run over a not in A+
-//                 (transposed cross table XTT[f][t][b][:]).
-// Per window the CTA stages Bu/Bl[t][b] = G_t(b) +- beta_t(b) and Au/Al[a] =
-// G_f(a) +- alpha(a), with alpha + beta = K (sqrt E_f(a) |v|_f + sqrt E_t(b) |v|_t +
-// E_f(a) + E_t(b)) the rigorous bound of |estimate - reference float value|
-// (|v|_x: the window's norm over template x's non-zero channels)
-// (K carries slack for the few float operations of this regrouping).  Partial
-// correlations made by transforms (vc2 given: the windows' energies per channel)
-// are off by at most (64 + 3 n_x) u |T_x| |z|_x instead, z the pair of windows
-// transformed together (fft256.cuh): that is added once per template, and K keeps
-// the reference's own rounding only.  Phase B
-// bounds every row from shared-memory maxima (each component at least the
-// item's, same monotone float order) and keeps the rows that can reach the
-// window's seed; a quick lower bound from the best row of each warp prunes
-// them further.  Phase C scans the kept rows two at a time per warp (all
-// loads of both rows in flight together): LB = max(LB items) and per-row
-// maxima of UB.  Phase D lists the items of rows reaching max(LB, seed, 0)
-// whose UB does; score_kernel scores them exactly.
-__global__ void __launch_bounds__(kScrThreads, 2) screen_kernel(
-    Dims d, const float* __restrict__ V, const float* __restrict__ T, const float* __restrict__ L,
-    const float* __restrict__ theta, const float2* __restrict__ Etab, const float* __restrict__ XT,
-    const float* __restrict__ XTT, const float* __restrict__ G, uint32_t k0, uint32_t kcount,
-    const uint32_t* __restrict__ flag, DevStatus* status, const uint32_t* __restrict__ best_lab,
-    const uint32_t* __restrict__ best_idx, const float* __restrict__ best_lik, unsigned long long* keys,
-    const float* __restrict__ mx, unsigned long long* gcand, uint32_t gcand_cap,
-    const unsigned long long* __restrict__ chmask, float* bscratch, const uint32_t* __restrict__ order,
-    const float* __restrict__ vc2)
+//   rows, kind 0: (a in A+, t) -- a fixed, the lanes run over b (XT[f][t][a][:]);
+//   rows, kind 1: (t, b) with L_t(b) > 0 -- b fixed, the lanes run over a not in A+
+//                 (XTT[f][t][b][:]),
+// A+ the in-bounds shifts with L_f > 0.  An item's interval is its estimate
+// (G_f(a) + G_t(b)) - X +- margin.  A row is taken up while an upper bound (largest G
+// of its variable shift, largest -X of the pair) reaches the seed and the lower bound
+// so far, then those of its chunks of 32 items whose own bound (largest G and largest
+// -X of the chunk) does, then their items, which raise the lower bound; the rows of
+// the a with the largest G_f come first.  Chunks with an item that reaches the lower
+// bound are kept, and their items listed for score_kernel in the end.
+//
+// 32 rows are tested at a time, one a lane; the chunks that pass are queued per warp
+// and evaluated eight at a time, their loads in flight together.  About 270 (16
+// channels x 40 templates) and 300 chunks (64 x 200) are evaluated per window, and 1 to
+// 9 items of it reach the exact scoring.  Measured per pursuit, against whole rows
+// scanned after staging G +- margin of every template and shift: 300 s of 16 channels
+// 31.9 -> 14.5 ms, 20 s of 64 channels 37.4 -> 14.3 ms (and 8.5 M -> 0.16 M items
+// scored exactly there, by the margin's count of non-zero channels).  Bounded by
+// instruction issue and latency together: 49 % of the issue slots, 28 warps per SM.
+__global__ void __launch_bounds__(kScrThreads, kScrPerSm) screen_kernel(const __grid_constant__ ScreenArgs P)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ ScreenShared sh;
-    __shared__ uint32_t s_gbase;
-    typedef cub::BlockReduce<float, kScrThreads> RF;
-    typedef cub::BlockScan<uint32_t, kScrThreads> SC;
-    __shared__ union {
-        typename RF::TempStorage rf;
-        typename SC::TempStorage sc;
-    } tmp;
-    const uint32_t S = d.S, W = d.W, M = d.M, S2 = 2 * S + 1;
-    const uint32_t s2p = (S2 + 3) & ~3u, mp = (M + 3) & ~3u;
+    const Dims& d = P.d;
+    const uint32_t S = d.S, W = d.W, M = d.M, C = d.C, S2 = 2 * S + 1, nch = scr_chunks(S2);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = kScrThreads / 32;
-    const bool staged = (uint64_t)M * S2 * 8 <= kBStage;
-    // shared layout
-    float* Au = reinterpret_cast<float*>(smraw);   // [S2] G_f(a) + alpha(a), a in bounds
-    float* Al = Au + s2p;                          // [S2] G_f(a) - alpha(a)
-    float* Au2 = Al + s2p;                         // [S2] as Au for a in bounds and not in A+, else -inf
-    float* Al2 = Au2 + s2p;
-    uint32_t* alist = reinterpret_cast<uint32_t*>(Al2 + s2p);   // [S2] A+ in ascending order
-    float* gmaxu = reinterpret_cast<float*>(alist + s2p);       // [M] max_b Bu[t][b]
-    float* nx = gmaxu + mp;                                     // [M] max -X_ft over items
-    float* nvt = nx + mp;                                       // [M] window norm over template t's channels
-    float* mft = nvt + mp;                                      // [M] bound of the transforms' rounding
-    float* ve = mft + mp;                                       // [C <= 256] window energy per channel
-    float* rowmax = ve + 256;                                   // [kRowCap]
-    uint32_t* rows = reinterpret_cast<uint32_t*>(rowmax + kRowCap);   // [kRowCap]
-    uint32_t* cand = rows + kRowCap;                            // [kCandCap][3]
-    uint8_t* fa = reinterpret_cast<uint8_t*>(cand + 3 * kCandCap);   // [S2] bit0 in bounds, bit1 L_f > 0
-    uint8_t* pt = fa + ((S2 + 15) & ~15u);                      // [M][S2] L_t(b) > 0, b in bounds
-    float* Bu = staged ? reinterpret_cast<float*>(pt + ((M * S2 + 15) & ~15u))
-                       : bscratch + (uint64_t)blockIdx.x * M * S2 * 2;   // [M][S2]
-    float* Bl = Bu + (size_t)M * S2;                                        // [M][S2]
+    const uint32_t full = 0xffffffffu, below = (1u << lane) - 1u;
+    float* Gf = reinterpret_cast<float*>(smraw);                       // [nch * 32] G_f, -inf out of bounds
+    uint32_t* alist = reinterpret_cast<uint32_t*>(Gf + nch * 32);      // [nch * 32] A+ in ascending order
+    float* gch = reinterpret_cast<float*>(alist + nch * 32);           // [M][nch] largest G_t of a chunk
+    uint32_t* pb = reinterpret_cast<uint32_t*>(gch + (size_t)M * nch); // [M][nch] shifts with L_t > 0
+    float* gmax = reinterpret_cast<float*>(pb + (size_t)M * nch);      // [M] largest G_t
+    float* nx = gmax + M;                                              // [M] largest -X_ft
+    float* cst = nx + M;                                               // [M] margin of the pair (f, t)
+    uint32_t* share = reinterpret_cast<uint32_t*>(cst + M);            // [M] f and t share a channel
+    float* afch = reinterpret_cast<float*>(share + M);                 // [nch] largest G_f of a chunk, a not in A+
+    float* ve = afch + nch;                                            // [C] window energies
+    float* ze = ve + C;                                                // [C] pair energies
+    uint32_t* chc = reinterpret_cast<uint32_t*>(ze + C);               // [kChunkCap] chunk << 23 | row (kind << 22 | t << 10 | y)
+    float* chu = reinterpret_cast<float*>(chc + kChunkCap);            // [kChunkCap] upper bound of its items
+    float* chg = chu + kChunkCap;                                      // [kChunkCap] the row's fixed G
+    uint32_t* rowc = reinterpret_cast<uint32_t*>(chg + kChunkCap);     // [kRowCap] rows (t, b) that can reach the seed
+    float* rowg = reinterpret_cast<float*>(rowc + kRowCap);            // [kRowCap] their G_t(b)
+    uint32_t* qc = reinterpret_cast<uint32_t*>(rowg + kRowCap) + warp * kQueue;   // this warp's chunks to evaluate
+    float* qg = reinterpret_cast<float*>(qc - warp * kQueue + nwarps * kQueue) + warp * kQueue;   // their rows' fixed G
     const uint64_t items = (uint64_t)S2 * S2 * M;
-    const uint64_t nloc = (items - 1) / d.WG + 1;
-    const uint64_t slots = nloc * d.WG;
+    const uint64_t slots = ((items - 1) / d.WG + 1) * d.WG;
     uint32_t lbits = 0;
     while ((1u << lbits) < d.WG) ++lbits;
-    const float u = 1.0f / 16777216.0f;
-    const float K = 1.01f * 1.05f * u * (vc2 ? 1.0f : 2.0f) * ((float)d.C * W + d.C + W + 32);
-    const uint32_t nflag = status->n_flag;
-    unsigned long long exact_n = 0, item_n = 0;
-    for (uint32_t jo = blockIdx.x; jo < kcount; jo += gridDim.x) {
-        const uint32_t kk = order[jo];
-        const uint32_t k = k0 + kk;
-        if (k >= nflag) continue;
-        const uint32_t id = flag[k];
-        const uint32_t f = best_lab[id], p = best_idx[id];
-        if (window_skipped(d, L, theta, f, p)) continue;
-        const float seed = best_lik[id];
-        const float thr0 = fmaxf(seed, 0.f);
-        const float* Gk = G + (uint64_t)kk * M * S2;
-        const unsigned long long mf = chmask[f];
-        __syncthreads();
-        // ---- phase A: window quantities.  The window's energy per channel gives,
-        // per template, the norm of the window over that template's channels: a
-        // template's products touch no other channel, so its part of the bound
-        // (Cauchy-Schwarz over its support) needs no more
-        const uint32_t kp = kk ^ 1u;   // the window transformed together with this one
-        const bool pair = vc2 != nullptr && kp < kcount && k0 + kp < nflag;
-        for (uint32_t c = threadIdx.x; vc2 != nullptr && c < d.C; c += blockDim.x) ve[c] = vc2[(size_t)kk * d.C + c];
-        for (uint32_t c = warp; vc2 == nullptr && c < d.C; c += nwarps) {
-            float e2 = 0.f;
+    const uint32_t nflag = P.status->n_flag;
+    const uint32_t live = nflag > P.k0 ? min(P.kc, nflag - P.k0) : 0u;
+    uint32_t evals = 0;   // chunks evaluated by this warp
+    for (uint32_t jo = blockIdx.x; jo < live; jo += gridDim.x) {
+        const uint32_t kk = P.order[jo];
+        const uint32_t id = P.flag[P.k0 + kk];
+        const uint32_t f = P.best_lab[id], p = P.best_idx[id];
+        if (window_skipped(d, P.L, P.theta, f, p)) continue;
+        const float thr0 = fmaxf(P.best_lik[id], 0.f);   // the seed
+        const float* Gk = P.G + (uint64_t)kk * M * S2;
+        // in-bounds shifts x: x + p >= S and x + p < N - W + S
+        const uint32_t xlo = p < S ? S - p : 0u;
+        const uint32_t xhi = (uint32_t)min((uint64_t)S2, (uint64_t)d.N - W + S - p);
+        __syncthreads();   // the previous window's shared state is read
+        for (uint32_t c = threadIdx.x; P.vc2 != nullptr && c < C; c += blockDim.x) {
+            ve[c] = P.vc2[(size_t)kk * C + c];
+            ze[c] = P.z2[(size_t)kk * C + c];
+        }
+        for (uint32_t c = warp; P.vc2 == nullptr && c < C; c += nwarps) {
+            float e = 0.f;
             for (uint32_t j = lane; j < W; j += 32) {
-                const float v = V[(uint64_t)c * d.N + p + j];
-                e2 = fmaf(v, v, e2);
+                const float v = P.V[(uint64_t)c * d.N + p + j];
+                e = fmaf(v, v, e);
             }
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, off);
-            if (lane == 0) ve[c] = e2;
+            for (int off = 16; off > 0; off >>= 1) e += __shfl_xor_sync(full, e, off);
+            if (lane == 0) {
+                ve[c] = e;
+                ze[c] = 0.f;
+            }
         }
-        for (uint32_t x = threadIdx.x; x < S2; x += blockDim.x) {
-            const uint64_t xp = (uint64_t)x + p;
-            const bool inb = xp >= S && xp < (uint64_t)d.N - W + S;
-            fa[x] = inb ? ((L[(uint64_t)f * d.N + xp - S] > 0.f) ? 3 : 1) : 0;
+        // template f's shifts
+        for (uint32_t ch = warp; ch < nch; ch += nwarps) {
+            const uint32_t x = ch * 32 + lane;
+            const bool in = x >= xlo && x < xhi;
+            const float g = in ? Gk[(uint64_t)f * S2 + x] : -INFINITY;
+            const bool pos = in && P.L[(uint64_t)f * d.N + p + x - S] > 0.f;
+            const uint32_t bits = __ballot_sync(full, pos);
+            const float m = warp_max(pos ? -INFINITY : g);
+            Gf[x] = g;
+            if (lane == 0) {
+                pb[(size_t)f * nch + ch] = bits;
+                afch[ch] = m;
+            }
         }
-        for (uint32_t t = threadIdx.x; t < M; t += blockDim.x) nx[t] = mx[(uint64_t)f * M + t];
         if (threadIdx.x == 0) {
-            sh.best = 0ull;
+            sh.lb = 0;
             sh.nrows = 0;
-            sh.ncand = 0;
-            sh.gfull = 0;
+            sh.nchunks = 0;
+            sh.full = 0;
+            sh.best = 0ull;
         }
         __syncthreads();
-        for (uint32_t t = threadIdx.x; t < M; t += blockDim.x) {
-            const unsigned long long mt = chmask[t];   // all ones above 64 channels
-            float e2 = 0.f, z2 = 0.f;
-            uint32_t n = 0;
-            for (uint32_t c = 0; c < d.C; ++c)
-                if (c >= 64 || ((mt >> c) & 1ull)) {
-                    e2 += ve[c];
-                    if (pair) z2 += vc2[(size_t)kp * d.C + c];
-                    ++n;
-                }
-            nvt[t] = sqrtf(e2) * 1.001f;
-            mft[t] = vc2 == nullptr ? 0.f
-                                    : 1.05f * u * (kFftTerms + 3.f * n) * mx[(size_t)M * M + t] * sqrtf(e2 + z2) * 1.001f;
-        }
-        __syncthreads();
-        const float nvf = nvt[f];
-        float ma2 = -INFINITY;
-        for (uint32_t x = threadIdx.x; x < S2; x += blockDim.x) {
-            const float2 ea = Etab[(uint64_t)f * S2 + x];
-            const float al = fmaf(K, fmaf(nvf, ea.y, ea.x), mft[f]);
-            const float g = Gk[(uint64_t)f * S2 + x];
-            const uint8_t fl = fa[x];
-            const float au = (fl & 1) ? g + al : -INFINITY, alo = (fl & 1) ? g - al : -INFINITY;
-            Au[x] = au;
-            Al[x] = alo;
-            Au2[x] = fl == 1 ? au : -INFINITY;
-            Al2[x] = fl == 1 ? alo : -INFINITY;
-            if (fl == 1) ma2 = fmaxf(ma2, au);
-        }
-#pragma unroll 4
-        for (uint32_t e = threadIdx.x; e < M * S2; e += blockDim.x) {
-            const uint32_t t = e / S2, x = e - t * S2;
-            const uint64_t xp = (uint64_t)x + p;
-            const bool inb = xp >= S && xp < (uint64_t)d.N - W + S;
-            const float2 eb = Etab[e];
-            const float be = fmaf(K, fmaf(nvt[t], eb.y, eb.x), mft[t]);
-            const float g = Gk[e];
-            Bu[e] = inb ? g + be : -INFINITY;
-            Bl[e] = inb ? g - be : -INFINITY;
-            pt[e] = (inb && L[(uint64_t)t * d.N + xp - S] > 0.f) ? 1 : 0;
-        }
         {
-            const float m2 = RF(tmp.rf).Reduce(ma2, cub::Max());
-            if (threadIdx.x == 0) sh.maxau2 = m2;
+            const unsigned long long mf = P.chmask[f];
+            const MarginPart pf = margin_part(P, f, ve, ze);
+            for (uint32_t t = threadIdx.x; t < M; t += blockDim.x) {
+                const unsigned long long mt = P.chmask[t];
+                const uint32_t U = C > 64 ? C : (uint32_t)__popcll((long long)(mf | mt));
+                cst[t] = pair_margin(d, pf, margin_part(P, t, ve, ze), U);
+                nx[t] = P.mx[(uint64_t)f * M + t];
+                share[t] = (mf & mt) != 0ull;
+            }
         }
-        __syncthreads();   // Bu/Bl (global scratch too: the block's own writes) visible
+        if (warp == nwarps - 1) {   // A+ in ascending order, and the a in A+ with the largest G_f
+            uint32_t n = 0, ba = 0;
+            float bg = -INFINITY;
+            for (uint32_t ch = 0; ch < nch; ++ch) {
+                const uint32_t bits = pb[(size_t)f * nch + ch];
+                if ((bits >> lane) & 1u) {
+                    const uint32_t at = n + __popc(bits & below);
+                    alist[at] = ch * 32 + lane;
+                    if (Gf[ch * 32 + lane] > bg) {
+                        bg = Gf[ch * 32 + lane];
+                        ba = at;
+                    }
+                }
+                n += __popc(bits);
+            }
+            const float top = warp_max(bg);
+            const uint32_t who = __ballot_sync(full, bg == top);
+            ba = __shfl_sync(full, ba, __ffs(who | 0x80000000u) - 1);
+            if (lane == 0) {
+                sh.nA = n;
+                sh.top = n ? ba : 0u;
+            }
+        }
+        __syncthreads();
+        float maxaf = -INFINITY;   // largest G_f(a), a not in A+
+        for (uint32_t ch = 0; ch < nch; ++ch) maxaf = fmaxf(maxaf, afch[ch]);
+        // every template's shifts, a warp per template: chunk maxima, signs, rows (t, b)
         for (uint32_t t = warp; t < M; t += nwarps) {
-            float m = -INFINITY;
-            for (uint32_t x = lane; x < S2; x += 32) m = fmaxf(m, Bu[(uint64_t)t * S2 + x]);
+            const float* gt = Gk + (uint64_t)t * S2;
+            const float* lt = P.L + (uint64_t)t * d.N + p - S;   // lt[x], x in bounds, lies in the row
+            const float room = (nx[t] + cst[t]) + maxaf;
+            float gm = -INFINITY;
+            for (uint32_t c0 = 0; c0 < nch; c0 += 8) {
+                float g[8], lv[8];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-            if (lane == 0) gmaxu[t] = m;
-        }
-        // A+ list in ascending order
-        {
-            uint32_t base = 0;
-            for (uint32_t x0 = 0; x0 < S2; x0 += blockDim.x) {
-                const uint32_t x = x0 + threadIdx.x;
-                const uint32_t fl = (x < S2 && fa[x] == 3) ? 1u : 0u;
-                uint32_t off, tot;
-                SC(tmp.sc).ExclusiveSum(fl, off, tot);
-                if (fl) alist[base + off] = x;
-                base += tot;
-                __syncthreads();
-            }
-            if (threadIdx.x == 0) sh.nA = base;
-        }
-        __syncthreads();
-        const uint32_t nA = sh.nA;
-        const float maxau2 = sh.maxau2;
-        const uint32_t rows1 = nA * M, rows_all = rows1 + M * S2;
-        // row r -> bound of every item in it (phase B), and its scan description
-        auto row_bound = [&](uint32_t r) -> float {
-            if (r < rows1) {
-                const uint32_t t = r % M;
-                return (Au[alist[r / M]] + gmaxu[t]) + nx[t];
-            }
-            const uint32_t e = r - rows1;
-            if (!pt[e]) return -INFINITY;
-            return (Bu[e] + maxau2) + nx[e / S2];
-        };
-        auto describe = [&](uint32_t r, ScreenRow& R) {
-            if (r < rows1) {
-                const uint32_t a = alist[r / M], t = r % M;
-                R.fixed_a = true;
-                R.t = t;
-                R.y = a;
-                R.uf = Au[a];
-                R.lf = Al[a];
-                R.ua = Bu + (size_t)t * S2;
-                R.la = Bl + (size_t)t * S2;
-                R.xr = (mf & chmask[t]) ? XT + (((uint64_t)f * M + t) * S2 + a) * S2 : nullptr;
-            } else {
-                const uint32_t e = r - rows1, t = e / S2, b = e - t * S2;
-                R.fixed_a = false;
-                R.t = t;
-                R.y = b;
-                R.uf = Bu[e];
-                R.lf = Bl[e];
-                R.ua = Au2;
-                R.la = Al2;
-                R.xr = (mf & chmask[t]) ? XTT + (((uint64_t)f * M + t) * S2 + b) * S2 : nullptr;
-            }
-            R.lo = max(0, (int)R.y - (int)W);
-            R.hi = min((int)S2, (int)R.y + (int)W + 1);
-        };
-        // scan of up to two rows by one warp: cross terms of both rows loaded
-        // together, then (listing == false) LB/UB maxima, or (listing) candidates
-        auto scan2 = [&](const ScreenRow (&R)[2], bool listing, float thr, float (&lbm)[2], float (&ubm)[2]) {
-            const int span = max(R[0].hi - R[0].lo, R[1].hi - R[1].lo);
-            for (int c0 = 0; c0 < span; c0 += 32 * kScanQ) {
-                float xv[2][kScanQ];
+                for (uint32_t q = 0; q < 8; ++q) {
+                    const uint32_t x = (c0 + q) * 32 + lane;
+                    const bool in = x >= xlo && x < xhi;   // false past the last chunk
+                    g[q] = in ? gt[x] : -INFINITY;
+                    lv[q] = in ? lt[x] : 0.f;
+                }
+                float mine = -INFINITY;
+                uint32_t bits = 0;
 #pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int q = 0; q < kScanQ; ++q) {
-                        const int x = R[i].lo + c0 + (int)lane + 32 * q;
-                        xv[i][q] = (x < R[i].hi && R[i].xr) ? __ldg(R[i].xr + x) : 0.f;
+                for (uint32_t q = 0; q < 8; ++q) {
+                    if (c0 + q >= nch) break;
+                    const float m = warp_max(g[q]);
+                    const uint32_t b = __ballot_sync(full, lv[q] > 0.f);
+                    gm = fmaxf(gm, m);
+                    if (lane == q) {
+                        mine = m;
+                        bits = b;
                     }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-#pragma unroll
-                    for (int q = 0; q < kScanQ; ++q) {
-                        const int x = R[i].lo + c0 + (int)lane + 32 * q;
-                        if (x >= R[i].hi) continue;
-                        const float ub = (R[i].uf + R[i].ua[x]) - xv[i][q];
-                        if (!listing) {
-                            const float lb = (R[i].lf + R[i].la[x]) - xv[i][q];
-                            lbm[i] = fmaxf(lbm[i], lb);
-                            ubm[i] = fmaxf(ubm[i], ub);
-                            continue;
-                        }
-                        if (!(ub >= thr)) continue;
-                        const uint32_t a = R[i].fixed_a ? R[i].y : (uint32_t)x;
-                        const uint32_t b = R[i].fixed_a ? (uint32_t)x : R[i].y;
-                        const uint32_t slot = atomicAdd(&sh.ncand, 1u);
-                        if (slot < (uint32_t)kCandCap) {
-                            cand[3 * slot] = a;
-                            cand[3 * slot + 1] = R[i].t;
-                            cand[3 * slot + 2] = b;
-                        } else {
-                            const uint32_t g = atomicAdd(&status->cand_count, 1u);
-                            if (g < gcand_cap)
-                                gcand[g] = ((unsigned long long)kk << 32) | ((unsigned long long)R[i].t << 20) |
-                                           ((unsigned long long)a << 10) | (unsigned long long)b;
-                            else
-                                sh.gfull = 1;
-                        }
+                    if (b == 0u) continue;
+                    const uint32_t keep = __ballot_sync(full, lv[q] > 0.f && g[q] + room >= thr0);
+                    if (keep == 0u) continue;
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(&sh.nrows, (uint32_t)__popc(keep));
+                    at = __shfl_sync(full, at, 0) + __popc(keep & below);
+                    if (((keep >> lane) & 1u) && at < kRowCap) {
+                        rowc[at] = (1u << 22) | (t << 10) | ((c0 + q) * 32 + lane);
+                        rowg[at] = g[q];
                     }
                 }
+                if (lane < 8 && c0 + lane < nch) {
+                    gch[(size_t)t * nch + c0 + lane] = mine;
+                    pb[(size_t)t * nch + c0 + lane] = bits;
+                }
             }
-        };
-        // ---- phase B: row bounds, keep rows that can reach the seed
-        for (uint32_t r = threadIdx.x; r < rows_all; r += blockDim.x) {
-            const float ub = row_bound(r);
-            if (!(ub >= thr0)) continue;
-            const uint32_t slot = atomicAdd(&sh.nrows, 1u);
-            if (slot < (uint32_t)kRowCap) { rows[slot] = r; rowmax[slot] = ub; }
+            if (lane == 0) gmax[t] = gm;
         }
         __syncthreads();
-        uint32_t nrows = sh.nrows;
-        const bool overflow = nrows > (uint32_t)kRowCap;
-        if (overflow) nrows = rows_all;
-        // ---- phase B2: a quick lower bound from the highest-bound row of each
-        // warp's share, then keep only rows whose bound reaches it
-        float lb = -INFINITY;
-        if (!overflow && nrows > 0) {
-            float bu = -INFINITY;
-            uint32_t bi = 0xFFFFFFFFu;
-            for (uint32_t i = warp + nwarps * lane; i < nrows; i += nwarps * 32)
-                if (rowmax[i] > bu) { bu = rowmax[i]; bi = i; }
+        // estimate of this lane's item in chunk ch of a row; -inf: no such item
+        auto item = [&](uint32_t row, float g, uint32_t ch) -> float {
+            const uint32_t y = row & 1023u, t = (row >> 10) & 4095u, x = ch * 32 + lane;
+            const bool k1 = (row >> 22) != 0u;
+            bool ok = x >= xlo && x < xhi && x + W >= y && x <= y + W;
+            if (k1) ok = ok && !((pb[(size_t)f * nch + ch] >> lane) & 1u);
+            const float v = !ok ? 0.f : (k1 ? Gf[x] : Gk[(uint64_t)t * S2 + x]);
+            const float xv = ok && share[t] ? __ldg((k1 ? P.XTT : P.XT) + (((uint64_t)f * M + t) * S2 + y) * S2 + x) : 0.f;
+            return ok ? (g + v) - xv : -INFINITY;
+        };
+        auto lower = [&]() { return fmaxf(__int_as_float(*(volatile int*)&sh.lb), thr0); };
+        uint32_t nq = 0;   // chunks in this warp's queue
+        // evaluates the queue's last (up to) eight chunks
+        auto drain8 = [&]() {
+            const uint32_t n = min(nq, 8u), b = nq - n;
+            nq = b;
+            evals += n;
+            float v[8];
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ou = __shfl_xor_sync(0xffffffffu, bu, off);
-                const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, off);
-                if (ou > bu || (ou == bu && oi < bi)) { bu = ou; bi = oi; }
+            for (uint32_t i = 0; i < 8; ++i)
+                v[i] = i < n ? item(qc[b + i] & 0x7FFFFFu, qg[b + i], qc[b + i] >> 23) : -INFINITY;
+            float m = -INFINITY;   // lane i < n: chunk i's largest estimate
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                const float w = warp_max(v[i]);
+                if (lane == i) m = w;
             }
-            if (bi != 0xFFFFFFFFu) {
-                ScreenRow R[2];
-                describe(rows[bi], R[0]);
-                R[1].lo = R[1].hi = 0;
-                float lbm[2] = {-INFINITY, -INFINITY}, ubm[2] = {-INFINITY, -INFINITY};
-                scan2(R, false, 0.f, lbm, ubm);
-                lb = lbm[0];
+            const uint32_t code = lane < n ? qc[b + lane] : 0u;
+            const float c = cst[(code >> 10) & 4095u];
+            const float lb = warp_max(lane < n ? m - c : -INFINITY);
+            if (lane == 0 && lb > __int_as_float(*(volatile int*)&sh.lb)) atomicMax(&sh.lb, __float_as_int(lb));
+            if (lane < n && m + c >= fmaxf(lb, lower())) {
+                const uint32_t at = atomicAdd(&sh.nchunks, 1u);
+                if (at < kChunkCap) {
+                    chc[at] = code;
+                    chu[at] = m + c;
+                    chg[at] = qg[b + lane];
+                }
             }
-        }
-        {
-            const float lb1 = RF(tmp.rf).Reduce(lb, cub::Max());
-            if (threadIdx.x == 0) sh.lb = lb1;
+            __syncwarp();
+        };
+        // Batches of 32 rows, one a lane: first the rows (a, t) of the largest G_f(a), over all
+        // warps, then the other rows (a in A+, t), then the rows (t, b) with L_t(b) > 0, from
+        // their list or, if they are more than it holds, word by word of the signs.  One
+        // place in the code for all of them: copies of the evaluation overrun the
+        // instruction cache (17 of 29 cycles per instruction waiting for it).
+        const uint32_t nA = sh.nA, top = sh.top, nrow0 = nA * M, nrow1 = sh.nrows, ntask = M * nch;
+        const bool listed = nrow1 <= kRowCap;
+        const uint32_t n0 = (nrow0 + 31) / 32, n1 = listed ? (nrow1 + 31) / 32 : ntask;
+#pragma unroll 1
+        for (uint32_t phase = 0; phase < 2; ++phase) {
+            const uint32_t last = phase ? n0 + n1 : (nA ? (M + 31) / 32 * nwarps : 0u);
+#pragma unroll 1
+            for (uint32_t i = warp; i < last; i += nwarps) {
+                float ub = -INFINITY, g = 0.f;
+                uint32_t row = 0;
+                if (phase == 0 || i < n0) {
+                    const uint32_t r = i * 32 + lane, ai = phase ? r / M : top;
+                    const uint32_t t = phase ? r - ai * M : warp + nwarps * (lane + 32 * (i / nwarps));
+                    if (phase ? (r < nrow0 && ai != top) : t < M) {
+                        const uint32_t a = alist[ai];
+                        g = Gf[a];
+                        row = (t << 10) | a;
+                        ub = ((g + gmax[t]) + nx[t]) + cst[t];
+                    }
+                } else if (listed) {
+                    const uint32_t r = (i - n0) * 32 + lane;
+                    if (r < nrow1) {
+                        row = rowc[r];
+                        g = rowg[r];
+                        const uint32_t t = (row >> 10) & 4095u;
+                        ub = ((g + maxaf) + nx[t]) + cst[t];
+                    }
+                } else {
+                    const uint32_t e = i - n0, t = e / nch, x = (e - t * nch) * 32 + lane;
+                    if ((pb[e] >> lane) & 1u) {
+                        g = Gk[(uint64_t)t * S2 + x];
+                        row = (1u << 22) | (t << 10) | x;
+                        ub = ((g + maxaf) + nx[t]) + cst[t];
+                    }
+                }
+                // the chunks that reach the lower bound, of the rows that do
+                const float need = lower();
+                const bool want = ub >= need;
+                const uint32_t y = row & 1023u, t = (row >> 10) & 4095u;
+                const bool k1 = (row >> 22) != 0u;
+                const float* xc = k1 ? P.XCT + (((uint64_t)f * M + t) * S2 + y) * nch
+                                     : P.XC + (((uint64_t)f * S2 + y) * M + t) * nch;
+                const float* gm = k1 ? afch : gch + (size_t)t * nch;
+                const bool sharing = want && share[t];
+                const float gc = want ? g + cst[t] : -INFINITY;
+                const uint32_t c1 = __any_sync(full, want) ? nch : 0u;
+                const bool closing = i + nwarps >= last;   // this warp's last batch: empty the queue
+                for (uint32_t c0 = 0; c0 < c1 || (closing && c0 == 0); c0 += 8) {
+                    float xv[8];
+                    uint32_t km = 0;
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q) xv[q] = sharing && c0 + q < nch ? __ldg(xc + c0 + q) : 0.f;
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q)
+                        if (c0 + q < nch && (gm[c0 + q] + xv[q]) + gc >= need) km |= 1u << q;
+                    uint32_t any = __reduce_or_sync(full, km);
+                    const bool end = closing && c0 + 8 >= c1;
+                    do {
+                        if (any) {
+                            const uint32_t q = __ffs(any) - 1;
+                            any &= any - 1;
+                            const bool mine = (km >> q) & 1u;
+                            const uint32_t pm = __ballot_sync(full, mine), at = nq + __popc(pm & below);
+                            if (mine) {
+                                qc[at] = ((c0 + q) << 23) | row;
+                                qg[at] = g;
+                            }
+                            nq += __popc(pm);
+                            __syncwarp();
+                        }
+                        // evaluate while the queue has no room for 32 more, or at the end
+                        while (nq > (end && any == 0u ? 0u : kQueue - 32u)) drain8();
+                    } while (any);
+                }
+            }
             __syncthreads();
-            const float thr1 = fmaxf(sh.lb, thr0);
-            if (!overflow) {
-                // compact the rows reaching thr1 (order kept), reusing the row arrays in place
-                uint32_t base = 0;
-                for (uint32_t i0 = 0; i0 < nrows; i0 += blockDim.x) {
-                    const uint32_t i = i0 + threadIdx.x;
-                    const bool keep = i < nrows && rowmax[i] >= thr1;
-                    const uint32_t r = keep ? rows[i] : 0u;
-                    uint32_t off, tot;
-                    SC(tmp.sc).ExclusiveSum(keep ? 1u : 0u, off, tot);
-                    __syncthreads();
-                    if (keep) rows[base + off] = r;
-                    base += tot;
-                    __syncthreads();
-                }
-                nrows = base;
-            }
         }
-        // a kept row (or, after an overflow, any row whose bound reaches thr),
-        // else an empty range
-        auto describe_kept = [&](uint32_t i, float thr, bool use_rowmax, ScreenRow& R) {
-            R.lo = R.hi = 0;
-            if (i >= nrows) return;
-            const uint32_t r = overflow ? i : rows[i];
-            if (overflow ? !(row_bound(r) >= thr) : (use_rowmax && !(rowmax[i] >= thr))) return;
-            describe(r, R);
+        // the list of chunks too small for this window: look at every item instead
+        const bool over = sh.nchunks > kChunkCap;
+        const uint32_t nchunks = over ? 0u : sh.nchunks;
+        // every item of the window, row by row: visit(row, chunk, estimates)
+        auto every = [&](auto&& visit) {
+            for (uint32_t r = warp; r < nA * M; r += nwarps) {
+                const uint32_t ai = r / M, t = r - ai * M, a = alist[ai];
+                for (uint32_t ch = 0; ch < nch; ++ch) visit((t << 10) | a, ch, item((t << 10) | a, Gf[a], ch));
+            }
+            for (uint32_t e = warp; e < ntask; e += nwarps) {
+                const uint32_t t = e / nch;
+                for (uint32_t bits = pb[e]; bits; bits &= bits - 1) {
+                    const uint32_t b = (e - t * nch) * 32 + __ffs(bits) - 1, row = (1u << 22) | (t << 10) | b;
+                    const float g = Gk[(uint64_t)t * S2 + b];
+                    for (uint32_t ch = 0; ch < nch; ++ch) visit(row, ch, item(row, g, ch));
+                }
+            }
         };
-        // ---- phase C: lower bound and per-row upper bounds, two rows per warp at a time
-        {
-            uint64_t scanned = 0;
-            for (uint32_t i = 2 * warp; i < nrows; i += 2 * nwarps) {
-                ScreenRow R[2];
-                describe_kept(i, thr0, false, R[0]);
-                describe_kept(i + 1, thr0, false, R[1]);
-                scanned += (uint64_t)(R[0].hi - R[0].lo) + (uint64_t)(R[1].hi - R[1].lo);
-                float lbm[2] = {-INFINITY, -INFINITY}, ubm[2] = {-INFINITY, -INFINITY};
-                scan2(R, false, 0.f, lbm, ubm);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    float m = ubm[q];
-#pragma unroll
-                    for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-                    ubm[q] = m;
-                    lb = fmaxf(lb, lbm[q]);
-                }
-                if (!overflow && lane == 0) {
-                    rowmax[i] = ubm[0];
-                    if (i + 1 < nrows) rowmax[i + 1] = ubm[1];
-                }
-            }
-            if (lane == 0) item_n += scanned;
-        }
-        const float lbs = RF(tmp.rf).Reduce(lb, cub::Max());
-        if (threadIdx.x == 0) sh.lb = lbs;
-        __syncthreads();
-        const float thr = fmaxf(fmaxf(sh.lb, seed), 0.f);
-        // ---- phase D: candidate list from the rows reaching thr, two per warp at a time
-        for (uint32_t i = 2 * warp; i < nrows; i += 2 * nwarps) {
-            ScreenRow R[2];
-            describe_kept(i, thr, true, R[0]);
-            describe_kept(i + 1, thr, true, R[1]);
-            if (R[0].hi == R[0].lo && R[1].hi == R[1].lo) continue;
-            float lbm[2], ubm[2];
-            scan2(R, true, thr, lbm, ubm);
-        }
-        __syncthreads();
-        const uint32_t ncand = sh.ncand;
+        const float thr = fmaxf(__int_as_float(sh.lb), thr0);
+        // list the items that reach it; where the global list is full, score them here
         unsigned long long kbest = 0ull;
-        // hand the listed candidates to the scoring kernel (the listing already
-        // spilled past kCandCap straight into the global list)
-        const uint32_t nlisted = min(ncand, (uint32_t)kCandCap);
-        if (threadIdx.x == 0) s_gbase = atomicAdd(&status->cand_count, nlisted);
-        __syncthreads();
-        const uint32_t gbase = s_gbase;
-        const bool handed = (uint64_t)gbase + nlisted <= gcand_cap && !sh.gfull;
-        if (handed) {
-            for (uint32_t i = threadIdx.x; i < nlisted; i += blockDim.x)
-                gcand[gbase + i] = ((unsigned long long)kk << 32) | ((unsigned long long)cand[3 * i + 1] << 20) |
-                                   ((unsigned long long)cand[3 * i] << 10) | (unsigned long long)cand[3 * i + 2];
-        } else {
-            // the global list is full: mark this window's slots in it empty and
-            // score every item of the reaching rows here
-            for (uint64_t i = (uint64_t)gbase + threadIdx.x; i < gcand_cap && i < (uint64_t)gbase + nlisted;
-                 i += blockDim.x)
-                gcand[i] = ~0ull;
-            for (uint32_t i = threadIdx.x; i < nrows; i += blockDim.x) {
-                const uint32_t r = overflow ? i : rows[i];
-                if (!(row_bound(r) >= thr)) continue;
-                ScreenRow R;
-                describe(r, R);
-                for (int x = R.lo; x < R.hi; ++x) {
-                    const float xv = R.xr ? R.xr[x] : 0.f;
-                    const float ub = (R.uf + R.ua[x]) - xv;
-                    if (!(ub >= thr)) continue;
-                    const uint32_t a = R.fixed_a ? R.y : (uint32_t)x, b = R.fixed_a ? (uint32_t)x : R.y;
-                    const float v = pair_exact_g(d, T, V, f, R.t, p, a, b, mf | chmask[R.t]);
-                    ++exact_n;
-                    if (!(v > 0.f)) continue;
-                    const uint64_t rr0 = (uint64_t)R.t + (uint64_t)M * a + (uint64_t)M * S2 * b;
-                    uint32_t pr = item_priority(rr0, d.WG, lbits);
-                    for (uint64_t rr = rr0 + items; rr < slots; rr += items) {
-                        const uint32_t p2 = item_priority(rr, d.WG, lbits);
-                        pr = p2 < pr ? p2 : pr;
-                    }
-                    const unsigned long long key =
-                        ((unsigned long long)__float_as_uint(v) << 32) | (unsigned long long)(0xFFFFFFFFu - pr);
-                    kbest = key > kbest ? key : kbest;
-                }
+        auto list_items = [&](uint32_t row, uint32_t ch, float est, bool here) {
+            const uint32_t y = row & 1023u, t = (row >> 10) & 4095u, x = ch * 32 + lane;
+            const bool k1 = (row >> 22) != 0u;
+            const bool reach = est + cst[t] >= thr;
+            const uint32_t m = __ballot_sync(full, reach);
+            if (m == 0u) return;
+            const uint32_t a = k1 ? x : y, b = k1 ? y : x;
+            if (!here) {
+                uint32_t base = 0;
+                if (lane == 0) base = atomicAdd(&P.status->cand_count, (uint32_t)__popc(m));
+                const uint32_t at = __shfl_sync(full, base, 0) + __popc(m & ((1u << lane) - 1u));
+                if (!reach) return;
+                if (at < P.cand_cap)
+                    P.gcand[at] = ((unsigned long long)kk << 32) | ((unsigned long long)t << 20) |
+                                  ((unsigned long long)a << 10) | (unsigned long long)b;
+                else
+                    sh.full = 1;
+                return;
             }
+            if (!reach) return;
+            const float v = pair_exact_call(d, P.T, P.V, f, t, p, a, b, P.chmask[f] | P.chmask[t]);
+            if (!(v > 0.f)) return;
+            const uint64_t r0 = (uint64_t)t + (uint64_t)M * a + (uint64_t)M * S2 * b;
+            uint32_t pr = item_priority(r0, d.WG, lbits);
+            for (uint64_t rr = r0 + items; rr < slots; rr += items) pr = min(pr, item_priority(rr, d.WG, lbits));
+            const unsigned long long key =
+                ((unsigned long long)__float_as_uint(v) << 32) | (unsigned long long)(0xFFFFFFFFu - pr);
+            kbest = key > kbest ? key : kbest;
+        };
+        auto list_window = [&](bool here) {
+            if (over) {
+                every([&](uint32_t row, uint32_t ch, float est) {
+                    list_items(row, ch, est, here);
+                    __syncwarp();
+                });
+                return;
+            }
+            for (uint32_t e = warp; e < nchunks; e += nwarps) {
+                if (!(chu[e] >= thr)) continue;
+                const uint32_t row = chc[e] & 0x7FFFFFu, ch = chc[e] >> 23;
+                list_items(row, ch, item(row, chg[e], ch), here);
+                __syncwarp();
+            }
+        };
+#pragma unroll 1
+        for (int here = 0; here < 2; ++here) {
+            list_window(here != 0);
+            __syncthreads();
+            if (!sh.full) break;   // the same for the whole CTA
+            if (!here) continue;
+            if (kbest) atomicMax(&sh.best, kbest);
+            __syncthreads();
+            if (threadIdx.x == 0 && sh.best) atomicMax(&P.keys[P.k0 + kk], sh.best);
         }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const unsigned long long o = __shfl_down_sync(0xffffffffu, kbest, off);
-            kbest = o > kbest ? o : kbest;
-        }
-        if (lane == 0 && kbest) atomicMax(&sh.best, kbest);
-        __syncthreads();
-        if (threadIdx.x == 0 && sh.best) keys[k] = sh.best;
     }
-    if (exact_n) atomicAdd(&status->n_pair_exact, (uint32_t)exact_n);
-    if (item_n) atomicAdd(&status->pair_items, item_n);
+    if (lane == 0 && evals) atomicAdd(&P.status->pair_items, 32ull * evals);
 }
 
 // Screening order of a batch of flagged windows: grouped by best label f (a
@@ -923,25 +993,29 @@ int launch_overlap_tables(const Dims& d, const Work& w, const float* T, cudaStre
 {
     const Layout& L = *w.lay;
     if (!L.screened) return FBP_OK;
-    const uint32_t S2 = 2 * d.S + 1;
-    count_launch(4);
-    energy_table_kernel<<<(d.M * S2 + 255) / 256, 256, 0, st>>>(d, T, w.at<float2>(L.off_et));
-    const size_t smem = (size_t)2 * d.C * d.W * 4 + 8 + (size_t)kLagChunk * (d.W + 1) * 8;
-    if (smem > 200 * 1024) return fail(FBP_E_ARG, "template too large for the pair table kernel");
+    const unsigned long long* chmask = w.at<unsigned long long>(L.off_tchm);
+    float* mx = w.at<float>(L.off_mx);
+    count_launch(2);
+    energy_table_kernel<<<d.M, 128, (d.W + 1) * 8, st>>>(d, T, w.at<float2>(L.off_et), mx + (size_t)d.M * d.M);
+    auto cross_smem = [&](int lags) { return (size_t)2 * d.C * d.W * 4 + (size_t)lags * ((d.W + 1) | 1u) * 8; };
+    const int lags = cross_smem(32) <= 100 * 1024 ? 32 : 16;   // two CTAs per SM, or the shorter chunk
+    if (cross_smem(lags) > 201 * 1024) return fail(FBP_E_ARG, "template too large for the pair table kernel");
     FBP_CUDA(allow_max_dyn_smem(cross_table_kernel));
-    cross_table_kernel<<<d.M * d.M, 256, smem, st>>>(d, T, w.at<float>(L.off_xt), w.at<float>(L.off_xtt),
-                                                     w.at<float>(L.off_mx));
-    energy_max_kernel<<<(d.M + 127) / 128, 128, 0, st>>>(d, w.at<float2>(L.off_et), w.at<float>(L.off_mx) + (size_t)d.M * d.M);
-    template_order_kernel<<<1, 256, d.M * 4, st>>>(d, T, w.at<uint32_t>(L.off_perm),
-                                                  reinterpret_cast<unsigned long long*>(w.at<uint32_t>(L.off_perm) + ((d.M + 1) & ~1u)));
+    cross_table_kernel<<<d.M * d.M, kCrossThreads, cross_smem(lags), st>>>(
+        d, T, chmask, lags, w.at<float>(L.off_xt), w.at<float>(L.off_xtt), w.at<float>(L.off_xc), w.at<float>(L.off_xct),
+        mx);
     FBP_CUDA(cudaGetLastError());
-    // channel unions of the template groups decide how many templates a
+    if (window_corr_by_fft(d)) return FBP_OK;
+    count_launch();
+    template_order_kernel<<<1, 256, d.M * 4, st>>>(d, w.at<uint8_t>(L.off_clist), w.at<uint32_t>(L.off_ccnt),
+                                                  w.at<uint32_t>(L.off_perm));
+    FBP_CUDA(cudaGetLastError());
+    // channel unions of the template groups decide how many templates a direct
     // partial-correlation CTA can stage: read the order and masks back once
     std::vector<uint32_t> perm(d.M);
     std::vector<unsigned long long> mask(d.M);
     FBP_CUDA(cudaMemcpyAsync(perm.data(), w.at<uint32_t>(L.off_perm), d.M * 4, cudaMemcpyDeviceToHost, st));
-    FBP_CUDA(cudaMemcpyAsync(mask.data(), w.at<uint32_t>(L.off_perm) + ((d.M + 1) & ~1u), d.M * 8,
-                             cudaMemcpyDeviceToHost, st));
+    FBP_CUDA(cudaMemcpyAsync(mask.data(), chmask, d.M * 8, cudaMemcpyDeviceToHost, st));
     FBP_CUDA(cudaStreamSynchronize(st));
     PcConfig& pc = pc_config();
     pc.Q = 0;
@@ -995,24 +1069,47 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
     const size_t smem_a = pc.smem;
     const bool fft = window_corr_by_fft(d);
     if (Q == 0 && !fft) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
-    float* vc2 = fft ? w.at<float>(L.off_vc2) : nullptr;
     const uint32_t pc_threads = 32u * std::min<uint32_t>((S2 + 15) / 16, kPcMaxWarps);
-    const bool bstaged = (uint64_t)d.M * S2 * 8 <= kBStage;
-    const size_t smem_b = screen_smem_bytes(d.M, S2, bstaged);
+    const size_t smem_b = screen_smem_bytes(d.M, S2, d.C);
     if (smem_b > 200 * 1024) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
     FBP_CUDA(allow_max_dyn_smem(screen_kernel));
-    const uint32_t groups = (d.M + Q - 1) / Q;
+    int scr_per_sm = 1;
+    FBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scr_per_sm, screen_kernel, kScrThreads, smem_b));
+    const uint32_t groups = Q > 0 ? (d.M + Q - 1) / Q : 0u;
     float* G = w.at<float>(L.off_g);
     const float2* Et = w.at<float2>(L.off_et);
-    const float* XT = w.at<float>(L.off_xt);
     const uint32_t* perm = w.at<uint32_t>(L.off_perm);
-    const unsigned long long* chm = reinterpret_cast<const unsigned long long*>(perm + ((d.M + 1) & ~1u));
+    const unsigned long long* chm = w.at<unsigned long long>(L.off_tchm);
+    ScreenArgs P;
+    P.d = d;
+    P.V = V;
+    P.T = T;
+    P.L = w.L();
+    P.theta = theta;
+    P.XT = w.at<float>(L.off_xt);
+    P.XTT = w.at<float>(L.off_xtt);
+    P.XC = w.at<float>(L.off_xc);
+    P.XCT = w.at<float>(L.off_xct);
+    P.mx = w.at<float>(L.off_mx);
+    P.G = G;
+    P.vc2 = fft ? w.at<float>(L.off_vc2) : nullptr;
+    P.z2 = fft ? w.at<float>(L.off_z2) : nullptr;
+    P.flag = w.flag();
+    P.status = w.status();
+    P.best_lab = w.best_lab();
+    P.best_idx = w.best_idx();
+    P.best_lik = w.best_lik();
+    P.keys = w.keys();
+    P.gcand = w.at<unsigned long long>(L.off_cand);
+    P.cand_cap = (uint32_t)L.cand_cap;
+    P.chmask = chm;
+    P.order = w.at<uint32_t>(L.off_order);
     for (uint32_t k0 = 0; k0 < nflag_max; k0 += (uint32_t)L.gbatch) {
         const uint32_t kc = (uint32_t)((nflag_max - k0) < L.gbatch ? (nflag_max - k0) : L.gbatch);
         count_launch(2);
         if (fft) {
         KScope ks(&fbp_chunk_stats::ms_partial_corr, st);
-        FBP_TRY(launch_window_corr(d, w, V, theta, Et, k0, kc, G, vc2, st));
+        FBP_TRY(launch_window_corr(d, w, V, theta, Et, k0, kc, G, w.at<float>(L.off_vc2), w.at<float>(L.off_z2), st));
         } else {
         KScope ks(&fbp_chunk_stats::ms_partial_corr, st);
         count_launch();
@@ -1037,21 +1134,19 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
         }
 #undef FBP_PC
         }
-        const uint32_t gb = kc < kScreenGrid ? kc : kScreenGrid;
         uint32_t* order = w.at<uint32_t>(L.off_order);
         count_launch();
         label_order_kernel<<<1, 1024, (d.M + 1) * 4, st>>>(d, w.flag(), w.status(), w.best_lab(), k0, kc, order);
         FBP_CUDA(cudaMemsetAsync(&w.status()->cand_count, 0, 4, st));
-        unsigned long long* gcand = w.at<unsigned long long>(L.off_cand);
         {
         KScope ks(&fbp_chunk_stats::ms_screen, st);
-        screen_kernel<<<gb, kScrThreads, smem_b, st>>>(d, V, T, w.L(), theta, Et, XT, w.at<float>(L.off_xtt), G, k0, kc,
-                                                       w.flag(), w.status(), w.best_lab(), w.best_idx(), w.best_lik(),
-                                                       w.keys(), w.at<float>(L.off_mx), gcand, (uint32_t)L.cand_cap, chm,
-                                                       bstaged ? nullptr : w.at<float>(L.off_bscr), order, vc2);
+        P.k0 = k0;
+        P.kc = kc;
+        const uint32_t grid = std::min<uint32_t>(kc, 148u * (scr_per_sm > 0 ? scr_per_sm : 1));
+        screen_kernel<<<grid, kScrThreads, smem_b, st>>>(P);
         }
         KScope ks(&fbp_chunk_stats::ms_score, st);
-        score_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, w.flag(), k0, w.best_lab(), w.best_idx(), gcand,
+        score_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, w.flag(), k0, w.best_lab(), w.best_idx(), P.gcand,
                                               (uint32_t)L.cand_cap, w.status(), w.keys(), chm);
         FBP_CUDA(cudaGetLastError());
     }

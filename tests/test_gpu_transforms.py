@@ -52,3 +52,35 @@ def test_pursuit_matches_oracle(case, recheck):
     assert len(want[0]) > 0
     for g, w in zip(got, want):
         assert np.array_equal(np.asarray(g), np.asarray(w)), (case, W, S)
+
+
+def _same_as_oracle(V, si, sm, S):
+    want = oracle.binary_pursuit(V, np.float32, si, copy.deepcopy(sm), n_max_shift_inds=S,
+                                 global_mem_size=183 * 1024 ** 3)
+    got = binary_pursuit(V, np.float32, si, copy.deepcopy(sm), n_max_shift_inds=S, verbose=False)
+    assert len(want[0]) > 0
+    for g, w in zip(got, want):
+        assert np.array_equal(np.asarray(g), np.asarray(w), equal_nan=True)
+
+
+def test_samples_that_are_not_numbers_stay_in_their_windows():
+    """Windows and stretches are transformed in pairs: a NaN must not reach the other one's
+    spikes.  (An infinite sample's likelihood stays infinite after every subtraction: the
+    reference's loop does not end on it, so there is nothing to compare with.)"""
+    V, si, sm, _ = synth.make_recording(29, n_chans=4, duration_s=0.4, n_units=6,
+                                        rate_model=("uniform", 30.0, 60.0), overlap_frac=0.3)
+    si["get_adjusted_clips"] = True
+    V = V.copy()
+    V[1, 5000] = np.nan
+    V[0, 9100:9104] = np.nan
+    V[3, 12345] = -np.nan
+    _same_as_oracle(V, si, sm, si["n_samples_per_chan"] - 1)
+
+
+@pytest.mark.parametrize("amp", [(6.0, 12.0), (20.0, 60.0)])
+def test_many_similar_units_on_the_same_channels(amp):
+    """More rows and chunks of items reach the bounds than the screen's lists hold."""
+    V, si, sm, _ = synth.make_recording(31, n_chans=3, fs=30000, duration_s=0.12, n_units=70,
+                                        rate_model=("uniform", 5.0, 15.0), overlap_frac=0.5, amp=amp)
+    si["get_adjusted_clips"] = True
+    _same_as_oracle(V, si, sm, si["n_samples_per_chan"] - 1)
