@@ -923,46 +923,128 @@ __global__ void __launch_bounds__(1024) label_order_kernel(Dims d, const uint32_
     }
 }
 
-// Exact scores of the listed candidates, one thread each: entry = window slot
-// kk (32 bits) | t (12) | a (10) | b (10).  Folds the canonical winner key into
-// keys[k0 + kk].
-__global__ void __launch_bounds__(256) score_kernel(Dims d, const float* __restrict__ V, const float* __restrict__ T,
-                                                    const uint32_t* __restrict__ flag, uint32_t k0,
-                                                    const uint32_t* __restrict__ best_lab,
-                                                    const uint32_t* __restrict__ best_idx,
-                                                    const unsigned long long* __restrict__ gcand, uint32_t cap,
-                                                    DevStatus* status, unsigned long long* keys,
-                                                    const unsigned long long* __restrict__ chmask)
+// Exact scores of the listed candidates, entry = window slot kk (32 bits) | t (12) |
+// a (10) | b (10), in the reference's float order (pair_exact_g).  Folds the
+// canonical winner key into keys[k0 + kk].
+//
+// A warp takes up to 16 candidates.  Channel by channel of each candidate's own
+// non-zero ones, 32 taps at a time, the lanes form the products of one candidate
+// after the other (a product rounds the same wherever it is formed) in shared memory;
+// then lane e adds candidate e's products with the window and lane 16 + e its squares,
+// one by one in tap order.  The loads of eight candidates are in flight together,
+// where a thread per candidate waited for its own at every eighth tap: per pursuit
+// 16.8 -> 2.7 ms (20 s of 64 channels x 200 templates, 0.16 M candidates in 36
+// launches), 1.04 -> 0.39 ms (43 s of 11 x 27), 0.20 -> 0.17 ms (30 s of 4 x 6); with
+// 1.2 M candidates (300 s of 16 x 40) the two are alike, 3.6 and 3.8 ms.  Fewer
+// candidates a warp when there are not enough to fill the SMs.
+constexpr int kScoreThreads = 128;
+constexpr uint32_t kScoreMany = 16;
+
+__global__ void __launch_bounds__(kScoreThreads) score_kernel(
+    Dims d, const float* __restrict__ V, const float* __restrict__ T, const uint32_t* __restrict__ flag, uint32_t k0,
+    const uint32_t* __restrict__ best_lab, const uint32_t* __restrict__ best_idx,
+    const unsigned long long* __restrict__ gcand, uint32_t cap, DevStatus* status, unsigned long long* keys,
+    const unsigned long long* __restrict__ chmask)
 {
+    __shared__ float prod[kScoreThreads / 32][2 * kScoreMany * 33];   // [kind][candidate][32 taps, padded]
+    __shared__ uint4 rows[kScoreThreads / 32][kScoreMany];            // template rows and voltage row of the channel
+    __shared__ int2 shift[kScoreThreads / 32][kScoreMany];            // first template samples
     const uint32_t n = min(status->cand_count, cap);
-    const uint32_t S2 = 2 * d.S + 1, M = d.M;
+    const uint32_t S2 = 2 * d.S + 1, M = d.M, C = d.C, W = d.W;
     const uint64_t items = (uint64_t)S2 * S2 * M;
-    const uint64_t nloc = (items - 1) / d.WG + 1;
-    const uint64_t slots = nloc * d.WG;
+    const uint64_t slots = ((items - 1) / d.WG + 1) * d.WG;
     uint32_t lbits = 0;
     while ((1u << lbits) < d.WG) ++lbits;
-    uint32_t done = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const unsigned long long e = gcand[i];
-        if (e == ~0ull) continue;
-        const uint32_t kk = (uint32_t)(e >> 32);
-        const uint32_t t = (uint32_t)(e >> 20) & 0xFFFu, a = (uint32_t)(e >> 10) & 0x3FFu, b = (uint32_t)e & 0x3FFu;
-        if ((uint64_t)k0 + kk >= status->n_flag || t >= M || a >= S2 || b >= S2) continue;
-        const uint32_t id = flag[k0 + kk];
-        const uint32_t f = best_lab[id], p = best_idx[id];
-        const float acc = pair_exact_g(d, T, V, f, t, p, a, b, chmask[f] | chmask[t]);
-        ++done;
-        if (!(acc > 0.f)) continue;
-        const uint64_t r = (uint64_t)t + (uint64_t)M * a + (uint64_t)M * S2 * b;
-        uint32_t pr = item_priority(r, d.WG, lbits);
-        for (uint64_t rr = r + items; rr < slots; rr += items) {
-            const uint32_t p2 = item_priority(rr, d.WG, lbits);
-            pr = p2 < pr ? p2 : pr;
+    const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = lane & 15u;
+    const uint32_t nwarps = gridDim.x * (kScoreThreads / 32);
+    uint32_t G = kScoreMany;
+    while (G > 2 && (n + G - 1) / G < nwarps) G >>= 1;
+    float* mine = prod[warp] + (lane >> 4) * (kScoreMany * 33) + e * 33;
+    for (uint32_t i0 = (blockIdx.x * (kScoreThreads / 32) + warp) * G; i0 < n; i0 += nwarps * G) {
+        // candidate e on lanes e and 16 + e
+        const uint32_t have = min(G, n - i0);
+        const unsigned long long code = e < have ? gcand[i0 + e] : ~0ull;
+        const uint32_t kk = (uint32_t)(code >> 32);
+        const uint32_t t = (uint32_t)(code >> 20) & 0xFFFu, a = (uint32_t)(code >> 10) & 0x3FFu, b = (uint32_t)code & 0x3FFu;
+        const bool ok = code != ~0ull && (uint64_t)k0 + kk < status->n_flag && t < M && a < S2 && b < S2;
+        uint32_t f = 0, p = 0;
+        unsigned long long left = 0ull;   // channels still to sum (C <= 64)
+        if (ok) {
+            const uint32_t id = flag[k0 + kk];
+            f = best_lab[id];
+            p = best_idx[id];
+            left = chmask[f] | chmask[t];
         }
-        atomicMax(&keys[k0 + kk],
-                  ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned long long)(0xFFFFFFFFu - pr));
+        uint32_t next = 0;                // channel (C > 64: all of them)
+        if (lane < kScoreMany) shift[warp][e] = make_int2((int)d.S - (int)a, (int)d.S - (int)b);
+        float acc = 0.f;                  // lanes < 16
+        for (;;) {
+            const bool on = ok && (C > 64 ? next < C : left != 0ull);
+            const uint32_t act = __ballot_sync(full, on) & 0xFFFFu;
+            if (act == 0u) break;
+            const uint32_t c = C > 64 ? next : (uint32_t)__ffsll((long long)left) - 1u;
+            if (on) {
+                left &= left - 1;
+                ++next;
+                if (lane < kScoreMany) {
+                    const uint64_t vo = (uint64_t)c * d.N + p;
+                    rows[warp][e] = make_uint4((f * C + c) * W, (t * C + c) * W, (uint32_t)vo, (uint32_t)(vo >> 32));
+                }
+            }
+            __syncwarp();
+            float sum = lane < kScoreMany ? acc : 0.f;
+            for (uint32_t j0 = 0; j0 < W; j0 += 32) {
+                const uint32_t j = j0 + lane;
+                for (uint32_t g0 = 0; g0 < G; g0 += 8) {
+                    if (((act >> g0) & 0xFFu) == 0u) continue;
+                    float fv[8], tv[8], vv[8];
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q) {
+                        fv[q] = tv[q] = vv[q] = 0.f;
+                        if (!((act >> (g0 + q)) & 1u)) continue;   // the same for the whole warp
+                        const uint4 r = rows[warp][g0 + q];
+                        const int2 s = shift[warp][g0 + q];
+                        const int jf = (int)j + s.x, jt = (int)j + s.y;
+                        if (j < W) {
+                            vv[q] = __ldg(V + (((uint64_t)r.w << 32) | r.z) + j);
+                            if (jf >= 0 && jf < (int)W) fv[q] = __ldg(T + r.x + jf);
+                            if (jt >= 0 && jt < (int)W) tv[q] = __ldg(T + r.y + jt);
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q) {
+                        if (!((act >> (g0 + q)) & 1u)) continue;
+                        const float sv = fadd(fv[q], tv[q]);
+                        prod[warp][(g0 + q) * 33 + lane] = fmul(sv, vv[q]);
+                        prod[warp][(kScoreMany + g0 + q) * 33 + lane] = fmul(sv, sv);
+                    }
+                }
+                __syncwarp();
+                if (on) {
+                    const uint32_t m = min(32u, W - j0);
+                    if (m == 32u) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 32; ++k) sum = fadd(sum, mine[k]);
+                    } else {
+#pragma unroll 4
+                        for (uint32_t k = 0; k < m; ++k) sum = fadd(sum, mine[k]);
+                    }
+                }
+                __syncwarp();
+            }
+            const float ss = __shfl_sync(full, sum, lane | 16u);
+            if (on && lane < kScoreMany) acc = ss > 0.f ? fsub(sum, fmul(0.5f, ss)) : sum;
+        }
+        if (ok && lane < kScoreMany && acc > 0.f) {
+            const uint64_t r = (uint64_t)t + (uint64_t)M * a + (uint64_t)M * S2 * b;
+            uint32_t pr = item_priority(r, d.WG, lbits);
+            for (uint64_t rr = r + items; rr < slots; rr += items) pr = min(pr, item_priority(rr, d.WG, lbits));
+            atomicMax(&keys[k0 + kk],
+                      ((unsigned long long)__float_as_uint(acc) << 32) | (unsigned long long)(0xFFFFFFFFu - pr));
+        }
+        const uint32_t done = __popc(__ballot_sync(full, ok) & 0xFFFFu);
+        if (lane == 0 && done) atomicAdd(&status->n_pair_exact, done);
     }
-    if (done) atomicAdd(&status->n_pair_exact, done);
 }
 
 }  // namespace
@@ -1146,7 +1228,7 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
         screen_kernel<<<grid, kScrThreads, smem_b, st>>>(P);
         }
         KScope ks(&fbp_chunk_stats::ms_score, st);
-        score_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, w.flag(), k0, w.best_lab(), w.best_idx(), P.gcand,
+        score_kernel<<<148 * 6, kScoreThreads, 0, st>>>(d, V, T, w.flag(), k0, w.best_lab(), w.best_idx(), P.gcand,
                                               (uint32_t)L.cand_cap, w.status(), w.keys(), chm);
         FBP_CUDA(cudaGetLastError());
     }
