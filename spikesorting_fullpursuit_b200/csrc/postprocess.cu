@@ -13,7 +13,7 @@
 //     over the rows in order, then divided by n (numpy's order for an axis-0
 //     reduction of a C-contiguous array).
 //   * sse_kernel: np.sum((clip - template) ** 2) in float32 with numpy's
-//     pairwise summation (blocks of at most 128 values summed with 8 partial
+//     pairwise summation (pieces of at most 128 values summed with 8 partial
 //     sums, larger ranges split in two at a multiple of 8).
 //   * The walk is sequential in the reference.  At a spike j with
 //     ev[j] - max(ev[0..j-1]) > tol no earlier spike is within tol of it, so
@@ -21,55 +21,148 @@
 //     segments, one thread each (segment_start_kernel, walk_kernel).
 #include <cub/cub.cuh>
 
+#include <algorithm>
+
 #include "fbp_internal.cuh"
+#include "pairwise.cuh"
 
 namespace fbp {
 namespace {
 
-__global__ void mean_clip_kernel(const float* __restrict__ clips, uint32_t n, uint32_t len, float* mean)
+// One thread per column; sixteen rows are in flight while their values are
+// added in row order (one row at a time a unit of 300 clips took 82 us, now 16).
+constexpr int kMeanThreads = 64;   // few columns a CTA: a unit has one or two thousand
+
+__global__ void __launch_bounds__(kMeanThreads) mean_clip_kernel(const float* __restrict__ clips, uint32_t n,
+                                                                 uint32_t len, float* mean)
 {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < len; k += gridDim.x * blockDim.x) {
-        float acc = clips[k];
-        for (uint32_t i = 1; i < n; ++i) acc = __fadd_rn(acc, clips[(uint64_t)i * len + k]);
-        mean[k] = __fdiv_rn(acc, (float)n);
+    const uint32_t k = blockIdx.x * kMeanThreads + threadIdx.x;
+    if (k >= len) return;
+    const float* x = clips + k;
+    float acc = x[0];
+    uint32_t i = 1;
+    float v[16];
+    for (; i + 16 <= n; i += 16) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = __ldg(x + (uint64_t)(i + q) * len);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) acc = __fadd_rn(acc, v[q]);
     }
+    for (; i < n; ++i) acc = __fadd_rn(acc, __ldg(x + (uint64_t)i * len));
+    mean[k] = __fdiv_rn(acc, (float)n);
 }
 
 __device__ __forceinline__ float sq_diff(const float* __restrict__ a, const float* __restrict__ b, uint32_t i)
 {
-    const float d = __fsub_rn(a[i], b[i]);
+    const float d = __fsub_rn(__ldg(a + i), __ldg(b + i));
     return __fmul_rn(d, d);
 }
 
-// numpy's pairwise sum of (a - b)^2 over [0, n)
-__device__ float pairwise_sq(const float* __restrict__ a, const float* __restrict__ b, uint32_t n)
+// Sum of (a - b)^2 over [0, n <= 128) in numpy's order by 8 lanes (lane j of the group:
+// the values j, j + 8, ... of the whole eights, combined as a tree, then the rest in
+// order); n < 8: in order.  The sum on every lane of the group.
+__device__ __forceinline__ float piece_sum(const float* __restrict__ a, const float* __restrict__ b, uint32_t n,
+                                           uint32_t j, uint32_t mask)
 {
-    if (n < 8) {
-        float res = 0.f;
-        for (uint32_t i = 0; i < n; ++i) res = __fadd_rn(res, sq_diff(a, b, i));
-        return res;
+    const uint32_t n8 = n - n % 8;
+    float r = 0.f;
+    if (n8) {
+        r = sq_diff(a, b, j);
+#pragma unroll 8
+        for (uint32_t i = 8 + j; i < n8; i += 8) r = __fadd_rn(r, sq_diff(a, b, i));
+        r = __fadd_rn(r, __shfl_xor_sync(mask, r, 1));
+        r = __fadd_rn(r, __shfl_xor_sync(mask, r, 2));
+        r = __fadd_rn(r, __shfl_xor_sync(mask, r, 4));
     }
-    if (n <= 128) {
-        float r[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) r[j] = sq_diff(a, b, j);
-        uint32_t i = 8;
-        for (; i < n - (n % 8); i += 8) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) r[j] = __fadd_rn(r[j], sq_diff(a, b, i + j));
-        }
-        float res = __fadd_rn(__fadd_rn(__fadd_rn(r[0], r[1]), __fadd_rn(r[2], r[3])),
-                              __fadd_rn(__fadd_rn(r[4], r[5]), __fadd_rn(r[6], r[7])));
-        for (; i < n; ++i) res = __fadd_rn(res, sq_diff(a, b, i));
-        return res;
-    }
-    uint32_t n2 = n / 2;
-    n2 -= n2 % 8;
-    return __fadd_rn(pairwise_sq(a, b, n2), pairwise_sq(a + n2, b + n2, n - n2));
+    for (uint32_t i = n8; i < n; ++i) r = __fadd_rn(r, sq_diff(a, b, i));
+    return r;
 }
 
-__global__ void sse_kernel(const float* __restrict__ clips, const float* __restrict__ tmpl, uint32_t n, uint32_t len,
-                           float* sse)
+// The pieces of clips of one length and the additions of their sums, in order: step k
+// adds the sum at right[k] to the one at left[k] (made on the host, passed by value).
+constexpr uint32_t kPieces = 256;   // pieces of 64 values at least: clips of 16,384 samples fit
+struct PieceList {
+    uint16_t count;
+    uint16_t first[kPieces + 1];
+    uint8_t left[kPieces], right[kPieces];
+};
+
+PieceList make_pieces(uint32_t len)
+{
+    PieceList l{};
+    uint32_t adds = 0;
+    pairwise_sum<uint32_t>(   // a sum is the place of its leftmost piece
+        len,
+        [&](uint32_t at, uint32_t) {
+            l.first[l.count] = (uint16_t)at;
+            return (uint32_t)l.count++;
+        },
+        [&](uint32_t a, uint32_t b) {
+            l.left[adds] = (uint8_t)a;
+            l.right[adds++] = (uint8_t)b;
+            return a;
+        });
+    l.first[l.count] = (uint16_t)len;
+    return l;
+}
+
+// A warp per clip: its pieces by groups of 8 lanes, their sums added by one lane.
+// (A thread per clip read its clip alone, 4 bytes of every 32-byte sector at a time:
+// 188 us for a unit of 300 clips x 1616 samples, now 20.)  Longer clips than
+// kPieces allows by a thread each.
+constexpr int kSseThreads = 128;
+
+__global__ void __launch_bounds__(kSseThreads) sse_kernel(const float* __restrict__ clips,
+                                                          const float* __restrict__ tmpl, uint32_t n, uint32_t len,
+                                                          const __grid_constant__ PieceList P, float* sse)
+{
+    __shared__ float sums[kSseThreads / 32][kPieces];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 3, j = lane & 7u;
+    const uint32_t count = P.count, nwarps = gridDim.x * (kSseThreads / 32);
+    for (uint32_t i = blockIdx.x * (kSseThreads / 32) + warp; i < n; i += nwarps) {
+        const float* c = clips + (uint64_t)i * len;
+        for (uint32_t k = g; k < count; k += 4) {
+            const float s = piece_sum(c + P.first[k], tmpl + P.first[k], P.first[k + 1] - P.first[k], j, 0xFFu << (8 * g));
+            if (j == 0) sums[warp][k] = s;
+        }
+        __syncwarp();
+        if (lane == 0) {
+            for (uint32_t k = 0; k + 1 < count; ++k)
+                sums[warp][P.left[k]] = __fadd_rn(sums[warp][P.left[k]], sums[warp][P.right[k]]);
+            sse[i] = sums[warp][0];
+        }
+        __syncwarp();
+    }
+}
+
+// numpy's pairwise sum of (a - b)^2 over [0, n) by one thread
+__device__ float pairwise_sq(const float* __restrict__ a, const float* __restrict__ b, uint32_t len)
+{
+    return pairwise_sum<float>(
+        len,
+        [&](uint32_t at, uint32_t n) {
+            const float *x = a + at, *y = b + at;
+            const uint32_t n8 = n - n % 8;
+            float res = 0.f;
+            if (n8) {
+                float r[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) r[j] = sq_diff(x, y, j);
+                for (uint32_t i = 8; i < n8; i += 8) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) r[j] = __fadd_rn(r[j], sq_diff(x, y, i + j));
+                }
+                res = __fadd_rn(__fadd_rn(__fadd_rn(r[0], r[1]), __fadd_rn(r[2], r[3])),
+                                __fadd_rn(__fadd_rn(r[4], r[5]), __fadd_rn(r[6], r[7])));
+            }
+            for (uint32_t i = n8; i < n; ++i) res = __fadd_rn(res, sq_diff(x, y, i));
+            return res;
+        },
+        [](float l, float r) { return __fadd_rn(l, r); });
+}
+
+__global__ void sse_long_kernel(const float* __restrict__ clips, const float* __restrict__ tmpl, uint32_t n,
+                                uint32_t len, float* sse)
 {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         sse[i] = pairwise_sq(clips + (uint64_t)i * len, tmpl, len);
@@ -153,7 +246,7 @@ extern "C" int fbp_mean_clip(const float* clips, uint32_t n, uint32_t clip_len, 
     if (n == 0 || clip_len == 0) return fail(FBP_E_ARG, "no clips");
     if (!clips || !mean) return fail(FBP_E_ARG, "null pointer argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    mean_clip_kernel<<<(clip_len + 255) / 256, 256, 0, st>>>(clips, n, clip_len, mean);
+    mean_clip_kernel<<<(clip_len + kMeanThreads - 1) / kMeanThreads, kMeanThreads, 0, st>>>(clips, n, clip_len, mean);
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -175,7 +268,11 @@ extern "C" int fbp_bp_duplicates(const int64_t* event_indices, const float* clip
     float* sse = reinterpret_cast<float*>(ws);
     uint8_t* start = ws + ((size_t)n * 4 + 255) / 256 * 256;
     const uint32_t g = (n + 255) / 256 < 148u * 16 ? (n + 255) / 256 : 148u * 16;
-    sse_kernel<<<g, 256, 0, st>>>(clips, unit_template, n, clip_len, sse);
+    if (clip_len <= 64 * kPieces)   // a piece has at least 64 values once there are two
+        sse_kernel<<<std::min<uint32_t>((n + kSseThreads / 32 - 1) / (kSseThreads / 32), 148u * 16), kSseThreads, 0, st>>>(
+            clips, unit_template, n, clip_len, make_pieces(clip_len), sse);
+    else
+        sse_long_kernel<<<g, 256, 0, st>>>(clips, unit_template, n, clip_len, sse);
     segment_start_kernel<<<1, kScanThreads, 0, st>>>(event_indices, n, tol_inds, start);
     walk_kernel<<<g, 256, 0, st>>>(event_indices, bp, sse, start, n, tol_inds, keep);
     FBP_CUDA(cudaGetLastError());
