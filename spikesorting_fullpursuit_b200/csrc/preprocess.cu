@@ -11,15 +11,16 @@
 //     numpy computes it: med = median(x); mad = median(|x - med|) / 0.6745;
 //     the template is median(x[med - mad < x < med + mad]), or med if that set is
 //     empty.  Medians are exact order statistics (the mean of the two middle
-//     values for an even count, as np.median), found by radix selection over
-//     order-preserving integer keys: 4 passes of 8 bits, each a shared-memory
-//     histogram of the candidates.  A CTA handles 32 adjacent columns, lanes
-//     over columns, so every pass reads rows of 128 contiguous bytes.
+//     values for an even count, as np.median) of order-preserving integer keys.
+//     Up to 2048 clips a warp keeps a column's keys in registers and finds the
+//     middle one bit by bit; above, robust_template_large_kernel selects by radix
+//     (4 passes of 8 bits over shared-memory histograms, 32 columns a CTA).
 //   * covariance_kernel: per channel, the FP64 covariance (ddof 0) of the
-//     selected residual rows' samples on that channel: column means summed over
-//     the rows in order (numpy's axis-0 order), then centred products.  numpy
-//     multiplies with BLAS, so covariances agree to FP64 rounding.
-#include <cub/cub.cuh>
+//     selected residual rows' samples on that channel: column means, then centred
+//     products.  numpy multiplies with BLAS, so covariances agree to FP64 rounding.
+#include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "fbp_internal.cuh"
 
@@ -125,8 +126,8 @@ __device__ float column_median(const float* __restrict__ clips, uint32_t n, uint
     return (c & 1u) ? a : __fdiv_rn(__fadd_rn(a, b), 2.0f);
 }
 
-__global__ void __launch_bounds__(kRtThreads) robust_template_kernel(const float* __restrict__ clips, uint32_t n,
-                                                                     uint32_t len, float* tmpl)
+__global__ void __launch_bounds__(kRtThreads) robust_template_large_kernel(const float* __restrict__ clips,
+                                                                           uint32_t n, uint32_t len, float* tmpl)
 {
     __shared__ uint32_t hist[kRtCols * 256];
     __shared__ uint32_t s_prefix[kRtCols], s_k[kRtCols], kth[kRtCols], cnt[kRtCols];
@@ -163,40 +164,212 @@ __global__ void __launch_bounds__(kRtThreads) robust_template_kernel(const float
     if (threadIdx.x < kRtCols && col < len) tmpl[col] = cnt[threadIdx.x] > 0 ? sel : med;
 }
 
-// Per channel c (blockIdx.y) and output row i (blockIdx.x): means of the
-// channel's selected residual rows (rows[c][0..n_rows)) over its samples
-// [c*Wc, (c+1)*Wc), and row i of its covariance.
-// Residual row r = clips[rows[r]] - template[unit[rows[r]]] in float32, then FP64.
-__global__ void covariance_kernel(const float* __restrict__ clips, const float* __restrict__ tmpls,
-                                  const uint32_t* __restrict__ unit_of, const int64_t* __restrict__ rows,
-                                  uint32_t n_rows, uint32_t len, uint32_t wc, double* cov)
+// Median of the `cnt` valid keys of a warp's column (lane slots, 0xFFFFFFFF where
+// there is none): the middle key bit by bit -- the largest value with at most k
+// smaller keys -- and, for an even count, the next one.
+template <int NV>
+__device__ __forceinline__ float warp_median(const uint32_t (&key)[NV], uint32_t cnt)
 {
-    extern __shared__ double mean[];   // [wc]
-    const uint32_t c = blockIdx.y, i = blockIdx.x;
-    const uint32_t base = c * wc;
-    for (uint32_t j = threadIdx.x; j < wc; j += blockDim.x) {
-        double acc = 0.0;
-        bool first = true;
-        for (uint32_t r = 0; r < n_rows; ++r) {
-            const uint64_t row = (uint64_t)rows[(uint64_t)c * n_rows + r];
-            const double x = (double)__fsub_rn(clips[row * len + base + j], tmpls[(uint64_t)unit_of[row] * len + base + j]);
-            acc = first ? x : __dadd_rn(acc, x);
-            first = false;
+    const uint32_t full = 0xffffffffu, k = cnt > 0 ? (cnt - 1) / 2 : 0u;
+    uint32_t a = 0;
+    for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t cand = a | (1u << bit);
+        uint32_t below = 0;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) below += key[i] < cand ? 1u : 0u;
+        if (__reduce_add_sync(full, below) <= k) a = cand;
+    }
+    if (cnt & 1u) return unkey(a);
+    uint32_t upto = 0, next = 0xFFFFFFFFu;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        upto += key[i] <= a ? 1u : 0u;
+        next = key[i] > a && key[i] < next ? key[i] : next;
+    }
+    upto = __reduce_add_sync(full, upto);
+    next = __reduce_min_sync(full, next);
+    return __fdiv_rn(__fadd_rn(unkey(a), unkey(upto > cnt / 2 ? a : next)), 2.0f);
+}
+
+// A warp per column, n <= 32 NV clips in registers (8 adjacent columns a CTA: the
+// 32-byte sectors of the clips are read once).  Three selections of 32 steps over NV
+// keys a lane bound it.  40 units of about 600 clips x 1616 samples: 27.7 ms by radix
+// selection from memory, 1616 / 32 CTAs a unit, against 1.9 ms.
+template <int NV>
+__global__ void __launch_bounds__(kRtThreads) robust_template_kernel(const float* __restrict__ clips, uint32_t n,
+                                                                     uint32_t len, float* tmpl)
+{
+    const uint32_t lane = threadIdx.x & 31, col = blockIdx.x * (kRtThreads / 32) + (threadIdx.x >> 5);
+    if (col >= len) return;
+    float x[NV];
+    uint32_t key[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const uint32_t r = i * 32 + lane;
+        x[i] = r < n ? __ldg(clips + (uint64_t)r * len + col) : 0.f;
+        key[i] = r < n ? fkey(x[i]) : 0xFFFFFFFFu;
+    }
+    const float med = warp_median<NV>(key, n);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) key[i] = i * 32 + lane < n ? fkey(fabsf(__fsub_rn(x[i], med))) : 0xFFFFFFFFu;
+    const float mad = __fdiv_rn(warp_median<NV>(key, n), 0.6745f);
+    const float lo = __fsub_rn(med, mad), hi = __fadd_rn(med, mad);
+    uint32_t cnt = 0;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const bool in = i * 32 + lane < n && x[i] > lo && x[i] < hi;
+        key[i] = in ? fkey(x[i]) : 0xFFFFFFFFu;
+        cnt += in ? 1u : 0u;
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    const float sel = warp_median<NV>(key, cnt);
+    if (lane == 0) tmpl[col] = cnt > 0 ? sel : med;
+}
+
+// Covariance of one channel (blockIdx.z) between two tiles of kCovTile of its samples
+// (blockIdx.y), over the channel's selected residual rows (rows[c][0..n_rows)):
+// residual row r = clips[rows[r]] - template[unit[rows[r]]] in float32, then FP64.
+// One pass: products and sums of x - s, s the mean of the first rows (at most
+// kCovProbe), give sum (x - s)(y - s) - sum (x - s) sum (y - s) / n; s lies within a
+// fraction of a standard deviation of the mean, so nothing cancels.  A cluster shares
+// the rows; a thread accumulates 7 x 7 of the tile (on the diagonal only its upper
+// 16-blocks) while the next rows are on their way, and the CTAs' parts are added in
+// rank order through shared memory.  16 channels x 101 samples x 10,000 rows: 7.5 ms
+// with the means summed by every output row's CTA, one scattered load at a time,
+// 1.9 ms with a pass of its own for them, 0.5 ms now.
+constexpr uint32_t kCovTile = 112, kCovRows = 16, kCovCluster = 8, kCovThreads = 256, kCovProbe = 32;
+constexpr uint32_t kCovLoads = kCovRows * kCovTile / kCovThreads;   // elements of a step a thread loads
+
+template <bool DIAG>
+__global__ void __cluster_dims__(kCovCluster, 1, 1) __launch_bounds__(kCovThreads, 1)
+    covariance_kernel(const float* __restrict__ clips, const float* __restrict__ tmpls,
+                      const uint32_t* __restrict__ unit_of, const int64_t* __restrict__ rows, uint32_t n_rows,
+                      uint32_t len, uint32_t wc, double* cov)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) double csm[];
+    constexpr uint32_t kTiles = DIAG ? 1 : 2;
+    double* part = csm;                              // [kCovTile][kCovTile] this CTA's products
+    double* xs = part + kCovTile * kCovTile;         // [kTiles][kCovRows][kCovTile] rows of a step
+    double* sums = xs + 2 * kCovRows * kCovTile;     // [2][kCovTile] this CTA's sums
+    double* shift = sums + 2 * kCovTile;             // [2][kCovTile] s
+    double* total = shift + 2 * kCovTile;            // [2][kCovTile] the cluster's sums
+    __shared__ uint64_t s_clip[2][kCovRows], s_tmpl[2][kCovRows];   // row offsets of two steps
+    const uint32_t nt = (wc + kCovTile - 1) / kCovTile, c = blockIdx.z, rank = cluster.block_rank();
+    // tile pair: the diagonal launch numbers the tiles, the other one the ordered pairs
+    const uint32_t it = DIAG ? blockIdx.y : blockIdx.y / (nt - 1);
+    uint32_t jt = DIAG ? it : blockIdx.y % (nt - 1);
+    if (!DIAG && jt >= it) ++jt;
+    const uint32_t base[2] = {it * kCovTile, jt * kCovTile};
+    const uint32_t cols[2] = {min(kCovTile, wc - base[0]), min(kCovTile, wc - base[1])};
+    const uint32_t share = (n_rows + kCovCluster - 1) / kCovCluster;
+    const uint32_t r0 = min(n_rows, rank * share), r1 = min(n_rows, r0 + share);
+    const int64_t* mine = rows + (uint64_t)c * n_rows;
+    // provisional means
+    const uint32_t probe = min(n_rows, kCovProbe);
+    for (uint32_t k = threadIdx.x; k < kTiles * kCovTile; k += kCovThreads) {
+        const uint32_t w = k / kCovTile, j = k - w * kCovTile;
+        double s = 0.0;
+        if (j < cols[w])
+#pragma unroll 8
+            for (uint32_t r = 0; r < probe; ++r) {
+                const uint64_t row = (uint64_t)__ldg(mine + r), at = (uint64_t)c * wc + base[w] + j;
+                s += (double)__fsub_rn(__ldg(clips + row * len + at), __ldg(tmpls + (uint64_t)__ldg(unit_of + row) * len + at));
+            }
+        shift[k] = s / (double)probe;
+    }
+    auto offsets = [&](uint32_t step) {   // row offsets of a step, by its first threads
+        const uint32_t r = r0 + step * kCovRows + threadIdx.x;
+        if (threadIdx.x < kCovRows && r < r1) {
+            const uint64_t row = (uint64_t)__ldg(mine + r);
+            s_clip[step & 1u][threadIdx.x] = row * len + (uint64_t)c * wc;
+            s_tmpl[step & 1u][threadIdx.x] = (uint64_t)__ldg(unit_of + row) * len + (uint64_t)c * wc;
         }
-        mean[j] = acc / (double)n_rows;
+    };
+    float xv[kTiles][kCovLoads], tv[kTiles][kCovLoads];
+    auto fetch = [&](uint32_t step) {     // a step's values into registers
+#pragma unroll
+        for (uint32_t w = 0; w < kTiles; ++w)
+#pragma unroll
+            for (uint32_t q = 0; q < kCovLoads; ++q) {
+                const uint32_t e = threadIdx.x + q * kCovThreads, r = e / kCovTile, k = e - r * kCovTile;
+                const bool in = r0 + step * kCovRows + r < r1 && k < cols[w];
+                xv[w][q] = in ? __ldg(clips + s_clip[step & 1u][r] + base[w] + k) : 0.f;
+                tv[w][q] = in ? __ldg(tmpls + s_tmpl[step & 1u][r] + base[w] + k) : 0.f;
+            }
+    };
+    const uint32_t steps = (r1 - r0 + kCovRows - 1) / kCovRows;
+    offsets(0);
+    __syncthreads();   // the provisional means too
+    if (steps > 0) fetch(0);
+    const uint32_t tx = threadIdx.x & 15u, ty = threadIdx.x >> 4;
+    double acc[7][7], sum = 0.0;
+#pragma unroll
+    for (int a = 0; a < 7; ++a)
+#pragma unroll
+        for (int b = 0; b < 7; ++b) acc[a][b] = 0.0;
+    for (uint32_t st = 0; st < steps; ++st) {
+        const uint32_t nr = min(kCovRows, r1 - (r0 + st * kCovRows));
+#pragma unroll
+        for (uint32_t w = 0; w < kTiles; ++w)
+#pragma unroll
+            for (uint32_t q = 0; q < kCovLoads; ++q) {
+                const uint32_t e = threadIdx.x + q * kCovThreads, r = e / kCovTile, k = e - r * kCovTile;
+                xs[w * kCovRows * kCovTile + e] =
+                    r < nr && k < cols[w] ? (double)__fsub_rn(xv[w][q], tv[w][q]) - shift[w * kCovTile + k] : 0.0;
+            }
+        offsets(st + 1);
+        __syncthreads();
+        if (st + 1 < steps) fetch(st + 1);
+        const double* second = DIAG ? xs : xs + kCovRows * kCovTile;
+        for (uint32_t r = 0; r < nr; ++r) {
+            double u[7], v[7];
+#pragma unroll
+            for (int a = 0; a < 7; ++a) {
+                u[a] = xs[r * kCovTile + ty + 16 * a];
+                v[a] = second[r * kCovTile + tx + 16 * a];
+            }
+#pragma unroll
+            for (int a = 0; a < 7; ++a)
+#pragma unroll
+                for (int b = 0; b < 7; ++b)
+                    if (!DIAG || b >= a) acc[a][b] = fma(u[a], v[b], acc[a][b]);
+        }
+        if (threadIdx.x < kTiles * kCovTile) {
+            const uint32_t w = threadIdx.x / kCovTile, k = threadIdx.x - w * kCovTile;
+            for (uint32_t r = 0; r < nr; ++r) sum += xs[(w * kCovRows + r) * kCovTile + k];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < kTiles * kCovTile) sums[threadIdx.x] = sum;
+#pragma unroll
+    for (int a = 0; a < 7; ++a)
+#pragma unroll
+        for (int b = 0; b < 7; ++b)
+            if (!DIAG || b >= a) part[(ty + 16 * a) * kCovTile + tx + 16 * b] = acc[a][b];
+    cluster.sync();
+    for (uint32_t k = threadIdx.x; k < kTiles * kCovTile; k += kCovThreads) {
+        double s = 0.0;
+        for (uint32_t b = 0; b < kCovCluster; ++b) s += cluster.map_shared_rank(sums, b)[k];
+        total[k] = s;
     }
     __syncthreads();
-    for (uint32_t j = threadIdx.x; j < wc; j += blockDim.x) {
-        double acc = 0.0;
-        for (uint32_t r = 0; r < n_rows; ++r) {
-            const uint64_t row = (uint64_t)rows[(uint64_t)c * n_rows + r];
-            const uint64_t u = (uint64_t)unit_of[row] * len + base;
-            const double xi = (double)__fsub_rn(clips[row * len + base + i], tmpls[u + i]) - mean[i];
-            const double xj = (double)__fsub_rn(clips[row * len + base + j], tmpls[u + j]) - mean[j];
-            acc = fma(xi, xj, acc);
+    // this CTA's share of the tile, parts added in rank order
+    const double inv = 1.0 / (double)n_rows;   // np.cov scales by 1 / fact
+    for (uint32_t e = rank * kCovThreads + threadIdx.x; e < cols[0] * cols[1]; e += kCovCluster * kCovThreads) {
+        uint32_t i = e / cols[1], j = e - i * cols[1];
+        const uint32_t oi = i, oj = j;
+        if (DIAG && j < i) {   // the covariance is symmetric: only its upper 16-blocks are there
+            i = oj;
+            j = oi;
         }
-        cov[((uint64_t)c * wc + i) * wc + j] = acc * (1.0 / (double)n_rows);   // np.cov scales by 1 / fact
+        double s = 0.0;
+        for (uint32_t b = 0; b < kCovCluster; ++b) s += cluster.map_shared_rank(part, b)[i * kCovTile + j];
+        s -= (total[i] * total[(DIAG ? 0 : kCovTile) + j]) * inv;   // the same for (j, i)
+        cov[((uint64_t)c * wc + base[0] + oi) * wc + base[1] + oj] = s * inv;
     }
+    cluster.sync();   // no CTA leaves while another reads its part
 }
 
 }  // namespace
@@ -225,8 +398,18 @@ extern "C" int fbp_robust_template(const float* clips, uint32_t n, uint32_t clip
     set_error("");
     if (n == 0 || clip_len == 0) return fail(FBP_E_ARG, "no clips");
     if (!clips || !tmpl) return fail(FBP_E_ARG, "null pointer argument");
-    robust_template_kernel<<<(clip_len + kRtCols - 1) / kRtCols, kRtThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        clips, n, clip_len, tmpl);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const uint32_t grid = (clip_len + kRtThreads / 32 - 1) / (kRtThreads / 32);
+    if (n <= 256)
+        robust_template_kernel<8><<<grid, kRtThreads, 0, st>>>(clips, n, clip_len, tmpl);
+    else if (n <= 512)
+        robust_template_kernel<16><<<grid, kRtThreads, 0, st>>>(clips, n, clip_len, tmpl);
+    else if (n <= 1024)
+        robust_template_kernel<32><<<grid, kRtThreads, 0, st>>>(clips, n, clip_len, tmpl);
+    else if (n <= 2048)
+        robust_template_kernel<64><<<grid, kRtThreads, 0, st>>>(clips, n, clip_len, tmpl);
+    else   // more keys than a warp holds
+        robust_template_large_kernel<<<(clip_len + kRtCols - 1) / kRtCols, kRtThreads, 0, st>>>(clips, n, clip_len, tmpl);
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -239,10 +422,18 @@ extern "C" int fbp_residual_covariance(const float* clips, const float* template
     if (n_rows == 0 || n_chans == 0 || n_samples_per_chan == 0) return fail(FBP_E_ARG, "invalid sizes");
     if ((uint64_t)n_chans * n_samples_per_chan > clip_len) return fail(FBP_E_ARG, "clip shorter than channels x samples");
     if (!clips || !templates || !unit_of || !rows || !cov) return fail(FBP_E_ARG, "null pointer argument");
-    const size_t smem = (size_t)n_samples_per_chan * 8;
-    if (smem > 48 * 1024) return fail(FBP_E_ARG, "samples per channel too large");
-    covariance_kernel<<<dim3(n_samples_per_chan, n_chans), 128, smem, static_cast<cudaStream_t>(stream)>>>(
+    if ((size_t)n_samples_per_chan * 8 > 48 * 1024) return fail(FBP_E_ARG, "samples per channel too large");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t smem = (kCovTile * kCovTile + 2 * kCovRows * kCovTile + 6 * kCovTile) * sizeof(double);
+    const uint32_t nt = (n_samples_per_chan + kCovTile - 1) / kCovTile;
+    FBP_CUDA(allow_max_dyn_smem(covariance_kernel<true>));
+    covariance_kernel<true><<<dim3(kCovCluster, nt, n_chans), kCovThreads, smem, st>>>(
         clips, templates, unit_of, rows, n_rows, clip_len, n_samples_per_chan, cov);
+    if (nt > 1) {
+        FBP_CUDA(allow_max_dyn_smem(covariance_kernel<false>));
+        covariance_kernel<false><<<dim3(kCovCluster, nt * (nt - 1), n_chans), kCovThreads, smem, st>>>(
+            clips, templates, unit_of, rows, n_rows, clip_len, n_samples_per_chan, cov);
+    }
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
