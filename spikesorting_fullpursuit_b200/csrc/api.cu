@@ -5,9 +5,10 @@
 // state resident on the device.  The reference copies three arrays to the host
 // and back every pass and compacts window lists with np.nonzero
 // (binary_pursuit_parallel.py:966-979, 1210-1251); here the lists are compacted
-// on the device and the host reads one 48-byte status word per pass.
+// on the device and the host reads one status word per pass.
 #include <algorithm>
 #include <chrono>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -106,8 +107,7 @@ bool make_layout(const fbp_dims* d, uint32_t flags, Layout* L)
     L->off_pwin = take(nw * 4);
     L->off_pconf = take(nw);
     L->off_keys = take(nw * 8);
-    L->off_blk = take(L->nblk * 4);
-    L->off_status = take(sizeof(DevStatus));
+    L->off_status = take(256 + 3 * L->nblk * 8);   // DevStatus, then the compactions' look-back states
     if (!(flags & FBP_PLAIN_FP32)) {
         // tensor-core likelihood: the voltage sample-major in 4-channel rows
         // (channels padded to a multiple of 8), the templates in MMA order and
@@ -304,17 +304,18 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
     }
     // per-window state starts at zero (binary_pursuit_parallel.py:595-654)
     FBP_CUDA(cudaMemsetAsync(w.base + lay.off_best_lik, 0, lay.off_list - lay.off_best_lik, st));
-    FBP_CUDA(cudaMemsetAsync(w.status(), 0, sizeof(DevStatus), st));
+    const size_t all_bytes = 256 + 3 * lay.nblk * 8, pass_bytes = all_bytes - offsetof(DevStatus, n_flag);
+    FBP_CUDA(cudaMemsetAsync(w.status(), 0, all_bytes, st));
     FBP_TRY(launch_iota(w.list(), d.nw, st));
     if (!plain) FBP_TRY(launch_template_info(d, w, templates, st));
     if (use_tc) {
         FBP_TRY(launch_tc_prepare_templates(d, w, templates, st));
         if (ready.n == 0) FBP_TRY(launch_tc_update_voltage(d, w, voltage, nullptr, nullptr, 0, true, st));
     }
-    if (lazy) FBP_CUDA(cudaMemsetAsync(w.base + lay.off_wflag, 0, lay.nw * lay.M, st));
     if (!plain && overlap) FBP_TRY(launch_overlap_tables(d, w, templates, st));
     uint32_t nlist = d.nw, total = 0;
     api_detail::StageTimer tm;
+    DevStatus hs{};
     for (int32_t pass = 1;; ++pass) {
         if (max_passes > 0 && pass > max_passes) {
             S.n_spikes = total;
@@ -325,7 +326,8 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         }
         S.passes = pass;
         S.listed += nlist;
-        FBP_CUDA(cudaMemsetAsync(&w.status()->chain_overflow, 0, 8, st));
+        if (pass > 1)   // the pass's counters and look-back states
+            FBP_CUDA(cudaMemsetAsync(&w.status()->n_flag, 0, pass_bytes, st));
         tm.start(timing, st, &S.ms_likelihood);
         if (pass == 1 && ready.n > 0) {
             // first pass behind the upload: of each arrived range, the spans (or
@@ -366,14 +368,14 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         }
         tm.stop();
         tm.start(timing, st, &S.ms_argmax);
-        if (lazy)
-            FBP_TRY(launch_argmax_lazy(d, w, w.list(), nlist, st));
+        if (lazy)   // and the list of flagged windows
+            FBP_TRY(launch_argmax_lazy(d, w, nlist, overlap, st));
         else
             FBP_TRY(launch_argmax(d, w, w.list(), nlist, st));
         tm.stop();
         tm.start(timing, st, &S.ms_overlap);
         if (overlap) {
-            FBP_TRY(launch_compact_flagged(d, w, nlist, st));
+            if (!lazy) FBP_TRY(launch_compact_flagged(d, w, nlist, st));
             if (plain)
                 FBP_TRY(launch_overlap_plain(d, w, voltage, templates, theta, nlist, st));
             else
@@ -386,7 +388,6 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         if (lazy) FBP_TRY(launch_lazy_fix(d, w, voltage, templates, bias, nlist, st));
         FBP_TRY(launch_next_list(d, w, st));
         tm.stop();
-        DevStatus hs;
         FBP_CUDA(cudaMemcpyAsync(&hs, w.status(), sizeof(hs), cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaStreamSynchronize(st));
         if (hs.error) return fail(FBP_E_DEVICE, "device status error " + std::to_string(hs.error));
@@ -401,11 +402,9 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
             *n_spikes = total + n;   // at least this many outputs are needed
             return fail(FBP_E_CAPACITY, "spike capacity exceeded");
         }
-        FBP_CUDA(cudaMemcpyAsync(spike_idx + total, w.pidx(), (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
-        FBP_CUDA(cudaMemcpyAsync(spike_lab + total, w.plab(), (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
-        FBP_CUDA(cudaMemsetAsync(w.orech(), 0, d.nw, st));
         tm.start(timing, st, &S.ms_residual);
-        FBP_TRY(launch_residual(d, w, voltage, templates, w.pidx(), w.plab(), w.pwin(), n, st));
+        FBP_TRY(launch_residual(d, w, voltage, templates, w.pidx(), w.plab(), w.pwin(), n, st, spike_idx + total,
+                                spike_lab + total));
         if (use_tc) FBP_TRY(launch_tc_update_voltage(d, w, voltage, w.pidx(), w.pwin(), n, false, st));
         tm.stop();
         total += n;
@@ -419,9 +418,6 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         cudaEventDestroy(t_begin);
         cudaEventDestroy(t_end);
     }
-    DevStatus hs;
-    FBP_CUDA(cudaMemcpyAsync(&hs, w.status(), sizeof(hs), cudaMemcpyDeviceToHost, st));
-    FBP_CUDA(cudaStreamSynchronize(st));
     S.pair_exact = (plain || !lay.screened) ? hs.pair_items : hs.n_pair_exact;
     S.fixups += 4ull * hs.n_fix_local;
     S.pc_macs = hs.pc_macs;

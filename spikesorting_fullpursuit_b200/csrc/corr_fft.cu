@@ -611,13 +611,11 @@ int launch_likelihood_fft(const Dims& d, const Work& w, const float* V, const fl
     P.wpos = w.at<uint8_t>(L.off_wpos);
     P.wflag = w.at<uint8_t>(L.off_wflag);
     P.wslots = lik_slots(d.W);
-    FBP_CUDA(cudaMemsetAsync(&w.status()->n_fix, 0, 8, st));   // and n_units
     if (all) {
-        if (span0 == 0) {
-            FBP_CUDA(cudaMemsetAsync(P.wkey, 0, (size_t)d.nw * 8, st));
-            FBP_CUDA(cudaMemsetAsync(P.wpos, 0, (size_t)d.nw, st));
-            FBP_CUDA(cudaMemsetAsync(P.wflag, 0, (size_t)d.nw * d.M, st));
-        }
+        if (span0 == 0)   // window keys, positive flags, estimate flags
+            FBP_CUDA(cudaMemsetAsync(P.wkey, 0, L.off_wflag + L.nw * L.M - L.off_wkey, st));
+        else              // a later range of the first pass: its own queue
+            FBP_CUDA(cudaMemsetAsync(&w.status()->n_fix, 0, 4, st));
     } else {
         count_launch();
         lik_units_kernel<<<std::min<uint32_t>((nlist + 127) / 128, 148 * 8), 128, 0, st>>>(

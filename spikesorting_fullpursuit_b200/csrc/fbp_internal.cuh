@@ -78,20 +78,26 @@ class KScope {
 // Device status word: counters the kernels of one pass publish.
 // ---------------------------------------------------------------------------
 struct DevStatus {
+    // of the whole call
+    uint32_t error;         // nonzero: a kernel detected an inconsistent state
+    uint32_t n_pair_exact;  // overlap items recomputed exactly
+    unsigned long long pair_items;  // items evaluated by the overlap recheck
+    unsigned long long pc_macs;     // multiply-adds done by the partial correlations
+    uint32_t n_fix_local;   // runs recomputed inside the likelihood kernel
+    uint32_t reserved;
+    // of one pass: from here to the end, and the look-back states behind it, zeroed at its start
     uint32_t n_flag;        // windows flagged for the overlap recheck this pass
     uint32_t n_spikes;      // spikes accepted this pass
     uint32_t n_next;        // windows listed for the next pass
     uint32_t chain_overflow;// a prune/reassign chain was longer than the walk limit
-    uint32_t error;         // nonzero: a kernel detected an inconsistent state
     uint32_t n_fix;         // runs of 4 likelihood samples queued for exact recomputation
     uint32_t n_units;       // spans of listed windows the transform likelihood takes this pass
-    uint32_t n_pair_exact;  // overlap items recomputed exactly
-    uint32_t n_conf;        // spikes of this pass overlapping an earlier one
-    unsigned long long pair_items;  // items evaluated by the overlap recheck
     uint32_t cand_count;    // candidates appended to the exact-scoring list (per batch)
-    uint32_t n_fix_local;   // runs recomputed inside the likelihood kernel (whole call)
-    unsigned long long pc_macs;   // multiply-adds done by the partial correlations (whole call)
+    uint32_t ticket[3];     // next tile of the pass's three compactions
+    uint32_t n_conf;        // spikes of a residual overlapping an earlier one
+    uint32_t residual_done; // CTAs of a residual that are done
 };
+static_assert(sizeof(DevStatus) <= 256, "the allocation-free residual keeps 256 bytes for it");
 
 // ---------------------------------------------------------------------------
 // Workspace layout (all offsets 256-byte aligned)
@@ -101,7 +107,7 @@ struct Layout {
     size_t off_L, off_best_lik, off_best_lab, off_best_idx, off_ov_idx, off_ov_lab;
     size_t off_check, off_orech, off_orech_fin, off_list, off_list2, off_flag;
     size_t off_has, off_newval, off_pidx, off_plab, off_pwin, off_pconf, off_keys;
-    size_t off_blk, off_status;
+    size_t off_status;
     // tensor-core likelihood (mode 1)
     size_t off_vt_hi, off_tt_hi, off_tpad, off_fix, off_tnorm, off_tchm;
     uint64_t Cp, Mp, n_fix_cap, vq_rows;
@@ -146,8 +152,9 @@ struct Work {
     uint32_t* pwin() const { return at<uint32_t>(lay->off_pwin); }
     uint8_t* pconf() const { return at<uint8_t>(lay->off_pconf); }
     unsigned long long* keys() const { return at<unsigned long long>(lay->off_keys); }
-    uint32_t* blk() const { return at<uint32_t>(lay->off_blk); }
     DevStatus* status() const { return at<DevStatus>(lay->off_status); }
+    // look-back states of the pass's compactions [3][nblk], behind the status word
+    unsigned long long* tiles() const { return reinterpret_cast<unsigned long long*>(base + lay->off_status + 256); }
 };
 
 // Where the tensor-core likelihood left estimates (lazy exactness): readers of
@@ -180,6 +187,8 @@ int launch_likelihood_exact(const Dims& d, const float* V, const float* T, const
 int launch_argmax(const Dims& d, const Work& w, const uint32_t* list, uint32_t nlist,
                   cudaStream_t st);
 int launch_compact_flagged(const Dims& d, const Work& w, uint32_t nlist, cudaStream_t st);
+// per-window argmax from the window keys (lazy exactness); with `overlap`, the flagged list too
+int launch_argmax_lazy(const Dims& d, const Work& w, uint32_t nlist, bool overlap, cudaStream_t st);
 int launch_overlap_plain(const Dims& d, const Work& w, const float* V, const float* T,
                          const float* theta, uint32_t nflag_max, cudaStream_t st);
 int launch_parse_reassign(const Dims& d, const Work& w, const float* theta, uint32_t nflag_max,
@@ -190,7 +199,7 @@ int launch_accept(const Dims& d, const Work& w, const float* theta, uint32_t nli
 int launch_next_list(const Dims& d, const Work& w, cudaStream_t st);
 int launch_residual(const Dims& d, const Work& w, float* V, const float* T,
                     const uint32_t* idx, const uint32_t* lab, const uint32_t* win, uint32_t n,
-                    cudaStream_t st);
+                    cudaStream_t st, uint32_t* out_idx = nullptr, uint32_t* out_lab = nullptr);
 int launch_adjusted_clips(const Dims& d, const float* V, const float* T, const uint32_t* idx,
                           const uint32_t* lab, uint32_t n, float* clips, cudaStream_t st);
 
@@ -206,10 +215,8 @@ int launch_tc_pack_range(const Dims& d, const Work& w, const float* V, uint64_t 
 uint64_t tc_tile_rows(const Dims& d);
 int launch_fixup(const Dims& d, const Work& w, const float* V, const float* T, const float* bias, float* Lk, bool lazy,
                  cudaStream_t st);
-// Lazy exactness: per-window argmax from the window keys, and the exact
-// recomputation of estimates whose voltage the coming residual changes in
-// windows the next pass does not relist.
-int launch_argmax_lazy(const Dims& d, const Work& w, const uint32_t* list, uint32_t nlist, cudaStream_t st);
+// Lazy exactness: the exact recomputation of estimates whose voltage the coming
+// residual changes in windows the next pass does not relist.
 int launch_lazy_fix(const Dims& d, const Work& w, const float* V, const float* T, const float* bias,
                     uint32_t nmax, cudaStream_t st);
 int launch_tc_prepare_templates(const Dims& d, const Work& w, const float* T, cudaStream_t st);

@@ -172,92 +172,143 @@ __global__ void argmax_kernel(Dims d, const float* __restrict__ L, const uint32_
     }
 }
 
+// Per-window argmax from the window keys (compute_template_maximum_likelihood,
+// binary_pursuit.cl:350-441): the maximum over the 3-window span of listed window
+// id is the best of the maxima of windows id-1, id and id+1, compared by value,
+// then template, then sample (the span's first maximum in template-major order).
+// The flags and outputs are those of argmax_kernel.
+struct ArgmaxLazy {
+    Dims d;
+    const uint32_t* list;
+    const unsigned long long* wkey;
+    const uint8_t* wpos;
+    float* best_lik;
+    uint32_t* best_lab;
+    uint32_t* best_idx;
+    uint8_t* check;
+    uint8_t* orech;
+    uint32_t* ov_idx;
+    uint32_t* ov_lab;
+};
+
+__device__ __forceinline__ void argmax_window(const ArgmaxLazy& a, uint32_t id)
+{
+    const Dims& d = a.d;
+    const uint64_t start = (uint64_t)id * d.W, end = start + d.W;
+    if (end >= (uint64_t)d.N - d.W) return;
+    bool have = false;
+    float bv = 0.f;
+    uint32_t bt = 0, bs = 0;
+    const uint32_t x0 = id > 0 ? id - 1 : 0;
+    for (uint32_t x = x0; x <= id + 1; ++x) {   // id + 1 < nw: end + W < N
+        const unsigned long long key = a.wkey[x];
+        if (key == 0ull) continue;
+        const float v = __uint_as_float((uint32_t)(key >> 32));
+        const uint32_t code = 0xFFFFFFFFu - (uint32_t)key;
+        const uint32_t t = code >> 10, s = x * d.W + (code & 1023u);
+        if (!have || v > bv || (v == bv && (t < bt || (t == bt && s < bs)))) {
+            have = true; bv = v; bt = t; bs = s;
+        }
+    }
+    if (a.wpos[id]) a.check[id] = 1;
+    uint32_t lab = a.best_lab[id], idx = a.best_idx[id];
+    float bl = 0.f;
+    if (have) { bl = bv; lab = bt; idx = bs; }
+    a.orech[id] = (bl > 0.f && idx >= start && idx < end) ? 1 : 0;
+    a.best_lik[id] = bl;
+    a.best_lab[id] = lab;
+    a.best_idx[id] = idx;
+    a.ov_idx[id] = idx;
+    a.ov_lab[id] = lab;
+}
+
+__global__ void argmax_lazy_kernel(ArgmaxLazy a, uint32_t nlist)
+{
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nlist; k += gridDim.x * blockDim.x)
+        argmax_window(a, a.list[k]);
+}
+
 // ---------------------------------------------------------------------------
-// Ordered stream compaction: count per block, scan of block counts, scatter.
-// A functor supplies pred(i), emit(i, pos) and after(i) (run in the scatter).
+// Ordered stream compaction in one launch.  A functor supplies visit(i), which
+// evaluates item i once and says whether it is kept, and emit(i, pos).  Tiles are
+// numbered by a ticket, so that every tile before one that runs has started; a tile
+// publishes its count, then adds up the counts of the tiles before it, back to the
+// nearest one that knows its own position (decoupled look-back).  The wait for a
+// predecessor is limited; past it the error word is set and nothing is emitted.
+// (Count, scan and scatter as three launches took three times the launch gaps, and
+// evaluated every item twice.)
 // ---------------------------------------------------------------------------
 constexpr int kCompactThreads = 256;
 constexpr int kCompactItems = 4;
 constexpr int kCompactTile = kCompactThreads * kCompactItems;
+constexpr uint32_t kLookbackPolls = 1u << 22;
+
+constexpr unsigned long long kTileCount = 1ull << 62, kTilePlace = 2ull << 62, kTileFlags = 3ull << 62;
 
 template <class F>
-__global__ void __launch_bounds__(kCompactThreads) compact_count(F f, const uint32_t* n_dev, uint32_t n_host,
-                                                                  uint32_t* blk)
-{
-    typedef cub::BlockReduce<uint32_t, kCompactThreads> R;
-    __shared__ typename R::TempStorage tmp;
-    const uint32_t n = n_dev ? *n_dev : n_host;
-    const uint64_t base = (uint64_t)blockIdx.x * kCompactTile + threadIdx.x * kCompactItems;
-    uint32_t cnt = 0;
-#pragma unroll
-    for (int r = 0; r < kCompactItems; ++r) {
-        const uint64_t i = base + r;
-        if (i < n && f.pred((uint32_t)i)) ++cnt;
-    }
-    const uint32_t tot = R(tmp).Sum(cnt);
-    if (threadIdx.x == 0) blk[blockIdx.x] = tot;
-}
-
-__global__ void __launch_bounds__(1024) compact_scan(uint32_t* blk, uint32_t nblk, uint32_t* total)
-{
-    typedef cub::BlockScan<uint32_t, 1024> S;
-    __shared__ typename S::TempStorage tmp;
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (uint32_t b0 = 0; b0 < nblk; b0 += 1024) {
-        const uint32_t i = b0 + threadIdx.x;
-        const uint32_t v = i < nblk ? blk[i] : 0u;
-        uint32_t ex, agg;
-        S(tmp).ExclusiveSum(v, ex, agg);
-        if (i < nblk) blk[i] = ex + carry;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += agg;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0 && total) *total = carry;
-}
-
-template <class F>
-__global__ void __launch_bounds__(kCompactThreads) compact_scatter(F f, const uint32_t* n_dev, uint32_t n_host,
-                                                                    const uint32_t* blk)
+__global__ void __launch_bounds__(kCompactThreads) compact_kernel(F f, uint32_t n, unsigned long long* state,
+                                                                  uint32_t* ticket, uint32_t* total, DevStatus* status)
 {
     typedef cub::BlockScan<uint32_t, kCompactThreads> S;
     __shared__ typename S::TempStorage tmp;
-    const uint32_t n = n_dev ? *n_dev : n_host;
-    const uint64_t base = (uint64_t)blockIdx.x * kCompactTile + threadIdx.x * kCompactItems;
-    bool p[kCompactItems];
+    __shared__ uint32_t s_tile, s_base;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const uint64_t first = (uint64_t)tile * kCompactTile + threadIdx.x * kCompactItems;
+    bool keep[kCompactItems];
     uint32_t cnt = 0;
 #pragma unroll
     for (int r = 0; r < kCompactItems; ++r) {
-        const uint64_t i = base + r;
-        p[r] = i < n && f.pred((uint32_t)i);
-        cnt += p[r];
+        keep[r] = first + r < n && f.visit((uint32_t)(first + r));
+        cnt += keep[r];
     }
-    uint32_t ex;
-    S(tmp).ExclusiveSum(cnt, ex);
-    uint32_t pos = blk[blockIdx.x] + ex;
+    uint32_t ex, all;
+    S(tmp).ExclusiveSum(cnt, ex, all);
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        volatile unsigned long long* st = state;
+        if (lane == 0) st[tile] = (tile ? kTileCount : kTilePlace) | all;
+        uint32_t base = 0;
+        bool failed = false;
+        for (int64_t at = (int64_t)tile - 1; at >= 0 && !failed;) {   // 32 predecessors at a time, nearest on lane 0
+            const int64_t mine = at - lane;
+            unsigned long long v = kTilePlace;
+            if (mine >= 0) {
+                uint32_t polls = 0;
+                while (((v = st[mine]) & kTileFlags) == 0ull && ++polls < kLookbackPolls) {}
+            }
+            failed = __any_sync(0xffffffffu, (v & kTileFlags) == 0ull);
+            const uint32_t place = __ballot_sync(0xffffffffu, (v & kTileFlags) == kTilePlace);
+            const uint32_t upto = place ? (uint32_t)__ffs(place) - 1u : 31u;   // counts before it, and its position
+            base += __reduce_add_sync(0xffffffffu, lane <= upto ? (uint32_t)v : 0u);
+            if (place) break;
+            at -= 32;
+        }
+        if (lane == 0) {
+            if (failed) atomicOr(&status->error, 0x400u);
+            st[tile] = kTilePlace | (base + all);
+            s_base = failed ? 0xFFFFFFFFu : base;
+            if ((uint64_t)(tile + 1) * kCompactTile >= n) *total = base + all;
+        }
+    }
+    __syncthreads();
+    if (s_base == 0xFFFFFFFFu) return;
+    uint32_t pos = s_base + ex;
 #pragma unroll
-    for (int r = 0; r < kCompactItems; ++r) {
-        const uint64_t i = base + r;
-        if (p[r]) f.emit((uint32_t)i, pos++);
-        if (i < n) f.after((uint32_t)i);
-    }
+    for (int r = 0; r < kCompactItems; ++r)
+        if (keep[r]) f.emit((uint32_t)(first + r), pos++);
 }
 
+// `which` (0..2): the call's look-back state of the pass (zeroed at its start)
 template <class F>
-int compact(F f, const uint32_t* n_dev, uint32_t n_upper, uint32_t* blk, uint32_t* total,
-            cudaStream_t st)
+int compact(F f, const Work& w, int which, uint32_t n, uint32_t* total, cudaStream_t st)
 {
-    const uint32_t nb = (n_upper + kCompactTile - 1) / kCompactTile;
-    if (nb == 0) {
-        FBP_CUDA(cudaMemsetAsync(total, 0, sizeof(uint32_t), st));
-        return FBP_OK;
-    }
-    count_launch(3);
-    compact_count<F><<<nb, kCompactThreads, 0, st>>>(f, n_dev, n_upper, blk);
-    compact_scan<<<1, 1024, 0, st>>>(blk, nb, total);
-    compact_scatter<F><<<nb, kCompactThreads, 0, st>>>(f, n_dev, n_upper, blk);
+    const uint32_t nb = (n + kCompactTile - 1) / kCompactTile;
+    if (nb == 0) return FBP_OK;   // the pass starts with zero totals
+    count_launch();
+    compact_kernel<F><<<nb, kCompactThreads, 0, st>>>(f, n, w.tiles() + (size_t)which * w.lay->nblk,
+                                                      &w.status()->ticket[which], total, w.status());
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -266,34 +317,40 @@ struct FlagF {
     const uint32_t* list;
     const uint8_t* orech;
     uint32_t* out;
-    __device__ bool pred(uint32_t k) const { return orech[list[k]] == 1; }
-    __device__ void emit(uint32_t k, uint32_t pos) const { out[pos] = list[k]; }
-    __device__ void after(uint32_t) const {}
-};
-
-struct SpikeF {
-    const uint32_t* list;
-    const uint8_t* has;
-    const uint32_t* best_idx;
-    const uint32_t* best_lab;
-    uint32_t *pidx, *plab, *pwin;
-    __device__ bool pred(uint32_t k) const { return has[k] != 0; }
+    unsigned long long* keys;   // the recheck's winner keys of the pass start at zero
+    __device__ bool visit(uint32_t k) const { return orech[list[k]] == 1; }
     __device__ void emit(uint32_t k, uint32_t pos) const
     {
-        const uint32_t id = list[k];
-        pidx[pos] = best_idx[id];
-        plab[pos] = best_lab[id];
-        pwin[pos] = id;
+        out[pos] = list[k];
+        keys[pos] = 0ull;
     }
-    __device__ void after(uint32_t) const {}
 };
 
+// Per-window argmax from the window keys, then FlagF.
+struct ArgmaxFlagF {
+    ArgmaxLazy a;
+    FlagF f;
+    __device__ bool visit(uint32_t k) const
+    {
+        argmax_window(a, a.list[k]);
+        return f.visit(k);
+    }
+    __device__ void emit(uint32_t k, uint32_t pos) const { f.emit(k, pos); }
+};
+
+// Windows of the next pass; every window's flags of this one are cleared.
 struct NextF {
     uint8_t* check;
+    uint8_t* orech;
     uint32_t* out;
-    __device__ bool pred(uint32_t x) const { return check[x] != 0; }
+    __device__ bool visit(uint32_t x) const
+    {
+        const bool listed = check[x] != 0;
+        check[x] = 0;
+        orech[x] = 0;
+        return listed;
+    }
     __device__ void emit(uint32_t x, uint32_t pos) const { out[pos] = x; }
-    __device__ void after(uint32_t x) const { check[x] = 0; }
 };
 
 // ---------------------------------------------------------------------------
@@ -552,22 +609,20 @@ __device__ __forceinline__ bool moved_left(const Dims& d, const uint32_t* ov_idx
     return x > 1 && (uint64_t)ov_idx[x] < (uint64_t)x * d.W;
 }
 
-__global__ void reassign_resolve_kernel(Dims d, const uint32_t* __restrict__ flag, DevStatus* status,
-                                        const uint8_t* __restrict__ orech, const uint32_t* __restrict__ ov_idx,
-                                        uint8_t* orech_fin)
+// fin(id), id flagged with orech set; overflow set if the chain is longer than the walk limit
+__device__ uint8_t reassign_fin(const Dims& d, uint32_t id, const uint8_t* __restrict__ orech,
+                                const uint32_t* __restrict__ ov_idx, bool* overflow)
 {
-    const uint32_t nflag = status->n_flag;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nflag; k += gridDim.x * blockDim.x) {
-        const uint32_t id = flag[k];
-        if (!orech[id]) { orech_fin[id] = 0; continue; }
-        uint32_t j = id;
-        int steps = 0;
-        while (orech[j] && moved_left(d, ov_idx, j) && steps < kChainCap) { j -= 2; ++steps; }
-        if (steps >= kChainCap) { atomicOr(&status->chain_overflow, 1u); orech_fin[id] = 0; continue; }
-        uint8_t fv = orech[j] ? 1 : 0;
-        for (uint32_t x = j + 2; x <= id; x += 2) fv = (orech[x] && !(moved_left(d, ov_idx, x) && fv)) ? 1 : 0;
-        orech_fin[id] = fv;
+    uint32_t j = id;
+    int steps = 0;
+    while (orech[j] && moved_left(d, ov_idx, j) && steps < kChainCap) { j -= 2; ++steps; }
+    if (steps >= kChainCap) {
+        *overflow = true;
+        return 0;
     }
+    uint8_t fv = orech[j] ? 1 : 0;
+    for (uint32_t x = j + 2; x <= id; x += 2) fv = (orech[x] && !(moved_left(d, ov_idx, x) && fv)) ? 1 : 0;
+    return fv;
 }
 
 __device__ __forceinline__ void reassign_apply_one(const Dims& d, uint32_t id, bool fin_prev,
@@ -590,40 +645,42 @@ __device__ __forceinline__ void reassign_apply_one(const Dims& d, uint32_t id, b
     if ((uint64_t)ov_idx[id] >= end && (uint64_t)id + 2 < d.nwf) check[id + 2] = 2;
 }
 
-__global__ void reassign_apply_kernel(Dims d, const uint32_t* __restrict__ flag, const DevStatus* status,
-                                      const uint8_t* __restrict__ orech, const uint8_t* __restrict__ orech_fin,
-                                      uint32_t* best_idx, uint32_t* best_lab, uint8_t* check,
-                                      const uint32_t* __restrict__ ov_idx, const uint32_t* __restrict__ ov_lab)
+// Resolves and applies each flagged window; the flags themselves change in
+// reassign_commit_kernel, once every chain has been walked.
+__global__ void reassign_kernel(Dims d, const uint32_t* __restrict__ flag, DevStatus* status,
+                                const uint8_t* __restrict__ orech, uint8_t* orech_fin, uint32_t* best_idx,
+                                uint32_t* best_lab, uint8_t* check, const uint32_t* __restrict__ ov_idx,
+                                const uint32_t* __restrict__ ov_lab)
 {
-    if (status->chain_overflow) return;
     const uint32_t nflag = status->n_flag;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nflag; k += gridDim.x * blockDim.x) {
         const uint32_t id = flag[k];
-        if (!orech[id]) continue;
-        const bool prev = id > 1 && orech[id - 2] && orech_fin[id - 2];
+        if (!orech[id]) { orech_fin[id] = 0; continue; }
+        bool over = false;
+        orech_fin[id] = reassign_fin(d, id, orech, ov_idx, &over);
+        const bool prev = id > 1 && moved_left(d, ov_idx, id) && orech[id - 2] &&
+                          reassign_fin(d, id - 2, orech, ov_idx, &over);
+        if (over) { atomicOr(&status->chain_overflow, 1u); continue; }
         reassign_apply_one(d, id, prev, best_idx, best_lab, check, ov_idx, ov_lab);
     }
 }
 
-__global__ void reassign_commit_kernel(const uint32_t* __restrict__ flag, const DevStatus* status,
-                                       uint8_t* orech, const uint8_t* __restrict__ orech_fin)
+// The final flags.  If a chain exceeded the walk limit, one thread goes through all
+// flagged windows in order instead (applying again what was applied writes the same).
+__global__ void reassign_commit_kernel(Dims d, const uint32_t* __restrict__ flag, const DevStatus* status,
+                                       uint8_t* orech, const uint8_t* __restrict__ orech_fin, uint32_t* best_idx,
+                                       uint32_t* best_lab, uint8_t* check, const uint32_t* __restrict__ ov_idx,
+                                       const uint32_t* __restrict__ ov_lab)
 {
-    if (status->chain_overflow) return;
     const uint32_t nflag = status->n_flag;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nflag; k += gridDim.x * blockDim.x) {
-        const uint32_t id = flag[k];
-        if (orech[id]) orech[id] = orech_fin[id];
+    if (!(status->chain_overflow & 1u)) {
+        for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nflag; k += gridDim.x * blockDim.x) {
+            const uint32_t id = flag[k];
+            if (orech[id]) orech[id] = orech_fin[id];
+        }
+        return;
     }
-}
-
-// Sequential form, used only when a chain exceeded the walk limit.
-__global__ void reassign_sequential_kernel(Dims d, const uint32_t* __restrict__ flag, const DevStatus* status,
-                                           uint8_t* orech, uint32_t* best_idx, uint32_t* best_lab,
-                                           uint8_t* check, const uint32_t* __restrict__ ov_idx,
-                                           const uint32_t* __restrict__ ov_lab)
-{
-    if (!status->chain_overflow || threadIdx.x != 0 || blockIdx.x != 0) return;
-    const uint32_t nflag = status->n_flag;
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     for (uint32_t k = 0; k < nflag; ++k) {
         const uint32_t id = flag[k];
         if (!orech[id]) continue;
@@ -643,19 +700,30 @@ struct AcceptCtx {
     Dims d;
     const uint32_t* list;
     uint32_t n;
-    const uint8_t* has;
+    const uint8_t* orech;
     const uint8_t* check;   // values at kernel start (c0)
     const float* best_lik;
     const uint32_t* best_lab;
     const uint32_t* best_idx;
     const float* theta;
 
+    // does the entry at position k accept a spike?
+    __device__ bool has(uint32_t k) const
+    {
+        const uint32_t id = list[k];
+        const uint64_t start = (uint64_t)id * d.W, end = start + d.W;
+        float ml = 0.f;
+        uint32_t lab = 0, idx = 0;
+        if (end < (uint64_t)d.N - d.W) { ml = best_lik[id]; lab = best_lab[id]; idx = best_idx[id]; }
+        const bool o = orech[id] == 1;
+        return (ml > theta[lab] || o) && ((idx >= start && idx < end) || o);
+    }
     __device__ bool at(int64_t k, uint32_t x) const { return k >= 0 && k < (int64_t)n && list[k] == x; }
     __device__ bool same_group(uint32_t a, uint32_t b) const { return a / d.WG == b / d.WG; }
     // does the accept of the window at position kk write 3 into check[x]?
     __device__ bool writes3(uint32_t kk, uint32_t x) const
     {
-        if (!has[kk]) return false;
+        if (!has(kk)) return false;
         const uint32_t y = list[kk];
         return x == y || (y > 0 && x == y - 1) || ((uint64_t)y + 1 < d.nwf && x == y + 1);
     }
@@ -664,7 +732,7 @@ struct AcceptCtx {
     __device__ uint8_t cur(uint32_t k) const
     {
         const uint32_t x = list[k];
-        if (has[k]) return 3;
+        if (has(k)) return 3;
         if (x > 0 && at((int64_t)k - 1, x - 1) && writes3(k - 1, x)) return 3;
         if (at((int64_t)k + 1, x + 1) && same_group(k, k + 1) && writes3(k + 1, x)) return 3;
         return check[x];
@@ -672,7 +740,7 @@ struct AcceptCtx {
     __device__ bool needs_pred(uint32_t k) const
     {
         const uint32_t x = list[k];
-        if (has[k] || !guard(x) || x == 0) return false;
+        if (has(k) || !guard(x) || x == 0) return false;
         if (!at((int64_t)k - 1, x - 1)) return false;
         return (uint64_t)best_idx[x] < (uint64_t)x * d.W && cur(k) == 1;
     }
@@ -680,7 +748,7 @@ struct AcceptCtx {
     __device__ uint8_t post(uint32_t k, uint8_t pred_post) const
     {
         const uint32_t x = list[k];
-        if (has[k]) return 3;
+        if (has(k)) return 3;
         uint8_t v = cur(k);
         if (!guard(x)) return v;
         const float ml = best_lik[x];
@@ -719,25 +787,10 @@ struct AcceptCtx {
     }
 };
 
-__global__ void accept_decide_kernel(Dims d, const uint32_t* __restrict__ list, uint32_t n,
-                                     const float* __restrict__ theta, const float* __restrict__ best_lik,
-                                     const uint32_t* __restrict__ best_lab, const uint32_t* __restrict__ best_idx,
-                                     const uint8_t* __restrict__ orech, uint8_t* has)
-{
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t id = list[k];
-        const uint64_t start = (uint64_t)id * d.W, end = start + d.W;
-        float ml = 0.f;
-        uint32_t lab = 0, idx = 0;
-        if (end < (uint64_t)d.N - d.W) { ml = best_lik[id]; lab = best_lab[id]; idx = best_idx[id]; }
-        const bool o = orech[id] == 1;
-        has[k] = ((ml > theta[lab] || o) && ((idx >= start && idx < end) || o)) ? 1 : 0;
-    }
-}
-
-__global__ void accept_prune_kernel(AcceptCtx cx, uint8_t* newval, DevStatus* status)
+__global__ void accept_kernel(AcceptCtx cx, uint8_t* has, uint8_t* newval, DevStatus* status)
 {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cx.n; k += gridDim.x * blockDim.x) {
+        has[k] = cx.has(k) ? 1 : 0;
         uint32_t j = k;
         int steps = 0;
         while (cx.needs_pred(j) && steps < kChainCap) { --j; ++steps; }
@@ -748,7 +801,8 @@ __global__ void accept_prune_kernel(AcceptCtx cx, uint8_t* newval, DevStatus* st
     }
 }
 
-__global__ void accept_prune_sequential_kernel(AcceptCtx cx, uint8_t* newval, const DevStatus* status)
+// Sequential form, used only when a chain exceeded the walk limit (before the flags are written).
+__global__ void accept_sequential_kernel(AcceptCtx cx, uint8_t* newval, const DevStatus* status)
 {
     if (!(status->chain_overflow & 2u) || threadIdx.x != 0 || blockIdx.x != 0) return;
     uint8_t p = 0;
@@ -758,37 +812,73 @@ __global__ void accept_prune_sequential_kernel(AcceptCtx cx, uint8_t* newval, co
     }
 }
 
-__global__ void accept_write_kernel(AcceptCtx cx, const uint8_t* __restrict__ newval, uint8_t* check)
-{
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cx.n; k += gridDim.x * blockDim.x) {
+// The pass's spikes in list order; the windows' flags are written on the way (the
+// prune rules of every entry have read the old ones in accept_kernel).
+struct SpikeF {
+    AcceptCtx cx;
+    const uint8_t* has;
+    const uint8_t* newval;
+    uint8_t* check;
+    uint32_t *pidx, *plab, *pwin;
+    __device__ bool visit(uint32_t k) const
+    {
         const uint32_t x = cx.list[k];
         check[x] = newval[k];
-        if (cx.has[k]) {
-            if (x > 0 && !cx.at((int64_t)k - 1, x - 1)) check[x - 1] = 3;
-            if ((uint64_t)x + 1 < cx.d.nwf && !cx.at((int64_t)k + 1, x + 1)) check[x + 1] = 3;
-        }
+        if (!has[k]) return false;
+        if (x > 0 && !cx.at((int64_t)k - 1, x - 1)) check[x - 1] = 3;
+        if ((uint64_t)x + 1 < cx.d.nwf && !cx.at((int64_t)k + 1, x + 1)) check[x + 1] = 3;
+        return true;
     }
-}
+    __device__ void emit(uint32_t k, uint32_t pos) const
+    {
+        const uint32_t id = cx.list[k];
+        pidx[pos] = cx.best_idx[id];
+        plab[pos] = cx.best_lab[id];
+        pwin[pos] = id;
+    }
+};
 
 // ---------------------------------------------------------------------------
 // Residual (compute_residual, binary_pursuit.cl:57-102).  Spikes whose ranges
 // overlap an earlier spike of the list are deferred and applied in list order
 // by one CTA; all others are applied in parallel.
 // ---------------------------------------------------------------------------
-__global__ void residual_parallel_kernel(Dims d, float* V, const float* __restrict__ T,
+// Spikes whose ranges overlap an earlier spike of the list, in list order, by one CTA
+// (the last one to finish its own; other CTAs' subtractions are read past the L1).
+__device__ void residual_ordered(const Dims& d, float* V, const float* __restrict__ T, const uint32_t* idx,
+                                 const uint32_t* lab, uint32_t n, const volatile uint8_t* conf)
+{
+    const uint32_t CW = d.C * d.W;
+    for (uint32_t k = 0; k < n; ++k) {   // the same for the whole CTA
+        if (!conf[k]) continue;
+        const uint64_t s = idx[k];
+        const uint32_t l = lab[k];
+        for (uint32_t e = threadIdx.x; e < CW; e += blockDim.x) {
+            const uint32_t c = e / d.W, j = e - c * d.W;
+            if (s + j >= d.N) continue;
+            float* vp = V + (uint64_t)c * d.N + s + j;
+            __stcg(vp, fsub(__ldcg(vp), T[((uint64_t)l * d.C + c) * d.W + j]));
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void residual_kernel(Dims d, float* V, const float* __restrict__ T,
                                          const uint32_t* __restrict__ idx, const uint32_t* __restrict__ lab,
                                          const uint32_t* __restrict__ win, uint32_t n, uint32_t back,
-                                         uint8_t* conf, uint32_t* n_conf)
+                                         uint8_t* conf, DevStatus* status, uint32_t* out_idx, uint32_t* out_lab)
 {
     const uint32_t k = blockIdx.x;
-    if (k >= n) return;
     const uint64_t s = idx[k];
     const uint32_t l = lab[k];
-    if (l >= d.M) { if (threadIdx.x == 0) conf[k] = 0; return; }
-    __shared__ int s_conf;
+    __shared__ int s_conf, s_last;
     if (threadIdx.x == 0) {
         int c = 0;
-        for (int64_t kk = (int64_t)k - 1; kk >= 0; --kk) {
+        if (out_idx) {
+            out_idx[k] = (uint32_t)s;
+            out_lab[k] = l;
+        }
+        for (int64_t kk = (int64_t)k - 1; kk >= 0 && l < d.M; --kk) {
             if (win[k] - win[kk] > back) break;
             if (lab[kk] >= d.M) continue;
             const uint64_t s2 = idx[kk];
@@ -796,70 +886,43 @@ __global__ void residual_parallel_kernel(Dims d, float* V, const float* __restri
         }
         s_conf = c;
         conf[k] = (uint8_t)c;
-        if (c) atomicAdd(n_conf, 1u);
+        if (c) atomicAdd(&status->n_conf, 1u);
     }
     __syncthreads();
-    if (s_conf) return;
-    // one warp per channel row: the row's span [s, min(s+W, N)) is updated with
-    // 16-byte loads and stores over its 16-byte-aligned body, scalar at the ends
-    // (each element is still one float32 subtraction)
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const uint64_t end = s + d.W < d.N ? s + d.W : d.N;
-    for (uint32_t c = warp; c < d.C; c += nwarps) {
-        float* row = V + (uint64_t)c * d.N;
-        const float* tr = T + ((uint64_t)l * d.C + c) * d.W - s;   // tr[x] = T[l][c][x - s]
-        // first index at a 16-byte-aligned address (the row is float-aligned)
-        const uint64_t mis = (reinterpret_cast<uintptr_t>(row + s) >> 2) & 3u;
-        uint64_t a = s + ((4u - mis) & 3u);
-        a = a < end ? a : end;
-        const uint64_t b = a + ((end - a) & ~3ull);                    // end of the aligned body
-        for (uint64_t x = s + lane; x < a; x += 32) row[x] = fsub(row[x], tr[x]);
-        for (uint64_t x = a + 4ull * lane; x < b; x += 128) {
-            float4 v = *reinterpret_cast<float4*>(row + x);
-            v.x = fsub(v.x, tr[x]);
-            v.y = fsub(v.y, tr[x + 1]);
-            v.z = fsub(v.z, tr[x + 2]);
-            v.w = fsub(v.w, tr[x + 3]);
-            *reinterpret_cast<float4*>(row + x) = v;
-        }
-        for (uint64_t x = b + lane; x < end; x += 32) row[x] = fsub(row[x], tr[x]);
-    }
-}
-
-__global__ void __launch_bounds__(1024) residual_ordered_kernel(Dims d, float* V, const float* __restrict__ T,
-                                                                const uint32_t* __restrict__ idx,
-                                                                const uint32_t* __restrict__ lab, uint32_t n,
-                                                                const uint8_t* __restrict__ conf,
-                                                                const uint32_t* n_conf)
-{
-    if (*n_conf == 0) return;
-    typedef cub::BlockScan<uint32_t, 1024> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    __shared__ uint32_t todo[1024];
-    __shared__ uint32_t s_tot;
-    const uint32_t CW = d.C * d.W;
-    for (uint32_t b0 = 0; b0 < n; b0 += 1024) {
-        const uint32_t k = b0 + threadIdx.x;
-        const uint32_t f = (k < n && conf[k]) ? 1u : 0u;
-        uint32_t off, tot;
-        Scan(tmp).ExclusiveSum(f, off, tot);
-        if (f) todo[off] = k;
-        if (threadIdx.x == 0) s_tot = tot;
-        __syncthreads();
-        for (uint32_t i = 0; i < s_tot; ++i) {
-            const uint32_t kk = todo[i];
-            const uint64_t s = idx[kk];
-            const uint32_t l = lab[kk];
-            for (uint32_t e = threadIdx.x; e < CW; e += blockDim.x) {
-                const uint32_t c = e / d.W, j = e - c * d.W;
-                if (s + j >= d.N) continue;
-                float* vp = V + (uint64_t)c * d.N + s + j;
-                *vp = fsub(*vp, T[((uint64_t)l * d.C + c) * d.W + j]);
+    if (!s_conf && l < d.M) {
+        // one warp per channel row: the row's span [s, min(s+W, N)) is updated with
+        // 16-byte loads and stores over its 16-byte-aligned body, scalar at the ends
+        // (each element is still one float32 subtraction)
+        const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+        const uint64_t end = s + d.W < d.N ? s + d.W : d.N;
+        for (uint32_t c = warp; c < d.C; c += nwarps) {
+            float* row = V + (uint64_t)c * d.N;
+            const float* tr = T + ((uint64_t)l * d.C + c) * d.W - s;   // tr[x] = T[l][c][x - s]
+            // first index at a 16-byte-aligned address (the row is float-aligned)
+            const uint64_t mis = (reinterpret_cast<uintptr_t>(row + s) >> 2) & 3u;
+            uint64_t a = s + ((4u - mis) & 3u);
+            a = a < end ? a : end;
+            const uint64_t b = a + ((end - a) & ~3ull);                    // end of the aligned body
+            for (uint64_t x = s + lane; x < a; x += 32) row[x] = fsub(row[x], tr[x]);
+            for (uint64_t x = a + 4ull * lane; x < b; x += 128) {
+                float4 v = *reinterpret_cast<float4*>(row + x);
+                v.x = fsub(v.x, tr[x]);
+                v.y = fsub(v.y, tr[x + 1]);
+                v.z = fsub(v.z, tr[x + 2]);
+                v.w = fsub(v.w, tr[x + 3]);
+                *reinterpret_cast<float4*>(row + x) = v;
             }
-            __syncthreads();
+            for (uint64_t x = b + lane; x < end; x += 32) row[x] = fsub(row[x], tr[x]);
         }
-        __syncthreads();
     }
+    // the last CTA takes the spikes left over
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&status->residual_done, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (*(volatile uint32_t*)&status->n_conf) residual_ordered(d, V, T, idx, lab, n, conf);
 }
 
 // get_adjusted_clips (binary_pursuit.cl:1088-1130)
@@ -945,8 +1008,22 @@ int launch_argmax(const Dims& d, const Work& w, const uint32_t* list, uint32_t n
 int launch_compact_flagged(const Dims& d, const Work& w, uint32_t nlist, cudaStream_t st)
 {
     (void)d;
-    FlagF f{w.list(), w.orech(), w.flag()};
-    return compact(f, nullptr, nlist, w.blk(), &w.status()->n_flag, st);
+    return compact(FlagF{w.list(), w.orech(), w.flag(), w.keys()}, w, 0, nlist, &w.status()->n_flag, st);
+}
+
+int launch_argmax_lazy(const Dims& d, const Work& w, uint32_t nlist, bool overlap, cudaStream_t st)
+{
+    if (nlist == 0) return FBP_OK;
+    const Layout& L = *w.lay;
+    const ArgmaxLazy a{d, w.list(), w.at<unsigned long long>(L.off_wkey), w.at<uint8_t>(L.off_wpos), w.best_lik(),
+                       w.best_lab(), w.best_idx(), w.check(), w.orech(), w.ov_idx(), w.ov_lab()};
+    if (overlap)
+        return compact(ArgmaxFlagF{a, FlagF{w.list(), w.orech(), w.flag(), w.keys()}}, w, 0, nlist,
+                       &w.status()->n_flag, st);
+    count_launch();
+    argmax_lazy_kernel<<<grid_for(nlist, 256, 148 * 16), 256, 0, st>>>(a, nlist);
+    FBP_CUDA(cudaGetLastError());
+    return FBP_OK;
 }
 
 int launch_overlap_plain(const Dims& d, const Work& w, const float* V, const float* T, const float* theta,
@@ -960,7 +1037,6 @@ int launch_overlap_plain(const Dims& d, const Work& w, const float* V, const flo
     smem += (size_t)kOvRound * 4 + 16;
     if (smem > 220 * 1024) return fail(FBP_E_ARG, "overlap recheck working set exceeds shared memory");
     FBP_CUDA(allow_max_dyn_smem(overlap_plain_kernel));
-    FBP_CUDA(cudaMemsetAsync(w.keys(), 0, sizeof(unsigned long long) * nflag_max, st));
     const uint64_t tasks = (uint64_t)nflag_max * d.M;
     const uint32_t grid = (uint32_t)(tasks < 148ull * 8 ? tasks : 148ull * 8);
     count_launch();
@@ -983,53 +1059,44 @@ int launch_parse_reassign(const Dims& d, const Work& w, const float* theta, uint
         z.wflag = w.at<uint8_t>(w.lay->off_wflag);
         z.tnorm = w.at<float>(w.lay->off_tnorm);
     }
-    count_launch(5);
+    count_launch(3);
     parse_kernel<<<gw, 256, 0, st>>>(d, w.L(), theta, w.flag(), w.status(), w.keys(), w.best_lik(),
                                     w.best_lab(), w.best_idx(), w.orech(), w.ov_idx(), w.ov_lab(), z);
-    reassign_resolve_kernel<<<g, 256, 0, st>>>(d, w.flag(), w.status(), w.orech(), w.ov_idx(), w.orech_fin());
-    reassign_apply_kernel<<<g, 256, 0, st>>>(d, w.flag(), w.status(), w.orech(), w.orech_fin(), w.best_idx(),
-                                             w.best_lab(), w.check(), w.ov_idx(), w.ov_lab());
-    reassign_sequential_kernel<<<1, 32, 0, st>>>(d, w.flag(), w.status(), w.orech(), w.best_idx(), w.best_lab(),
-                                                  w.check(), w.ov_idx(), w.ov_lab());
-    reassign_commit_kernel<<<g, 256, 0, st>>>(w.flag(), w.status(), w.orech(), w.orech_fin());
+    reassign_kernel<<<g, 256, 0, st>>>(d, w.flag(), w.status(), w.orech(), w.orech_fin(), w.best_idx(), w.best_lab(),
+                                       w.check(), w.ov_idx(), w.ov_lab());
+    reassign_commit_kernel<<<g, 256, 0, st>>>(d, w.flag(), w.status(), w.orech(), w.orech_fin(), w.best_idx(),
+                                              w.best_lab(), w.check(), w.ov_idx(), w.ov_lab());
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
 
-int launch_accept(const Dims& d, const Work& w, const float* theta, uint32_t nlist, cudaStream_t st)
+int launch_accept(const Dims& d, const Work& w, const float* theta, uint32_t nlist,
+                  cudaStream_t st)
 {
-    if (nlist == 0) {
-        FBP_CUDA(cudaMemsetAsync(&w.status()->n_spikes, 0, 4, st));
-        return FBP_OK;
-    }
-    const uint32_t g = grid_for(nlist, 256);
-    count_launch(4);
-    accept_decide_kernel<<<g, 256, 0, st>>>(d, w.list(), nlist, theta, w.best_lik(), w.best_lab(),
-                                            w.best_idx(), w.orech(), w.has());
-    AcceptCtx cx{d, w.list(), nlist, w.has(), w.check(), w.best_lik(), w.best_lab(), w.best_idx(), theta};
-    accept_prune_kernel<<<g, 256, 0, st>>>(cx, w.newval(), w.status());
-    accept_prune_sequential_kernel<<<1, 32, 0, st>>>(cx, w.newval(), w.status());
-    accept_write_kernel<<<g, 256, 0, st>>>(cx, w.newval(), w.check());
+    if (nlist == 0) return FBP_OK;
+    count_launch(2);
+    const AcceptCtx cx{d, w.list(), nlist, w.orech(), w.check(), w.best_lik(), w.best_lab(), w.best_idx(), theta};
+    accept_kernel<<<grid_for(nlist, 256), 256, 0, st>>>(cx, w.has(), w.newval(), w.status());
+    accept_sequential_kernel<<<1, 32, 0, st>>>(cx, w.newval(), w.status());
     FBP_CUDA(cudaGetLastError());
-    SpikeF f{w.list(), w.has(), w.best_idx(), w.best_lab(), w.pidx(), w.plab(), w.pwin()};
-    return compact(f, nullptr, nlist, w.blk(), &w.status()->n_spikes, st);
+    return compact(SpikeF{cx, w.has(), w.newval(), w.check(), w.pidx(), w.plab(), w.pwin()}, w, 1, nlist,
+                   &w.status()->n_spikes, st);
 }
 
 int launch_next_list(const Dims& d, const Work& w, cudaStream_t st)
 {
-    NextF f{w.check(), w.list2()};
-    return compact(f, nullptr, d.nw, w.blk(), &w.status()->n_next, st);
+    return compact(NextF{w.check(), w.orech(), w.list2()}, w, 2, d.nw, &w.status()->n_next, st);
 }
 
 int launch_residual(const Dims& d, const Work& w, float* V, const float* T, const uint32_t* idx,
-                    const uint32_t* lab, const uint32_t* win, uint32_t n, cudaStream_t st)
+                    const uint32_t* lab, const uint32_t* win, uint32_t n, cudaStream_t st, uint32_t* out_idx,
+                    uint32_t* out_lab)
 {
     if (n == 0) return FBP_OK;
     const uint32_t back = 4 + 2 * ((d.S + d.W - 1) / d.W);
-    FBP_CUDA(cudaMemsetAsync(&w.status()->n_conf, 0, 4, st));
-    count_launch(2);
-    residual_parallel_kernel<<<n, 128, 0, st>>>(d, V, T, idx, lab, win, n, back, w.pconf(), &w.status()->n_conf);
-    residual_ordered_kernel<<<1, 1024, 0, st>>>(d, V, T, idx, lab, n, w.pconf(), &w.status()->n_conf);
+    FBP_CUDA(cudaMemsetAsync(&w.status()->n_conf, 0, 8, st));   // and residual_done
+    count_launch();
+    residual_kernel<<<n, 128, 0, st>>>(d, V, T, idx, lab, win, n, back, w.pconf(), w.status(), out_idx, out_lab);
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }

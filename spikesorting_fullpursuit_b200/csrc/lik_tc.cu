@@ -1122,47 +1122,6 @@ __global__ void __launch_bounds__(256) fixup_kernel(Dims d, const float* __restr
     }
 }
 
-// Per-window argmax from the window keys (compute_template_maximum_likelihood,
-// binary_pursuit.cl:350-441): the maximum over the 3-window span of listed window
-// id is the best of the maxima of windows id-1, id and id+1, compared by value,
-// then template, then sample (the span's first maximum in template-major order).
-// The flags and outputs are those of argmax_kernel.
-__global__ void argmax_lazy_kernel(Dims d, const uint32_t* __restrict__ list, uint32_t nlist,
-                                   const unsigned long long* __restrict__ wkey, const uint8_t* __restrict__ wpos,
-                                   float* best_lik, uint32_t* best_lab, uint32_t* best_idx, uint8_t* check,
-                                   uint8_t* orech, uint32_t* ov_idx, uint32_t* ov_lab)
-{
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nlist; k += gridDim.x * blockDim.x) {
-        const uint32_t id = list[k];
-        const uint64_t start = (uint64_t)id * d.W, end = start + d.W;
-        if (end >= (uint64_t)d.N - d.W) continue;
-        bool have = false;
-        float bv = 0.f;
-        uint32_t bt = 0, bs = 0;
-        const uint32_t x0 = id > 0 ? id - 1 : 0;
-        for (uint32_t x = x0; x <= id + 1; ++x) {   // id + 1 < nw: end + W < N
-            const unsigned long long key = wkey[x];
-            if (key == 0ull) continue;
-            const float v = __uint_as_float((uint32_t)(key >> 32));
-            const uint32_t code = 0xFFFFFFFFu - (uint32_t)key;
-            const uint32_t t = code >> 10, s = x * d.W + (code & 1023u);
-            if (!have || v > bv || (v == bv && (t < bt || (t == bt && s < bs)))) {
-                have = true; bv = v; bt = t; bs = s;
-            }
-        }
-        if (wpos[id]) check[id] = 1;
-        uint32_t lab = best_lab[id], idx = best_idx[id];
-        float bl = 0.f;
-        if (have) { bl = bv; lab = bt; idx = bs; }
-        orech[id] = (bl > 0.f && idx >= start && idx < end) ? 1 : 0;
-        best_lik[id] = bl;
-        best_lab[id] = lab;
-        best_idx[id] = idx;
-        ov_idx[id] = idx;
-        ov_lab[id] = lab;
-    }
-}
-
 // Before a pass's residual: the positive values of flagged (window, template)
 // rows -- rows that may hold estimates -- of windows whose voltage the residual
 // changes and which the next pass does not recompute (check == 0 once the pass's
@@ -1324,19 +1283,6 @@ bool tc_supported(const Dims& d)
 {
     TcConfig c;
     return tc_config(d, &c);
-}
-
-int launch_argmax_lazy(const Dims& d, const Work& w, const uint32_t* list, uint32_t nlist, cudaStream_t st)
-{
-    if (nlist == 0) return FBP_OK;
-    const Layout& L = *w.lay;
-    count_launch();
-    const uint32_t grid = std::min<uint32_t>((nlist + 255) / 256, 148 * 16);
-    argmax_lazy_kernel<<<grid, 256, 0, st>>>(d, list, nlist, w.at<unsigned long long>(L.off_wkey),
-                                             w.at<uint8_t>(L.off_wpos), w.best_lik(), w.best_lab(), w.best_idx(),
-                                             w.check(), w.orech(), w.ov_idx(), w.ov_lab());
-    FBP_CUDA(cudaGetLastError());
-    return FBP_OK;
 }
 
 int launch_lazy_fix(const Dims& d, const Work& w, const float* V, const float* T, const float* bias,
@@ -1517,11 +1463,8 @@ int launch_likelihood_tc(const Dims& d, const Work& w, const float* V, const flo
     P.wpos = lazy ? w.at<uint8_t>(L.off_wpos) : nullptr;
     P.wflag = lazy ? w.at<uint8_t>(L.off_wflag) : nullptr;
     P.wslots = win_slots(d.W);
-    if (lazy && all && tile0 == 0) {
-        FBP_CUDA(cudaMemsetAsync(P.wkey, 0, (size_t)d.nw * 8, st));
-        FBP_CUDA(cudaMemsetAsync(P.wpos, 0, (size_t)d.nw, st));
-        FBP_CUDA(cudaMemsetAsync(P.wflag, 0, (size_t)d.nw * d.M, st));
-    }
+    if (lazy && all && tile0 == 0)   // window keys, positive flags, estimate flags
+        FBP_CUDA(cudaMemsetAsync(P.wkey, 0, L.off_wflag + L.nw * L.M - L.off_wkey, st));
     FBP_CUDA(cudaMemsetAsync(&w.status()->n_fix, 0, 4, st));
     PersistConfig pc;
     count_launch();

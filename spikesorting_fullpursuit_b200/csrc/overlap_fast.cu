@@ -1145,7 +1145,6 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
     if (nflag_max == 0) return FBP_OK;
     const uint32_t S2 = 2 * d.S + 1;
     if (S2 > 1024 || d.C > 256 || d.M > 4096) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
-    FBP_CUDA(cudaMemsetAsync(w.keys(), 0, sizeof(unsigned long long) * nflag_max, st));
     const PcConfig pc = pc_config();
     const int Q = pc.Q;
     const size_t smem_a = pc.smem;
@@ -1219,7 +1218,7 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
         uint32_t* order = w.at<uint32_t>(L.off_order);
         count_launch();
         label_order_kernel<<<1, 1024, (d.M + 1) * 4, st>>>(d, w.flag(), w.status(), w.best_lab(), k0, kc, order);
-        FBP_CUDA(cudaMemsetAsync(&w.status()->cand_count, 0, 4, st));
+        if (k0 > 0) FBP_CUDA(cudaMemsetAsync(&w.status()->cand_count, 0, 4, st));   // the pass starts with 0
         {
         KScope ks(&fbp_chunk_stats::ms_screen, st);
         P.k0 = k0;

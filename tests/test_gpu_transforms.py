@@ -84,3 +84,17 @@ def test_many_similar_units_on_the_same_channels(amp):
                                         rate_model=("uniform", 5.0, 15.0), overlap_frac=0.5, amp=amp)
     si["get_adjusted_clips"] = True
     _same_as_oracle(V, si, sm, si["n_samples_per_chan"] - 1)
+
+
+@pytest.mark.parametrize("recheck", [True, False])
+@pytest.mark.parametrize("windows", [1024, 1025, 33 * 1024 + 5, 70 * 1024 - 1])
+def test_window_lists_over_many_tiles(windows, recheck):
+    """The passes' lists are compacted in tiles of 1024 windows, each looking back over the
+    tiles before it, 32 at a time."""
+    fs, W = 20000, 9
+    V, si, sm, _ = synth.make_recording(windows, n_chans=1, fs=fs, duration_s=windows * W / fs, n_units=3,
+                                        rate_model=("uniform", 60.0, 120.0), overlap_frac=0.2,
+                                        clip_width=(-3.25 / fs, 4.75 / fs))
+    assert si["n_samples_per_chan"] == W and abs(V.shape[1] - windows * W) <= W
+    si["do_overlap_recheck"] = recheck
+    _same_as_oracle(V, si, sm, W - 1)
