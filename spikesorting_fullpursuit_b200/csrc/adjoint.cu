@@ -13,13 +13,18 @@
 //     dE/dtau_k   = -2 a_k sgn(tau_k) sum_{c,j} (T(c, j + dir) - T(c, j)) r(c, s_k + j)
 //                   (sgn(0) = +1: the tau >= 0 branch)
 //     dE/dT_l(c,i)= -2 sum_{k: l_k = l} a_k ((1 - u) r(c, s_k + i) + u r(c, s_k + i - dir))
-// Nothing is stored between the loss and the gradient: each CTA rebuilds its
-// spike's residual tile r(:, [s_k - 1, s_k + W]) in FP64 from the voltage and
-// every spike whose support meets the tile (spikes sorted by onset; the
-// neighbours are found by binary search).  Sums run in FP64; template gradients
-// accumulate with FP64 atomics.  The loss is sum v^2 plus, for every modelled
-// sample, r^2 - v^2 counted once, by the first spike (in onset order) whose
-// support holds it.
+// Nothing is stored between the loss and the gradient: residual values are rebuilt in
+// FP64 registers from the voltage and every spike whose support meets them (spikes
+// sorted by onset).  A warp takes 128 samples of one channel, four a lane, and the
+// spikes one after the other in onset order; a template row that is zero there is
+// left out (its product is exactly 0; not when amplitude or shift is not finite).
+// Sums run in FP64; template gradients accumulate with FP64 atomics.
+//
+// Bound by instruction issue: one CTA a spike over a (channel, sample) index with a
+// division and 64-bit compares an element took 469 us for the loss (and 122 us more
+// for the sum of v^2) and 521 us for the gradient at 16 channels x 60 s, 19200 spikes of
+// 101 samples, with the FP64 pipe 6-9% and the L2's atomics 9% busy; as here: 137 us and
+// 242 us.
 #include <cub/cub.cuh>
 
 #include "fbp_internal.cuh"
@@ -40,136 +45,239 @@ struct AdjArgs {
     uint32_t n;
 };
 
-__device__ __forceinline__ double tshift(const float* Tc, int W, double u, int dir, int j)
+constexpr int kAdjWarps = kAdjThreads / 32;
+constexpr int kAdjCols = 4;                 // columns a lane
+constexpr int kAdjSpan = 32 * kAdjCols;     // columns a warp
+
+// One spike as a warp's rows meet it
+struct AdjSpike {
+    double a, u;      // amplitude, |shift|
+    int32_t off;      // column of the template's sample 0
+    int32_t dir;      // -1 or +1
+    uint32_t lab;
+    uint32_t finite;  // amplitude and shift are finite
+};
+
+__device__ __forceinline__ AdjSpike adj_spike(const AdjArgs& A, uint32_t k, int64_t x0)
 {
-    const double a = (j >= 0 && j < W) ? (double)Tc[j] : 0.0;
-    const int jj = j + dir;
-    const double b = (jj >= 0 && jj < W) ? (double)Tc[jj] : 0.0;
-    return (1.0 - u) * a + u * b;
+    AdjSpike s;
+    const double t = A.tau[k];
+    s.a = A.amp[k];
+    s.u = t >= 0.0 ? t : -t;
+    s.dir = t >= 0.0 ? -1 : 1;
+    s.off = (int32_t)((int64_t)A.idx[k] - x0);
+    s.lab = A.lab[k];
+    s.finite = isfinite(s.a) && isfinite(s.u);
+    return s;
 }
 
-// first spike with onset >= key
-__device__ uint32_t lower_bound(const uint32_t* idx, uint32_t n, int64_t key)
+// first spike with onset >= key (a warp, 32 probes a step)
+__device__ uint32_t first_onset(const AdjArgs& A, int64_t key)
 {
-    uint32_t lo = 0, hi = n;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = A.n;   // below lo: onset < key; from hi on: >= key
     while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((int64_t)idx[mid] < key) lo = mid + 1; else hi = mid;
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint64_t at = (uint64_t)lo + (uint64_t)lane * step;
+        const bool less = at < hi && (int64_t)A.idx[at] < key;
+        const uint32_t c = __popc(__ballot_sync(0xffffffffu, less));   // probes 0 .. c-1 are below
+        if (c == 0) return lo;
+        const uint64_t top = (uint64_t)lo + (uint64_t)c * step;
+        lo = lo + (c - 1) * step + 1;
+        hi = top < hi ? (uint32_t)top : hi;
     }
     return lo;
 }
 
-// Residual tile of spike k: r[c][x - (s_k - 1)] for x in [s_k - 1, s_k + W], all
-// channels, in FP64 shared memory (samples outside [0, N) left at 0).
-__device__ void residual_tile(const AdjArgs& A, uint32_t k, double* r)
+// r[i] = residual of channel c at sample x0 + lane + 32 i (0 outside [0, N)), from
+// the spikes [k0, k1); `box` is the warp's, and holds those spikes already if `held`.
+__device__ __forceinline__ void residual_row(const AdjArgs& A, uint32_t c, int64_t x0, uint32_t k0, uint32_t k1,
+                                             AdjSpike* box, bool held, double (&r)[kAdjCols])
 {
-    const int W = (int)A.W, TL = W + 2;
-    const int64_t x0 = (int64_t)A.idx[k] - 1;
-    for (int e = threadIdx.x; e < (int)A.C * TL; e += blockDim.x) {
-        const int c = e / TL, q = e - c * TL;
-        const int64_t x = x0 + q;
-        r[e] = (x >= 0 && x < (int64_t)A.N) ? (double)A.V[(uint64_t)c * A.N + x] : 0.0;
+    const int lane = threadIdx.x & 31;
+    const float* v = A.V + ((int64_t)((uint64_t)c * A.N) + x0 + lane);
+    // columns [first, last) are samples of the recording
+    const int first = x0 < 0 ? (int)-x0 : 0;
+    const int last = x0 + kAdjSpan <= (int64_t)A.N ? kAdjSpan : (int)max((int64_t)A.N - x0, (int64_t)0);
+#pragma unroll
+    for (int i = 0; i < kAdjCols; ++i) {
+        const int q = lane + 32 * i;
+        r[i] = q >= first && q < last ? (double)v[32 * i] : 0.0;
     }
-    __syncthreads();
-    const uint32_t k_lo = lower_bound(A.idx, A.n, (int64_t)A.idx[k] - W - 1);
-    const uint32_t k_hi = lower_bound(A.idx, A.n, (int64_t)A.idx[k] + W + 2);
-    for (uint32_t kk = k_lo; kk < k_hi; ++kk) {
-        const uint32_t l = A.lab[kk];
-        if (l >= A.M) continue;
-        const double a = A.amp[kk], t = A.tau[kk];
-        const double u = t >= 0.0 ? t : -t;
-        const int dir = t >= 0.0 ? -1 : 1;
-        const int64_t off = (int64_t)A.idx[kk] - x0;   // tile column of the neighbour's j = 0
-        for (int e = threadIdx.x; e < (int)A.C * TL; e += blockDim.x) {
-            const int c = e / TL, q = e - c * TL;
-            const int64_t x = x0 + q;
-            const int j = (int)(q - off);
-            if (j < -1 || j > W || x < 0 || x >= (int64_t)A.N) continue;
-            r[e] -= a * tshift(A.T + ((uint64_t)l * A.C + c) * A.W, W, u, dir, j);
+    for (uint32_t kb = k0; kb < k1; kb += 32) {
+        const uint32_t m = min(32u, k1 - kb);
+        if (!held) {
+            __syncwarp();
+            if (lane < (int)m) box[lane] = adj_spike(A, kb + lane, x0);
+            __syncwarp();
         }
-        __syncthreads();
+        for (uint32_t i0 = 0; i0 < m; ++i0) {
+            const AdjSpike s = box[i0];
+            if (s.lab >= A.M) continue;
+            const float* Tc = A.T + ((uint64_t)s.lab * A.C + c) * A.W;
+            float ta[kAdjCols], tb[kAdjCols];   // zero outside the support
+            bool some = !s.finite;
+            const int j0 = lane - s.off;
+            const float *pa = Tc + j0, *pb = pa + s.dir;
+#pragma unroll
+            for (int i = 0; i < kAdjCols; ++i) {
+                const int j = j0 + 32 * i;
+                ta[i] = (uint32_t)j < A.W ? pa[32 * i] : 0.f;
+                tb[i] = (uint32_t)(j + s.dir) < A.W ? pb[32 * i] : 0.f;
+                some |= ta[i] != 0.f || tb[i] != 0.f;
+            }
+            if (!__any_sync(0xffffffffu, some)) continue;
+#pragma unroll
+            for (int i = 0; i < kAdjCols; ++i)
+                if (s.finite || (uint32_t)(j0 + 32 * i + 1) < A.W + 2)
+                    r[i] -= s.a * ((1.0 - s.u) * (double)ta[i] + s.u * (double)tb[i]);
+        }
+    }
+    if (first > 0 || last < kAdjSpan) {
+#pragma unroll
+        for (int i = 0; i < kAdjCols; ++i) {
+            const int q = lane + 32 * i;
+            if (q < first || q >= last) r[i] = 0.0;
+        }
     }
 }
 
+// E: a warp takes 128 samples of all channels at a time.
 __global__ void __launch_bounds__(kAdjThreads) adjoint_loss_kernel(AdjArgs A, double* loss)
 {
-    extern __shared__ double r[];
     typedef cub::BlockReduce<double, kAdjThreads> R;
     __shared__ typename R::TempStorage tmp;
-    const int W = (int)A.W, TL = W + 2;
+    __shared__ AdjSpike box[kAdjWarps][32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t nseg = ((uint64_t)A.N + kAdjSpan - 1) / kAdjSpan;
     double acc = 0.0;
-    for (uint32_t k = blockIdx.x; k < A.n; k += gridDim.x) {
-        __syncthreads();
-        residual_tile(A, k, r);
-        const int64_t x0 = (int64_t)A.idx[k] - 1;
-        // samples owned by this spike: not covered by an earlier one (the previous
-        // spike in onset order has the furthest-reaching earlier support)
-        const int64_t first = k > 0 ? (int64_t)A.idx[k - 1] + W + 1 : INT64_MIN;
-        for (int e = threadIdx.x; e < (int)A.C * TL; e += blockDim.x) {
-            const int c = e / TL, q = e - c * TL;
-            const int64_t x = x0 + q;
-            if (x < 0 || x >= (int64_t)A.N || x < first) continue;
-            const double v = A.V[(uint64_t)c * A.N + x];
-            acc += r[e] * r[e] - v * v;
+    for (uint64_t g = (uint64_t)blockIdx.x * kAdjWarps + warp; g < nseg; g += (uint64_t)gridDim.x * kAdjWarps) {
+        const int64_t x0 = (int64_t)(g * kAdjSpan);
+        const uint32_t k0 = first_onset(A, x0 - (int64_t)A.W);
+        uint32_t k1 = k0;   // past the last spike with onset <= x0 + 128
+        for (;;) {
+            const bool meets = (uint64_t)k1 + lane < A.n && (int64_t)A.idx[k1 + lane] <= x0 + kAdjSpan;
+            const uint32_t ones = __popc(__ballot_sync(0xffffffffu, meets));
+            k1 += ones;
+            if (ones < 32) break;
+        }
+        const bool one = k1 - k0 <= 32;
+        if (one) {
+            __syncwarp();
+            if (lane < k1 - k0) box[warp][lane] = adj_spike(A, k0 + lane, x0);
+            __syncwarp();
+        }
+        for (uint32_t c = 0; c < A.C; ++c) {
+            double r[kAdjCols];
+            residual_row(A, c, x0, k0, k1, box[warp], one, r);
+#pragma unroll
+            for (int i = 0; i < kAdjCols; ++i) acc += r[i] * r[i];
         }
     }
     const double s = R(tmp).Sum(acc);
-    if (threadIdx.x == 0 && s != 0.0) atomicAdd(loss, s);
+    if (threadIdx.x == 0) atomicAdd(loss, s);
 }
 
-__global__ void sumsq_kernel(const float* __restrict__ V, uint64_t n, double* out)
-{
-    typedef cub::BlockReduce<double, 256> R;
-    __shared__ typename R::TempStorage tmp;
-    double acc = 0.0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const double v = V[i];
-        acc += v * v;
-    }
-    const double s = R(tmp).Sum(acc);
-    if (threadIdx.x == 0) atomicAdd(out, s);
-}
-
-__global__ void __launch_bounds__(kAdjThreads) adjoint_grad_kernel(AdjArgs A, double scale, double* gT, float* g_amp,
+// A CTA takes a spike, a warp every fourth channel; a row's W + 2 columns are taken 126
+// at a time, with one more on either side for the shifted residual.
+__global__ void __launch_bounds__(kAdjThreads, 8) adjoint_grad_kernel(AdjArgs A, double scale, double* gT, float* g_amp,
                                                                   float* g_tau)
 {
-    extern __shared__ double r[];
-    typedef cub::BlockReduce<double, kAdjThreads> R;
-    __shared__ typename R::TempStorage tmp;
+    __shared__ AdjSpike box[kAdjWarps][32];
+    __shared__ double part[2][kAdjWarps];
     const int W = (int)A.W, TL = W + 2;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (uint32_t k = blockIdx.x; k < A.n; k += gridDim.x) {
-        __syncthreads();
-        residual_tile(A, k, r);
+        const int64_t s = A.idx[k];
         const uint32_t l = A.lab[k];
         double da = 0.0, dt = 0.0;
         if (l < A.M) {
-            const double a = A.amp[k], t = A.tau[k];
-            const double u = t >= 0.0 ? t : -t;
-            const int dir = t >= 0.0 ? -1 : 1;
-            const double sg = t >= 0.0 ? 1.0 : -1.0;
-            for (int e = threadIdx.x; e < (int)A.C * TL; e += blockDim.x) {
-                const int c = e / TL, q = e - c * TL;
-                const int j = q - 1;
-                const float* Tc = A.T + ((uint64_t)l * A.C + c) * A.W;
-                const double ts = tshift(Tc, W, u, dir, j);
-                const double tj = (j >= 0 && j < W) ? (double)Tc[j] : 0.0;
-                const int jj = j + dir;
-                const double td = (jj >= 0 && jj < W) ? (double)Tc[jj] : 0.0;
-                da += ts * r[e];
-                dt += (td - tj) * r[e];
-                // template sample i = j: (1 - u) r(s + i) + u r(s + i - dir)
-                if (j >= 0 && j < W) {
-                    const int q2 = q - dir;   // tile column of s + i - dir, in [0, TL)
-                    const double g = (1.0 - u) * r[e] + u * r[c * TL + q2];
-                    atomicAdd(&gT[((uint64_t)l * A.C + c) * A.W + j], -2.0 * scale * a * g);
+            const AdjSpike own = adj_spike(A, k, 0);
+            uint32_t k0 = k, k1 = k + 1;   // the spikes whose support meets [s - 1, s + W]
+            for (;;) {
+                const bool meets = k0 > lane && (int64_t)A.idx[k0 - 1 - lane] >= s - W - 1;
+                const uint32_t ones = __popc(__ballot_sync(0xffffffffu, meets));
+                k0 -= ones;
+                if (ones < 32) break;
+            }
+            for (;;) {
+                const bool meets = (uint64_t)k1 + lane < A.n && (int64_t)A.idx[k1 + lane] <= s + W + 1;
+                const uint32_t ones = __popc(__ballot_sync(0xffffffffu, meets));
+                k1 += ones;
+                if (ones < 32) break;
+            }
+            for (int q0 = 0; q0 < TL; q0 += kAdjSpan - 2) {
+                const int64_t x0 = s - 2 + q0;   // column 0 of the row; its column p is the tile's q0 - 1 + p
+                const bool one = k1 - k0 <= 32;
+                if (one) {
+                    __syncwarp();
+                    if (lane < k1 - k0) box[warp][lane] = adj_spike(A, k0 + lane, x0);
+                    __syncwarp();
+                }
+                for (uint32_t c = warp; c < A.C; c += kAdjWarps) {
+                    double r[kAdjCols];
+                    residual_row(A, c, x0, k0, k1, box[warp], one, r);
+                    const int j0 = q0 + (int)lane - 2;   // template sample of column `lane`
+                    const float* pa = A.T + ((uint64_t)l * A.C + c) * A.W + j0;
+                    const float* pb = pa + own.dir;
+                    double* gc = gT + ((uint64_t)l * A.C + c) * A.W + j0;
+                    float ta[kAdjCols], tb[kAdjCols];
+                    bool some = false;
+                    double next[kAdjCols];   // the column at q - dir
+#pragma unroll
+                    for (int i = 0; i < kAdjCols; ++i) {
+                        const int j = j0 + 32 * i;
+                        ta[i] = (uint32_t)j < A.W ? pa[32 * i] : 0.f;
+                        tb[i] = (uint32_t)(j + own.dir) < A.W ? pb[32 * i] : 0.f;
+                        some |= ta[i] != 0.f || tb[i] != 0.f || !isfinite(r[i]);
+                        next[i] = __shfl_sync(0xffffffffu, r[i], (lane - own.dir) & 31);
+                    }
+                    if (own.dir < 0) {
+#pragma unroll
+                        for (int i = 0; i < kAdjCols; ++i)
+                            if (lane == 31) next[i] = i + 1 < kAdjCols ? next[i + 1 < kAdjCols ? i + 1 : i] : 0.0;
+                    } else {
+#pragma unroll
+                        for (int i = kAdjCols - 1; i >= 0; --i)
+                            if (lane == 0) next[i] = i > 0 ? next[i > 0 ? i - 1 : 0] : 0.0;
+                    }
+                    if (__any_sync(0xffffffffu, some)) {
+#pragma unroll
+                        for (int i = 0; i < kAdjCols; ++i) {
+                            const int p = lane + 32 * i;
+                            if (p < 1 || p > kAdjSpan - 2 || j0 + 32 * i > W) continue;
+                            da += ((1.0 - own.u) * (double)ta[i] + own.u * (double)tb[i]) * r[i];
+                            dt += ((double)tb[i] - (double)ta[i]) * r[i];
+                        }
+                    }
+                    // template sample j: (1 - u) r(s + j) + u r(s + j - dir)
+#pragma unroll
+                    for (int i = 0; i < kAdjCols; ++i) {
+                        const int p = lane + 32 * i;
+                        if (p >= 1 && p <= kAdjSpan - 2 && (uint32_t)(j0 + 32 * i) < A.W)
+                            atomicAdd(&gc[32 * i], -2.0 * scale * own.a * ((1.0 - own.u) * r[i] + own.u * next[i]));
+                    }
                 }
             }
-            dt *= sg * a;
+            dt *= -own.dir * own.a;   // sgn(tau) = -dir
         }
-        const double sa = R(tmp).Sum(da);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            da += __shfl_down_sync(0xffffffffu, da, o);
+            dt += __shfl_down_sync(0xffffffffu, dt, o);
+        }
+        __syncthreads();   // the previous spike's sums have been read
+        if (lane == 0) {
+            part[0][warp] = da;
+            part[1][warp] = dt;
+        }
         __syncthreads();
-        const double st = R(tmp).Sum(dt);
         if (threadIdx.x == 0) {
+            double sa = 0.0, st = 0.0;
+            for (int w = 0; w < kAdjWarps; ++w) {
+                sa += part[0][w];
+                st += part[1][w];
+            }
             g_amp[k] = (float)(-2.0 * scale * sa);
             g_tau[k] = (float)(-2.0 * scale * st);
         }
@@ -230,13 +338,8 @@ extern "C" int fbp_adjoint_loss(const fbp_dims* dims, const float* voltage, cons
     const AdjArgs A = adj_args(dims, voltage, templates, spike_idx, spike_lab, amplitude, shift, n_spikes);
     FBP_CUDA(cudaMemsetAsync(loss, 0, sizeof(double), st));
     count_launch();
-    sumsq_kernel<<<148 * 4, 256, 0, st>>>(voltage, (uint64_t)A.C * A.N, loss);
-    if (n_spikes) {
-        const size_t smem = (size_t)A.C * (A.W + 2) * sizeof(double);
-        FBP_CUDA(allow_max_dyn_smem(adjoint_loss_kernel));
-        count_launch();
-        adjoint_loss_kernel<<<n_spikes < 148u * 16 ? n_spikes : 148u * 16, kAdjThreads, smem, st>>>(A, loss);
-    }
+    const uint64_t blocks = ((uint64_t)A.N + kAdjSpan * kAdjWarps - 1) / (kAdjSpan * kAdjWarps);
+    adjoint_loss_kernel<<<blocks < 148u * 16 ? (uint32_t)blocks : 148u * 16, kAdjThreads, 0, st>>>(A, loss);
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -256,10 +359,8 @@ extern "C" int fbp_adjoint_grad(const fbp_dims* dims, const float* voltage, cons
     const uint64_t nt = (uint64_t)A.M * A.C * A.W;
     FBP_CUDA(cudaMemsetAsync(grad_templates64, 0, nt * sizeof(double), st));
     if (n_spikes) {
-        const size_t smem = (size_t)A.C * (A.W + 2) * sizeof(double);
-        FBP_CUDA(allow_max_dyn_smem(adjoint_grad_kernel));
         count_launch();
-        adjoint_grad_kernel<<<n_spikes < 148u * 16 ? n_spikes : 148u * 16, kAdjThreads, smem, st>>>(
+        adjoint_grad_kernel<<<n_spikes < 148u * 16 ? n_spikes : 148u * 16, kAdjThreads, 0, st>>>(
             A, scale, grad_templates64, grad_amplitude, grad_shift);
     }
     count_launch();

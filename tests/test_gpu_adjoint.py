@@ -82,3 +82,20 @@ def test_adjoint_no_spikes_is_voltage_energy():
                         torch.zeros(0, dtype=torch.int64, device="cuda"),
                         torch.zeros(0, device="cuda"), torch.zeros(0, device="cuda"))
     assert abs(float(e) - float((V.astype(np.float64) ** 2).sum())) <= 1e-10 * float(e)
+
+
+@pytest.mark.parametrize("C,W,n", [(1, 1, 9), (3, 29, 40), (5, 124, 12), (4, 125, 12), (2, 126, 70), (6, 300, 50)])
+def test_adjoint_row_spans(C, W, n):
+    """Rows of one and of several 126-column steps; up to 32 and more spikes over one sample;
+    template rows that are zero; recordings that end inside a warp's 128 samples."""
+    rng = np.random.default_rng(1000 * C + W)
+    N, M = 3 * W + 133, 3
+    V = rng.standard_normal((C, N)).astype(np.float32)
+    T = rng.standard_normal((M, C, W)).astype(np.float32)
+    T[0, C // 2] = 0.0
+    T[1, 0, W // 2:] = 0.0
+    idx = np.sort(rng.integers(0, N, size=n))
+    lab = rng.integers(0, M, size=n)
+    amp = rng.normal(1.0, 0.1, size=n).astype(np.float32)
+    tau = rng.uniform(0.02, 0.9, size=n).astype(np.float32) * rng.choice([-1, 1], size=n).astype(np.float32)
+    _check(V, T, idx.astype(np.int64), lab.astype(np.int64), amp, tau)
