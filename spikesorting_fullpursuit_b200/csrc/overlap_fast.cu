@@ -85,7 +85,46 @@ __device__ __forceinline__ float warp_max(float v)
 // max -X (at least 0) per pair.  32 lags at a time: a lag is a lane, so that a warp
 // writes 32 consecutive shifts of a row (with the row index on the lanes every 4-byte
 // store was a sector of its own: 64 channels x 200 templates about 12 ms of a call).
+//
+// With few pairs the groups of lags are split over gridDim.y CTAs a pair, and the
+// bounds, which need whole rows, follow in a launch of their own: 4 channels, 6 templates,
+// 201 x 201 shifts 177 us by one CTA a pair, 17 + 12 us so.  With
+// many pairs one CTA does both, the rows then still being in the L1 and L2.
 constexpr int kCrossThreads = 256;
+
+// XC, XCT and max -X of pair `p`, rows `first`, first + step, ... (a warp a row)
+__device__ __forceinline__ void cross_bounds(const Dims& d, uint32_t p, uint32_t first, uint32_t step,
+                                             const float* XT, const float* XTT, float* XC, float* XCT, int* neg_bits)
+{
+    const uint32_t f = p / d.M, t = p % d.M, lane = threadIdx.x & 31;
+    const uint32_t S2 = 2 * d.S + 1, nch = (S2 + 31) / 32;
+    float neg = 0.f;
+    for (uint32_t e = first; e < 2 * S2; e += step) {
+        const uint32_t y = e >> 1;
+        const float* row = ((e & 1u) ? XTT : XT) + (uint64_t)p * S2 * S2 + (uint64_t)y * S2;
+        float* out = (e & 1u) ? XCT + ((uint64_t)p * S2 + y) * nch : XC + (((uint64_t)f * S2 + y) * d.M + t) * nch;
+#pragma unroll 4
+        for (uint32_t ch = 0; ch < nch; ++ch) {
+            const uint32_t x = ch * 32 + lane;
+            const bool in = x < S2 && x + d.W >= y && x <= y + d.W;
+            const float m = warp_max(in ? -row[x] : -INFINITY);
+            if (lane == 0) out[ch] = m;
+            neg = fmaxf(neg, m);
+        }
+    }
+    if (lane == 0) atomicMax(neg_bits, __float_as_int(neg));   // neg >= 0
+}
+
+__global__ void __launch_bounds__(kCrossThreads) cross_bound_kernel(Dims d,
+                                                                    const unsigned long long* __restrict__ chmask,
+                                                                    const float* XT, const float* XTT, float* XC,
+                                                                    float* XCT, float* max_negx)
+{
+    const uint32_t p = blockIdx.x, warps = kCrossThreads / 32;
+    if ((chmask[p / d.M] & chmask[p % d.M]) == 0ull) return;
+    cross_bounds(d, p, blockIdx.y * warps + (threadIdx.x >> 5), gridDim.y * warps, XT, XTT, XC, XCT,
+                 reinterpret_cast<int*>(max_negx) + p);
+}
 
 __global__ void __launch_bounds__(kCrossThreads) cross_table_kernel(Dims d, const float* __restrict__ T,
                                                                     const unsigned long long* __restrict__ chmask,
@@ -95,11 +134,11 @@ __global__ void __launch_bounds__(kCrossThreads) cross_table_kernel(Dims d, cons
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int s_neg;
     const uint32_t f = blockIdx.x / d.M, t = blockIdx.x % d.M;
-    const uint32_t S2 = 2 * d.S + 1, W = d.W, C = d.C, nch = (S2 + 31) / 32;
+    const uint32_t S2 = 2 * d.S + 1, W = d.W, C = d.C;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = kCrossThreads / 32;
     const unsigned long long both = chmask[f] & chmask[t];   // all ones above 64 channels
     if (both == 0ull) {
-        if (threadIdx.x == 0) max_negx[blockIdx.x] = 0.f;
+        if (threadIdx.x == 0 && blockIdx.y == 0) max_negx[blockIdx.x] = 0.f;
         return;
     }
     const uint32_t pitch = (W + 1) | 1u;   // odd: the lags of a warp read different banks
@@ -115,7 +154,7 @@ __global__ void __launch_bounds__(kCrossThreads) cross_table_kernel(Dims d, cons
     float* xt = XT + (uint64_t)blockIdx.x * S2 * S2;
     float* xtt = XTT + (uint64_t)blockIdx.x * S2 * S2;
     const int dmax = (int)min(W, 2 * d.S);
-    for (int d0 = -dmax; d0 <= dmax; d0 += lags) {
+    for (int d0 = -dmax + (int)blockIdx.y * lags; d0 <= dmax; d0 += (int)gridDim.y * lags) {
         for (int li = warp; li < lags; li += nwarps) {
             const int delta = d0 + li;
             double* q = Q + li * pitch;
@@ -162,21 +201,11 @@ __global__ void __launch_bounds__(kCrossThreads) cross_table_kernel(Dims d, cons
         }
         __syncthreads();
     }
-    float neg = 0.f;
-    for (uint32_t e = warp; e < 2 * S2; e += nwarps) {
-        const uint32_t y = e >> 1;
-        const float* row = ((e & 1u) ? xtt : xt) + (uint64_t)y * S2;
-        float* out = (e & 1u) ? XCT + ((uint64_t)blockIdx.x * S2 + y) * nch
-                              : XC + (((uint64_t)f * S2 + y) * d.M + t) * nch;
-        for (uint32_t ch = 0; ch < nch; ++ch) {
-            const uint32_t x = ch * 32 + lane;
-            const bool in = x < S2 && x + W >= y && x <= y + W;
-            const float m = warp_max(in ? -row[x] : -INFINITY);
-            if (lane == 0) out[ch] = m;
-            neg = fmaxf(neg, m);
-        }
+    if (gridDim.y > 1) {
+        if (threadIdx.x == 0 && blockIdx.y == 0) max_negx[blockIdx.x] = 0.f;   // cross_bound_kernel raises it
+        return;
     }
-    if (lane == 0) atomicMax(&s_neg, __float_as_int(neg));
+    cross_bounds(d, blockIdx.x, warp, nwarps, XT, XTT, XC, XCT, &s_neg);
     __syncthreads();
     if (threadIdx.x == 0) max_negx[blockIdx.x] = __int_as_float(s_neg);
 }
@@ -1083,9 +1112,16 @@ int launch_overlap_tables(const Dims& d, const Work& w, const float* T, cudaStre
     const int lags = cross_smem(32) <= 100 * 1024 ? 32 : 16;   // two CTAs per SM, or the shorter chunk
     if (cross_smem(lags) > 201 * 1024) return fail(FBP_E_ARG, "template too large for the pair table kernel");
     FBP_CUDA(allow_max_dyn_smem(cross_table_kernel));
-    cross_table_kernel<<<d.M * d.M, kCrossThreads, cross_smem(lags), st>>>(
+    const uint32_t pairs = d.M * d.M, groups = (2 * std::min(d.W, 2 * d.S) + lags) / lags;
+    const uint32_t split = std::max(1u, std::min(groups, 148u * 2 / pairs));
+    cross_table_kernel<<<dim3(pairs, split), kCrossThreads, cross_smem(lags), st>>>(
         d, T, chmask, lags, w.at<float>(L.off_xt), w.at<float>(L.off_xtt), w.at<float>(L.off_xc), w.at<float>(L.off_xct),
         mx);
+    if (split > 1) {
+        count_launch();
+        cross_bound_kernel<<<dim3(pairs, (2 * d.S + 8) / 8), kCrossThreads, 0, st>>>(   // two rows a warp
+            d, chmask, w.at<float>(L.off_xt), w.at<float>(L.off_xtt), w.at<float>(L.off_xc), w.at<float>(L.off_xct), mx);
+    }
     FBP_CUDA(cudaGetLastError());
     if (window_corr_by_fft(d)) return FBP_OK;
     count_launch();
