@@ -166,6 +166,11 @@ int fbp_pursue_chunk_staged(const fbp_dims* dims, uint32_t flags, float* voltage
                             void* const* ready_events, const uint32_t* ready_upto,
                             const uint32_t* ready_flags, uint32_t n_ready, void* stream);
 
+/* Copies `rows` rows of `width` bytes from host memory (page-locked or not) to the
+ * device in stream order; pitches in bytes, at least `width`. */
+int fbp_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width,
+                  uint32_t rows, void* stream);
+
 /* Adjusted clips: clips[k][c][j] = residual[c][idx_k + j] + templates[lab_k][c][j]
  * for idx_k + j < N, else left untouched (get_adjusted_clips,
  * binary_pursuit.cl:1088-1130).  clips is float32 [n][C*W]. */

@@ -29,7 +29,7 @@ EXPORTS = ("fbp_abi_version", "fbp_last_error", "fbp_workspace_bytes", "fbp_purs
            "fbp_adjoint_loss", "fbp_adjoint_grad", "fbp_mean_clip", "fbp_bp_duplicates_workspace",
            "fbp_bp_duplicates", "fbp_separability", "fbp_pair_separability", "fbp_gather_clips",
            "fbp_robust_template",
-           "fbp_residual_covariance", "fbp_set_tuning")
+           "fbp_residual_covariance", "fbp_set_tuning", "fbp_copy_rows")
 NOALLOC_MAX_SPIKES = 65536
 MAX_PASSES = 2048   # default pass limit of one chunk (the reference's loop has none)
 PASS_RING = 64
@@ -104,6 +104,8 @@ def lib():
     L.fbp_pursue_chunk_staged.restype = ctypes.c_int
     L.fbp_adjusted_clips.argtypes = [P(FbpDims), vp, vp, vp, vp, u32, vp, vp]
     L.fbp_adjusted_clips.restype = ctypes.c_int
+    L.fbp_copy_rows.argtypes = [vp, sz, vp, sz, sz, u32, vp]
+    L.fbp_copy_rows.restype = ctypes.c_int
     L.fbp_likelihood.argtypes = [P(FbpDims), ctypes.c_int, vp, vp, vp, vp, u32, vp, vp, sz, vp]
     L.fbp_likelihood.restype = ctypes.c_int
     L.fbp_residual.argtypes = [P(FbpDims), vp, vp, vp, vp, u32, vp, sz, vp]

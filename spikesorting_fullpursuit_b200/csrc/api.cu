@@ -460,6 +460,21 @@ extern "C" int fbp_pursue_chunk_staged(const fbp_dims* dims, uint32_t flags, flo
                         spike_lab, capacity, n_spikes, stats, max_passes, r, stream);
 }
 
+extern "C" int fbp_copy_rows(void* dst, size_t dst_pitch, const void* src, size_t src_pitch, size_t width,
+                             uint32_t rows, void* stream)
+{
+    g_err.clear();
+    if (rows == 0 || width == 0) return FBP_OK;
+    if (!dst || !src) return fail(FBP_E_ARG, "null pointer argument");
+    if (rows > 1 && (dst_pitch < width || src_pitch < width)) return fail(FBP_E_ARG, "rows overlap");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (rows == 1 || (dst_pitch == width && src_pitch == width))
+        FBP_CUDA(cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyHostToDevice, st));
+    else
+        FBP_CUDA(cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, cudaMemcpyHostToDevice, st));
+    return FBP_OK;
+}
+
 extern "C" int fbp_adjusted_clips(const fbp_dims* dims, const float* residual, const float* templates,
                                   const uint32_t* spike_idx, const uint32_t* spike_lab, uint32_t n,
                                   float* clips, void* stream)

@@ -121,130 +121,121 @@ def _ptr(t):
 
 
 class _Uploader:
-    """Host -> device copy of voltage chunks through pinned staging slabs.
+    """Host -> device copy of voltage chunks.
 
-    Host threads convert and copy pieces of the chunk (one channel row range
-    each) into page-locked slabs while the copy engine moves the previous
-    pieces to the device on a stream of its own; ``upload`` makes the caller's
-    stream wait for the last piece.  The source may be any real dtype and any
-    row-strided view: the float32 conversion happens in the slab copy."""
+    Short float32 chunks go as they are (``direct``).  Others go in blocks of some
+    samples of every channel: host threads convert and copy blocks into page-locked
+    slabs, each as soon as a slab is free, while the copy engine moves the earlier
+    blocks to the device on a stream of its own.  The source may be any real dtype and
+    any row-strided view: the float32 conversion happens in the slab copy.
 
-    SLAB_FLOATS = 2 << 20    # 8 MB per slab
-    N_SLABS = 32
-    N_THREADS = max(1, min(16, os.cpu_count() or 2))
-    RANGE_SAMPLES = 2 << 20  # staged upload: samples of every channel per ready range
+    Blocks of all channels keep both sides busy from the first one on: with a slab
+    per 2M samples of one channel, 16 of them filled before the first was sent,
+    16 channels x 120 s took 12.4 ms to upload, as here 9.0 ms."""
+
+    # 307 MB with 4 / 8 / 16 threads: slabs of 4 MB 11.6 / 9.0 / 11.4 ms, of 8 MB 12.8 / 9.7 /
+    # 10.8 ms, of 2 MB 11.0 / 12.3 / 16.1 ms; 8 to 32 slabs differ by less than 10%
+    SLAB_FLOATS = 1 << 20    # 4 MB per slab ...
+    LEAST_FLOATS = 1 << 19   # ... and less where a chunk has fewer than 16 of those, down to 2 MB
+    N_SLABS = 16
+    N_THREADS = max(1, min(8, os.cpu_count() or 2))
+    # Pageable memory goes at about 20 GB/s, read by the calling thread; slabs are faster
+    # once their threads run: 3.2 MB 0.2 (slabs 0.9), 38 MB 1.8 (3.4), 77 MB 5.4 (4.3) ms
+    DIRECT_BYTES = 48 << 20
 
     def __init__(self, torch, dev):
         self.torch = torch
         self.dev = dev
-        self.slabs = None
-        self.events = [None] * self.N_SLABS
-        self.stream = torch.cuda.Stream(dev)
-        self.pool = ThreadPoolExecutor(self.N_THREADS)
+        self.stream = None
+        self.pool = None
+
+    def direct(self, host, dst):
+        """Upload a short chunk on the caller's stream; False if the chunk is not one."""
+        C, N = host.shape
+        if not (isinstance(host, np.ndarray) and host.dtype == np.float32 and 4 * C * N <= self.DIRECT_BYTES
+                and host.strides[1] == 4 and (C == 1 or host.strides[0] >= 4 * N)):
+            return False
+        stream = ctypes.c_void_p(self.torch.cuda.current_stream(self.dev).cuda_stream)
+        with self.torch.cuda.device(self.dev):
+            _native.check(_native.lib().fbp_copy_rows(_ptr(dst), 4 * dst.stride(0), ctypes.c_void_p(host.ctypes.data),
+                                                      host.strides[0] if C > 1 else 4 * N, 4 * N, C, stream))
+        return True
 
     def upload(self, host, dst):
-        torch = self.torch
-        self._ensure_slabs()
-        C, N = host.shape
-        step = self.SLAB_FLOATS
-        pieces = [(c, a, min(N, a + step)) for c in range(C) for a in range(0, N, step)]
-        caller = torch.cuda.current_stream(self.dev)
-        self.stream.wait_stream(caller)   # dst may still be read by earlier work
-        half = self.N_SLABS // 2
-        for w0 in range(0, len(pieces), half):
-            wave = pieces[w0:w0 + half]
-            slots = [((w0 // half) % 2) * half + k for k in range(len(wave))]
-            for k in slots:
-                if self.events[k] is not None:
-                    self.events[k].synchronize()
-
-            def fill(job):
-                (c, a, b), k = job
-                np.copyto(self.slabs[k].numpy()[:b - a], host[c, a:b], casting="unsafe")
-
-            list(self.pool.map(fill, zip(wave, slots)))
-            with torch.cuda.stream(self.stream):
-                for (c, a, b), k in zip(wave, slots):
-                    dst[c, a:b].copy_(self.slabs[k][:b - a], non_blocking=True)
-                    ev = torch.cuda.Event()
-                    ev.record(self.stream)
-                    self.events[k] = ev
-        caller.wait_stream(self.stream)
-
-    def _ensure_slabs(self):
-        if self.slabs is None:
-            self.slabs = [self.torch.empty(self.SLAB_FLOATS, dtype=self.torch.float32, pin_memory=True)
-                          for _ in range(self.N_SLABS)]
+        """Upload ``host``; the caller's stream waits for it."""
+        if not self.direct(host, dst):
+            self.start_staged(host, dst)[3]()
 
     def start_staged(self, host, dst):
-        """Upload ``host`` on a host thread, time range by time range.
+        """Upload ``host`` on host threads, time range by time range.
 
         Returns (events, upto, flags, finish): events[k] completes once samples
         [0, upto[k]) of every channel are in ``dst``; flags[k] turns 1 once events[k]
         is recorded (the library waits for it before waiting on the event);
         ``finish()`` joins the thread and re-raises its error, if any."""
         torch = self.torch
-        self._ensure_slabs()
         C, N = host.shape
-        span = min(self.RANGE_SAMPLES, self.SLAB_FLOATS)
+        slab = min(self.SLAB_FLOATS, max(self.LEAST_FLOATS, -(-C * N // 16)))
+        span = max(1, slab // C)
         ranges = [(a, min(N, a + span)) for a in range(0, N, span)]
+        n_slabs = min(self.N_SLABS, len(ranges))
+        slabs = [torch.empty(C * span, dtype=torch.float32, pin_memory=True) for _ in range(n_slabs)]
+        if self.pool is None:
+            self.stream = torch.cuda.Stream(self.dev)
+            self.pool = ThreadPoolExecutor(self.N_THREADS)
+        stream, pool = self.stream, self.pool
         events = [torch.cuda.Event() for _ in ranges]
         flags = np.zeros(len(ranges), dtype=np.uint32)
         upto = np.array([b for _, b in ranges], dtype=np.uint32)
-        self.stream.wait_stream(torch.cuda.current_stream(self.dev))   # dst may still be read by earlier work
+        stream.wait_stream(torch.cuda.current_stream(self.dev))   # dst may still be read by earlier work
         for ev in events:   # creates the CUDA events (torch makes them at the first record)
-            ev.record(self.stream)
-        half = self.N_SLABS // 2
+            ev.record(stream)
+        copy_rows, handle = _native.lib().fbp_copy_rows, ctypes.c_void_p(stream.cuda_stream)
         failure = []
+
+        def fill(k):
+            if k >= n_slabs:
+                events[k - n_slabs].synchronize()   # the slab's previous block has left it
+            a, b = ranges[k]
+            np.copyto(slabs[k % n_slabs].numpy()[:C * (b - a)].reshape(C, b - a), host[:, a:b], casting="unsafe")
 
         def run():
             try:
                 with torch.cuda.device(self.dev):
-                    wave_no = 0
+                    filled = [pool.submit(fill, k) for k in range(n_slabs)]
                     for k, (a, b) in enumerate(ranges):
-                        pieces = [(c, a, b) for c in range(C)]
-                        for w0 in range(0, len(pieces), half):
-                            wave = pieces[w0:w0 + half]
-                            slots = [(wave_no % 2) * half + j for j in range(len(wave))]
-                            wave_no += 1
-                            for j in slots:
-                                if self.events[j] is not None:
-                                    self.events[j].synchronize()
-
-                            def fill(job):
-                                (c, x0, x1), j = job
-                                np.copyto(self.slabs[j].numpy()[:x1 - x0], host[c, x0:x1], casting="unsafe")
-
-                            list(self.pool.map(fill, zip(wave, slots)))
-                            with torch.cuda.stream(self.stream):
-                                for (c, x0, x1), j in zip(wave, slots):
-                                    dst[c, x0:x1].copy_(self.slabs[j][:x1 - x0], non_blocking=True)
-                                    ev = torch.cuda.Event()
-                                    ev.record(self.stream)
-                                    self.events[j] = ev
-                        events[k].record(self.stream)
+                        filled[k].result()
+                        width = 4 * (b - a)
+                        _native.check(copy_rows(ctypes.c_void_p(dst.data_ptr() + 4 * a), 4 * dst.stride(0),
+                                                _ptr(slabs[k % n_slabs]), width, width, C, handle))
+                        events[k].record(stream)
                         flags[k] = 1
+                        if k + n_slabs < len(ranges):
+                            filled.append(pool.submit(fill, k + n_slabs))
             except BaseException as e:   # the library must not wait for ranges that never come
                 failure.append(e)
                 with torch.cuda.device(self.dev):
                     for k in range(len(ranges)):
                         if not flags[k]:
-                            events[k].record(self.stream)
+                            events[k].record(stream)
                             flags[k] = 1
+            finally:   # the slabs go back to torch's pinned cache: their last copies must be done
+                stream.synchronize()
 
         th = threading.Thread(target=run, daemon=True)
         th.start()
 
         def finish():
             th.join()
-            torch.cuda.current_stream(self.dev).wait_stream(self.stream)
+            torch.cuda.current_stream(self.dev).wait_stream(stream)
             if failure:
                 raise failure[0]
 
         return events, upto, flags, finish
 
     def close(self):
-        self.pool.shutdown(wait=True)
+        if self.pool is not None:
+            self.pool.shutdown(wait=True)
 
 
 class _Pursuer:
@@ -259,9 +250,15 @@ class _Pursuer:
         self.flags = flags
         self.wg = work_group_size
         self.max_passes = int(max_passes)
-        self.T = torch.from_numpy(np.ascontiguousarray(templates, dtype=np.float32)).to(dev)
-        self.bias = torch.from_numpy(np.ascontiguousarray(bias, dtype=np.float32)).to(dev)
-        self.theta = torch.from_numpy(np.ascontiguousarray(theta, dtype=np.float32)).to(dev)
+        # templates, bias and thresholds in one copy, each part 256-byte aligned
+        parts = [np.ravel(x).astype(np.float32, copy=False) for x in (templates, bias, theta)]
+        at = np.cumsum([0] + [-(-x.size // 64) * 64 for x in parts])
+        flat = np.zeros(at[-1], dtype=np.float32)
+        for x, o in zip(parts, at):
+            flat[o:o + x.size] = x
+        flat = torch.from_numpy(flat).to(dev)
+        self.T, self.bias, self.theta = (flat[o:o + x.size] for x, o in zip(parts, at))
+        self.T = self.T.view(templates.shape)
         d = _native.dims(n_chans, max_chunk, self.M, W, S, work_group_size)
         nbytes = _native.workspace_bytes(d, flags)
         if nbytes == 0:
@@ -278,11 +275,12 @@ class _Pursuer:
         C, N = host_chunk.shape
         d = _native.dims(C, N, self.M, self.W, self.S, self.wg)
         V = self.V[:, :N] if N == self.V.shape[1] else self.V.view(-1)[:C * N].view(C, N)
-        # the first pass runs behind the upload unless the autotuner must see the voltage first
+        # the first pass runs behind the upload unless the chunk is short or the autotuner
+        # must see the voltage first
         ready = None
         if self.tuning == "auto":
             self.up.upload(host_chunk, V)
-        else:
+        elif not self.up.direct(host_chunk, V):
             ready = self.up.start_staged(host_chunk, V)
         nw = (N + self.W - 1) // self.W
         # every pass adds at most one spike per window; dense probes end with about five
@@ -424,7 +422,9 @@ def binary_pursuit(voltage, v_dtype, sort_info, separability_metrics, n_max_shif
     if idx_all:
         event_indices = np.int64(np.hstack(idx_all))
         neuron_labels = np.int64(np.hstack(lab_all))
-        adjusted_clips = np.vstack(clips_all).astype(v_dtype)
+        # one chunk's clips are already an array of the caller's own
+        adjusted_clips = clips_all[0] if len(clips_all) == 1 else np.vstack(clips_all)
+        adjusted_clips = np.atleast_2d(adjusted_clips).astype(v_dtype, copy=False)
         spike_bool = np.hstack(bool_all)
         event_indices += clip_init_samples
         if verbose:

@@ -117,3 +117,31 @@ def test_mean_clip_row_order(n, L):
     rng = np.random.default_rng(n * 1000 + L)
     clips = (rng.standard_normal((n, L)) * rng.uniform(0.1, 1e4, (n, 1))).astype(np.float32)
     assert np.array_equal(postprocessing.mean_clip(clips).cpu().numpy(), np.mean(clips, axis=0))
+
+
+@pytest.mark.parametrize("kind", ["float32", "rows_apart", "read_only", "every_other", "int16", "float64", "reversed"])
+@pytest.mark.parametrize("shape,limit", [((4, 5000), None), ((3, 1_000_003), 0), ((700, 4001), 0), ((1, 9_000_000), 0)])
+def test_uploads(kind, shape, limit, monkeypatch):
+    """Voltage chunks as they are and through slabs of one and of many samples a channel,
+    more blocks than slabs, any dtype and row stride."""
+    from spikesorting_fullpursuit_b200.overlap import binary_pursuit_parallel as bpp
+    if limit is not None:
+        monkeypatch.setattr(bpp._Uploader, "DIRECT_BYTES", limit)
+    rng = np.random.default_rng(shape[1])
+    C, N = shape
+    wide = rng.integers(-3000, 3000, size=(C, 2 * N)).astype(
+        {"int16": np.int16, "float64": np.float64}.get(kind, np.float32))
+    host = {"every_other": wide[:, ::2], "reversed": wide[:, N - 1::-1]}.get(kind, wide[:, :N])
+    if kind == "float32":
+        host = np.ascontiguousarray(host)
+    host.flags.writeable = kind != "read_only"
+    dev = torch.device("cuda", torch.cuda.current_device())
+    dst = torch.zeros((C, N), dtype=torch.float32, device=dev)
+    up = bpp._Uploader(torch, dev)
+    try:
+        for _ in range(2):
+            up.upload(host, dst)
+            assert np.array_equal(dst.cpu().numpy(), host.astype(np.float32))
+            dst.zero_()
+    finally:
+        up.close()
