@@ -542,60 +542,73 @@ __global__ void __launch_bounds__(kOvThreads) overlap_plain_kernel(
 // since it was computed, so the current voltage gives the exact value).  Called
 // by a whole warp with the same (t, s) on every lane.
 __device__ __forceinline__ float warp_lik_value(const Dims& d, const float* __restrict__ L, const LazyRef& z,
-                                                uint32_t t, uint32_t s)
+                                                uint32_t t, uint32_t s, float* buf)
 {
     const float v = L[(uint64_t)t * d.N + s];
     if (z.wflag != nullptr && v > 0.f && z.wflag[(uint64_t)(s / d.W) * d.M + t])
-        return warp_exact_lik(d, z.V, z.T, z.bias[t], t, s, z.tnorm);
+        return warp_exact_lik(d, z.V, z.T, z.bias[t], t, s, z.tnorm, buf);
     return v;
 }
 
-// One warp per flagged window (every lane evaluates the same decisions; lane 0
-// writes them).
-__global__ void parse_kernel(Dims d, const float* __restrict__ L, const float* __restrict__ theta,
-                             const uint32_t* __restrict__ flag, const DevStatus* status,
-                             const unsigned long long* __restrict__ keys, float* best_lik,
-                             const uint32_t* __restrict__ best_lab, const uint32_t* __restrict__ best_idx,
-                             uint8_t* orech, uint32_t* ov_idx, uint32_t* ov_lab, LazyRef z)
+// Two warps per flagged window, one for each template's likelihood; the first one's
+// lane 0 decides.
+constexpr uint32_t kParseThreads = 256;
+
+__global__ void __launch_bounds__(kParseThreads) parse_kernel(
+    Dims d, const float* __restrict__ L, const float* __restrict__ theta, const uint32_t* __restrict__ flag,
+    const DevStatus* status, const unsigned long long* __restrict__ keys, float* best_lik,
+    const uint32_t* __restrict__ best_lab, const uint32_t* __restrict__ best_idx, uint8_t* orech, uint32_t* ov_idx,
+    uint32_t* ov_lab, LazyRef z)
 {
+    __shared__ float buf[kParseThreads / 32][32 * kExactBlocks];
+    __shared__ float value[kParseThreads / 32];
     const uint32_t nflag = status->n_flag;
     const uint64_t S2 = 2ull * d.S + 1;
     const uint64_t items = S2 * S2 * d.M;
-    const bool lead = (threadIdx.x & 31) == 0;
     uint32_t lbits = 0;
     while ((1u << lbits) < d.WG) ++lbits;
-    const uint32_t wpb = blockDim.x >> 5;
-    for (uint32_t k = blockIdx.x * wpb + (threadIdx.x >> 5); k < nflag; k += gridDim.x * wpb) {
-        const uint32_t id = flag[k];
-        const float seed = best_lik[id];
-        const unsigned long long key = keys[k];
-        const bool have = key != 0ull;
-        const float gv = have ? __uint_as_float((uint32_t)(key >> 32)) : 0.f;
-        if (!have || gv <= seed || gv <= 0.f) {
-            if (lead) orech[id] = 0;
-            continue;
+    const uint32_t warp = threadIdx.x >> 5, per = kParseThreads / 64;
+    for (uint32_t k0 = blockIdx.x * per; k0 < nflag; k0 += gridDim.x * per) {
+        const uint32_t k = k0 + (warp >> 1);
+        const bool lead = (threadIdx.x & 63u) == 0;
+        bool pair = false;   // a winner better than the seed: its two likelihoods count
+        uint32_t id = 0, f = 0, t = 0, afi = 0, asi = 0;
+        float gv = 0.f;
+        if (k < nflag) {
+            id = flag[k];
+            const float seed = best_lik[id];
+            const unsigned long long key = keys[k];
+            gv = key != 0ull ? __uint_as_float((uint32_t)(key >> 32)) : 0.f;
+            const uint32_t prio = 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull);
+            const uint32_t g = prio / d.WG, lb = prio % d.WG;
+            const uint32_t l = lbits ? (__brev(lb) >> (32 - lbits)) : 0u;
+            const uint64_t r = (uint64_t)g * d.WG + l;
+            pair = !(key == 0ull || gv <= seed || gv <= 0.f) && r < items;
+            if (pair) {
+                f = best_lab[id];
+                const uint32_t p = best_idx[id];
+                t = (uint32_t)(r % d.M);
+                const uint64_t a = (r / d.M) % S2, b = (r / (S2 * d.M)) % S2;
+                afi = (uint32_t)(p + a - d.S);
+                asi = (uint32_t)(p + b - d.S);
+                const bool second = warp & 1u;
+                const float v = warp_lik_value(d, L, z, second ? t : f, second ? asi : afi, buf[warp]);
+                if ((threadIdx.x & 31) == 0) value[warp] = v;
+            } else if (lead) {
+                orech[id] = 0;
+            }
         }
-        const uint32_t prio = 0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull);
-        const uint32_t g = prio / d.WG, lb = prio % d.WG;
-        const uint32_t l = lbits ? (__brev(lb) >> (32 - lbits)) : 0u;
-        const uint64_t r = (uint64_t)g * d.WG + l;
-        if (r >= items) {
-            if (lead) orech[id] = 0;
-            continue;
+        __syncthreads();
+        if (pair && lead) {
+            const float l1 = value[warp], l2 = value[warp + 1];
+            if (gv < l1 || gv < l2) orech[id] = 0;
+            else if (l1 <= 0.f || l2 <= 0.f) orech[id] = 0;
+            else if (l1 >= l2 && l1 > theta[f]) { best_lik[id] = l1; ov_lab[id] = f; ov_idx[id] = afi; }
+            else if (l2 > l1 && l2 > theta[t]) { best_lik[id] = l2; ov_lab[id] = t; ov_idx[id] = asi; }
+            else if (l1 > theta[f]) { best_lik[id] = l1; ov_lab[id] = f; ov_idx[id] = afi; }
+            else { ov_idx[id] = best_idx[id]; ov_lab[id] = best_lab[id]; orech[id] = 0; }
         }
-        const uint32_t f = best_lab[id], p = best_idx[id];
-        const uint32_t t = (uint32_t)(r % d.M);
-        const uint64_t a = (r / d.M) % S2, b = (r / (S2 * d.M)) % S2;
-        const uint32_t afi = (uint32_t)(p + a - d.S), asi = (uint32_t)(p + b - d.S);
-        const float l1 = warp_lik_value(d, L, z, f, afi);
-        const float l2 = warp_lik_value(d, L, z, t, asi);
-        if (!lead) continue;
-        if (gv < l1 || gv < l2) { orech[id] = 0; continue; }
-        if (l1 <= 0.f || l2 <= 0.f) { orech[id] = 0; continue; }
-        if (l1 >= l2 && l1 > theta[f]) { best_lik[id] = l1; ov_lab[id] = f; ov_idx[id] = afi; }
-        else if (l2 > l1 && l2 > theta[t]) { best_lik[id] = l2; ov_lab[id] = t; ov_idx[id] = asi; }
-        else if (l1 > theta[f]) { best_lik[id] = l1; ov_lab[id] = f; ov_idx[id] = afi; }
-        else { ov_idx[id] = best_idx[id]; ov_lab[id] = best_lab[id]; orech[id] = 0; }
+        __syncthreads();   // the values are read, and this window's best_lik by both warps before
     }
 }
 
@@ -1053,14 +1066,14 @@ int launch_parse_reassign(const Dims& d, const Work& w, const float* theta, uint
 {
     if (nflag_max == 0) return FBP_OK;
     const uint32_t g = grid_for(nflag_max, 256);
-    const uint32_t gw = grid_for(nflag_max, 8);   // parse: one warp per window
+    const uint32_t gw = grid_for(nflag_max, kParseThreads / 64);   // parse: two warps per window
     LazyRef z{nullptr, nullptr, V, T, bias};
     if (lazy) {
         z.wflag = w.at<uint8_t>(w.lay->off_wflag);
         z.tnorm = w.at<float>(w.lay->off_tnorm);
     }
     count_launch(3);
-    parse_kernel<<<gw, 256, 0, st>>>(d, w.L(), theta, w.flag(), w.status(), w.keys(), w.best_lik(),
+    parse_kernel<<<gw, kParseThreads, 0, st>>>(d, w.L(), theta, w.flag(), w.status(), w.keys(), w.best_lik(),
                                     w.best_lab(), w.best_idx(), w.orech(), w.ov_idx(), w.ov_lab(), z);
     reassign_kernel<<<g, 256, 0, st>>>(d, w.flag(), w.status(), w.orech(), w.orech_fin(), w.best_idx(), w.best_lab(),
                                        w.check(), w.ov_idx(), w.ov_lab());

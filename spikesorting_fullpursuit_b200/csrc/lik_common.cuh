@@ -32,61 +32,71 @@ static __device__ float exact_likelihood(const Dims& d, const float* __restrict_
 }
 
 // Exact likelihood of (t, s) in the reference order (compute_maximum_likelihood,
-// binary_pursuit.cl:216-252) from the current voltage, by a whole warp: each
-// lane forms the products of 32 taps at a time (each product rounds the same
-// wherever it is formed), the operands of the next 32 on their way meanwhile,
-// and every lane adds them in tap order, so all lanes end with the reference's
-// sum.  Channels where the template is entirely zero add 0 * v terms in the
-// reference, which leave a nonzero sum unchanged.
+// binary_pursuit.cl:216-252) from the current voltage, by a whole warp: the lanes form
+// the products of four blocks of 32 taps (each product rounds the same wherever it is
+// formed) in shared memory, the operands of the next four on their way meanwhile, and
+// every lane adds them in tap order.  Channels where the template is entirely zero add
+// 0 * v terms in the reference, which leave a nonzero sum unchanged.
+//
+// With one block of 32 on its way, a value of 8 channels took the latency of 25 to 32
+// loads one after the other; the overlap recheck's parse, two such values a window,
+// took 24 us a pass (8 channels, 17 templates, 8 s) and takes 11.
+constexpr int kExactBlocks = 4;
+
 static __device__ float warp_exact_lik(const Dims& d, const float* __restrict__ V, const float* __restrict__ T, float b,
-                                       uint32_t t, uint32_t s, const float* __restrict__ tnorm)
+                                       uint32_t t, uint32_t s, const float* __restrict__ tnorm, float* buf)
 {
     const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31, C = d.C, W = d.W;
-    float acc = b;
     const float* tn = tnorm + (uint64_t)t * C;
-    for (uint32_t cb = 0; cb < C; cb += 32) {
-        uint32_t live = __ballot_sync(full, cb + lane < C && tn[cb + lane] != 0.f);
-        const float* tr = nullptr;
-        const float* vr = nullptr;
-        auto channel = [&]() {   // the next live channel's rows
-            const uint32_t c = cb + __ffs(live) - 1;
-            live &= live - 1;
-            tr = T + ((uint64_t)t * C + c) * W;
-            vr = V + (uint64_t)c * d.N + s;
-        };
-        bool more = live != 0u;
-        uint32_t j0 = 0;
-        float tv = 0.f, vv = 0.f;
-        if (more) {
-            channel();
-            if (lane < W) {
-                tv = __ldg(tr + lane);
-                vv = vr[lane];
-            }
-        }
-        while (more) {
-            const float p = __fmul_rn(tv, vv);
-            const uint32_t n = W - j0 < 32u ? W - j0 : 32u;
-            j0 += 32;
-            if (j0 >= W) {
-                more = live != 0u;
-                j0 = 0;
-                if (more) channel();
-            }
-            tv = 0.f;
-            vv = 0.f;
-            if (more && j0 + lane < W) {
-                tv = __ldg(tr + j0 + lane);
-                vv = vr[j0 + lane];
-            }
-            if (n == 32u) {
+    const float *tr = nullptr, *vr = nullptr;   // the channel's rows, at this lane
+    uint32_t cb = 0, j0 = W;                    // first channel of `live`, first tap of the block
+    uint32_t live = __ballot_sync(full, lane < C && tn[lane] != 0.f);
+    float tv[kExactBlocks], vv[kExactBlocks];
+    uint32_t n[kExactBlocks];
+    bool more = true;
+    auto fetch = [&]() {
 #pragma unroll
-                for (uint32_t k = 0; k < 32; ++k) acc = __fadd_rn(acc, __shfl_sync(full, p, k));
-            } else {
-#pragma unroll 8
-                for (uint32_t k = 0; k < n; ++k) acc = __fadd_rn(acc, __shfl_sync(full, p, k));
+        for (int q = 0; q < kExactBlocks; ++q) {
+            n[q] = 0;
+            if (!more) continue;
+            j0 += 32;
+            if (j0 >= W) {   // the next non-zero channel
+                while (live == 0u && (cb += 32) < C) live = __ballot_sync(full, cb + lane < C && tn[cb + lane] != 0.f);
+                if (live == 0u) {
+                    more = false;
+                    continue;
+                }
+                const uint32_t c = cb + __ffs(live) - 1;
+                live &= live - 1;
+                tr = T + ((uint64_t)t * C + c) * W + lane;
+                vr = V + (uint64_t)c * d.N + s + lane;
+                j0 = 0;
+            }
+            n[q] = min(W - j0, 32u);
+            if (lane < n[q]) {
+                tv[q] = __ldg(tr + j0);
+                vv[q] = vr[j0];
             }
         }
+    };
+    float acc = b;
+    fetch();
+    while (n[0] != 0u) {
+        uint32_t total = 0;
+#pragma unroll
+        for (int q = 0; q < kExactBlocks; ++q) {
+            if (lane < n[q]) buf[total + lane] = __fmul_rn(tv[q], vv[q]);
+            total += n[q];
+        }
+        __syncwarp();
+        fetch();
+        uint32_t i = 0;
+        for (; i + 16 <= total; i += 16) {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) acc = __fadd_rn(acc, buf[i + k]);
+        }
+        for (; i < total; ++i) acc = __fadd_rn(acc, buf[i]);
+        __syncwarp();
     }
     return acc;
 }

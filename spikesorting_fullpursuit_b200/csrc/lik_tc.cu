@@ -1090,34 +1090,112 @@ __global__ void __launch_bounds__(persist_threads(NE), 1) lik_tc_persist_kernel(
     }
 }
 
-// Exact recomputation of the queued runs (reference order, FP32), a warp per run.
-// An entry is (t << 40) | (mask << 32) | s0: samples s0 + k with bit k of the 4-bit
-// mask set.  The lanes form the products of 32 taps at a time (a product rounds the
-// same wherever it is formed; the next 32 taps' operands are already on their way),
-// and every lane adds them one by one in the reference's order, channel-major, taps
-// ascending, over the template's non-zero channels (the others add exact zeros).
-// The chain of additions (about 6 cycles each with its broadcast) bounds a run; one
-// thread per run, with its operands fetched four taps at a time, took 5 to 30 times
-// as long (12.2 ms per pursuit of 20 s of 64 channels x 200 templates).
-__global__ void __launch_bounds__(256) fixup_kernel(Dims d, const float* __restrict__ V, const float* __restrict__ T,
-                                                    const float* __restrict__ bias,
-                                                    const unsigned long long* __restrict__ fix, uint32_t cap,
-                                                    const DevStatus* status, float* L, unsigned long long* wkey,
-                                                    uint8_t* wpos, const float* __restrict__ tnorm)
+// Exact recomputation of the queued runs (reference order, FP32).  An entry is
+// (t << 40) | (mask << 32) | s0: samples s0 + k with bit k of the 4-bit mask set.
+// A warp takes four runs, or two or one where that fills the SMs better.  Block by
+// block of 32 taps of the template's non-zero channels (the others add exact zeros),
+// four blocks at a time -- one of each run, or as many more of the same -- the lanes
+// form the products of a block in shared memory, the operands of the next four on their
+// way meanwhile; then lane 4 e + k adds run e's sample k, product by product in the
+// reference's order, channel-major, taps ascending.  A
+// warp per sample, its sums by broadcasts from the lanes' registers, took two
+// instructions a tap and sample and waited for every block's loads: 300 s of 16
+// channels x 40 templates, 19 thousand runs a pass, 1.28 ms a pursuit, as here 0.97;
+// 3 to 12 s of 4 to 12 channels 20 us a pass, as here 16.
+constexpr int kFixThreads = 256;
+constexpr int kFixSlots = 4;
+constexpr int kFixPitch = 33 * 4;   // [32 taps][4 samples], padded: the lanes of a sum read 16 different banks
+
+__global__ void __launch_bounds__(kFixThreads, 4) fixup_kernel(
+    Dims d, const float* __restrict__ V, const float* __restrict__ T, const float* __restrict__ bias,
+    const unsigned long long* __restrict__ fix, uint32_t cap, const DevStatus* status, float* L,
+    unsigned long long* wkey, uint8_t* wpos, const uint8_t* __restrict__ clist, const uint32_t* __restrict__ ccnt)
 {
-    const uint32_t n = min(status->n_fix, cap), lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (uint32_t i = blockIdx.x * wpb + (threadIdx.x >> 5); i < n; i += gridDim.x * wpb) {
-        const unsigned long long e = fix[i];
-        const uint32_t t = (uint32_t)(e >> 40), s0 = (uint32_t)e;
-        uint32_t mask = (uint32_t)(e >> 32) & 0xFu;
-        while (mask) {
-            const uint32_t s = s0 + __ffs(mask) - 1;
-            mask &= mask - 1;
-            const float v = warp_exact_lik(d, V, T, bias[t], t, s, tnorm);
-            if (lane == 0) {
-                L[(uint64_t)t * d.N + s] = v;
-                note_window(d, wkey, wpos, v, t, s);
+    __shared__ __align__(16) float prod[kFixThreads / 32][kFixSlots * kFixPitch];
+    __shared__ uint4 desc[kFixThreads / 32][2][kFixSlots];   // template offset (low), taps | mask << 8 | offset (high) << 12, voltage offset
+    const uint32_t n = min(status->n_fix, cap), C = d.C, W = d.W;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, e = lane >> 2, k = lane & 3u;
+    const uint32_t nwarps = gridDim.x * (kFixThreads / 32);
+    uint32_t G = kFixSlots;
+    while (G > 1 && (n + G - 1) / G < nwarps) G >>= 1;
+    const uint32_t B = kFixSlots / G;   // blocks of a run at a time
+    for (uint32_t i0 = (blockIdx.x * (kFixThreads / 32) + warp) * G; i0 < n; i0 += nwarps * G) {
+        const bool ok = e < G && i0 + e < n;
+        const unsigned long long code = ok ? fix[i0 + e] : 0ull;
+        const uint32_t t = (uint32_t)(code >> 40), s0 = (uint32_t)code, mask = (uint32_t)(code >> 32) & 0xFu;
+        float acc = ok ? bias[t] : 0.f;
+        // lane 4 e + k describes slot k's block where run e owns the slot; all blocks
+        // are of 32 taps but a channel's last
+        const uint32_t nb = (W + 31) / 32, slot = lane & 3u;
+        const uint32_t own = slot % G;                        // the run of this lane's slot
+        const uint32_t st = __shfl_sync(0xffffffffu, t, own * 4), ss = __shfl_sync(0xffffffffu, s0, own * 4);
+        const uint32_t sm = __shfl_sync(0xffffffffu, mask, own * 4);
+        const uint32_t chans = i0 + own < n ? (C <= 256 ? ccnt[st] : C) : 0u;   // the channel list is of bytes
+        uint32_t at = slot / G, taps = 0;                     // the slot's block; its taps
+        auto advance = [&](uint32_t par) -> bool {            // the next blocks; false if no run has any
+            const uint32_t ord = at / nb, j0 = (at - ord * nb) * 32;
+            taps = ord < chans ? min(W - j0, 32u) : 0u;
+            at += B;
+            if (lane < kFixSlots) {
+                const uint32_t c = taps ? (C <= 256 ? clist[(uint64_t)st * C + ord] : ord) : 0u;
+                const uint64_t to = ((uint64_t)st * C + c) * W + j0, vo = (uint64_t)c * d.N + ss + j0;
+                desc[warp][par][lane] = make_uint4((uint32_t)to, taps | (sm << 8) | (uint32_t)(to >> 32) << 12,
+                                                   (uint32_t)vo, (uint32_t)(vo >> 32));
             }
+            __syncwarp();
+            return __any_sync(0xffffffffu, taps != 0u);
+        };
+        float tv[kFixSlots], vv[kFixSlots][4];
+        auto fetch = [&](uint32_t par) {
+#pragma unroll
+            for (int q = 0; q < kFixSlots; ++q) {
+                const uint4 r = desc[warp][par][q];
+                tv[q] = 0.f;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) vv[q][x] = 0.f;
+                if (lane < (r.y & 0xFFu)) {
+                    const float* v = V + (((uint64_t)r.w << 32) | r.z) + lane;
+                    tv[q] = __ldg(T + (((uint64_t)(r.y >> 12) << 32) | r.x) + lane);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+                        if ((r.y >> (8 + x)) & 1u) vv[q][x] = v[x];
+                }
+            }
+        };
+        uint32_t par = 0;
+        bool more = advance(par);
+        fetch(par);
+        while (more) {
+            const uint32_t cur = taps;   // of slot lane % 4
+#pragma unroll
+            for (int q = 0; q < kFixSlots; ++q)   // lanes past a block's taps add nothing (0 * 0)
+                *reinterpret_cast<float4*>(&prod[warp][q * kFixPitch + lane * 4]) =
+                    make_float4(__fmul_rn(tv[q], vv[q][0]), __fmul_rn(tv[q], vv[q][1]), __fmul_rn(tv[q], vv[q][2]),
+                                __fmul_rn(tv[q], vv[q][3]));
+            __syncwarp();
+            par ^= 1u;
+            more = advance(par);
+            fetch(par);
+            for (uint32_t b = 0; b < B; ++b) {
+                const uint32_t q = b * G + e;   // a slot where e < G
+                const uint32_t m = __shfl_sync(0xffffffffu, cur, q & 3u);
+                const float* x = prod[warp] + (q & 3u) * kFixPitch + k;
+                if (__all_sync(0xffffffffu, m == 32u)) {   // reading a slot for a lane without a run does no harm
+#pragma unroll
+                    for (int y = 0; y < 32; ++y) acc = __fadd_rn(acc, x[y * 4]);
+                } else {
+                    for (uint32_t j = 0; j < m; j += 8) {
+#pragma unroll
+                        for (int y = 0; y < 8; ++y) acc = __fadd_rn(acc, x[(j + y) * 4]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (ok && ((mask >> k) & 1u)) {
+            const uint32_t s = s0 + k;
+            L[(uint64_t)t * d.N + s] = acc;
+            note_window(d, wkey, wpos, acc, t, s);
         }
     }
 }
@@ -1396,10 +1474,11 @@ int launch_fixup(const Dims& d, const Work& w, const float* V, const float* T, c
     const Layout& L = *w.lay;
     count_launch();
     KScope ks(&fbp_chunk_stats::ms_fixup, st);
-    fixup_kernel<<<148 * 8, 256, 0, st>>>(d, V, T, bias, w.at<unsigned long long>(L.off_fix),
-                                          (uint32_t)L.n_fix_cap, w.status(), Lk,
-                                          lazy ? w.at<unsigned long long>(L.off_wkey) : nullptr,
-                                          lazy ? w.at<uint8_t>(L.off_wpos) : nullptr, w.at<float>(L.off_tnorm));
+    fixup_kernel<<<148 * 4, kFixThreads, 0, st>>>(d, V, T, bias, w.at<unsigned long long>(L.off_fix),
+                                                  (uint32_t)L.n_fix_cap, w.status(), Lk,
+                                                  lazy ? w.at<unsigned long long>(L.off_wkey) : nullptr,
+                                                  lazy ? w.at<uint8_t>(L.off_wpos) : nullptr,
+                                                  w.at<uint8_t>(L.off_clist), w.at<uint32_t>(L.off_ccnt));
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }

@@ -444,11 +444,20 @@ __device__ __forceinline__ uint32_t item_priority(uint64_t r, uint32_t WG, uint3
     return g * WG + br;
 }
 
-constexpr int kScrThreads = 128;
 constexpr uint32_t kChunkCap = 512;    // chunks of 32 items kept in shared memory
 constexpr uint32_t kRowCap = 768;      // rows (t, b) kept in shared memory
 constexpr uint32_t kQueue = 64;        // chunks a warp keeps for evaluation
-constexpr int kScrPerSm = 8;
+// Threads a window, and CTAs per SM.  A window alone takes its loads one after the
+// other: with no more listed windows than kScrFewWindows, of which a part is flagged,
+// the SMs are not full and 512 threads a window are faster (3 to 12 s of 4 to 12
+// channels, up to 300 flagged windows a pass: 70 -> 44 us; 20 s of 64 channels 14.3 ->
+// 12.5 ms a pursuit); many windows fill the SMs with 128 threads each, and a CTA of 512
+// waits for its slowest warp at every barrier (512 for all, 300 s of 16 channels: 14.1
+// -> 21.5 ms; the line at 2400, 5000 and 10000 windows: within 1% there, 12.6, 12.5 and
+// 13.2 ms with 64 channels).
+constexpr int kScrThreads = 128, kScrPerSm = 8;
+constexpr int kScrWideThreads = 512, kScrWidePerSm = 2;
+constexpr uint32_t kScrFewWindows = 5000;
 
 struct ScreenArgs {
     Dims d;
@@ -487,11 +496,11 @@ struct ScreenShared {
 __host__ __device__ inline uint32_t scr_chunks(uint32_t S2) { return (S2 + 31) / 32; }
 
 // Shared-memory bytes of screen_kernel.
-__host__ __device__ inline size_t screen_smem_bytes(uint32_t M, uint32_t S2, uint32_t C)
+__host__ __device__ inline size_t screen_smem_bytes(uint32_t M, uint32_t S2, uint32_t C, int threads)
 {
     const size_t nch = scr_chunks(S2);
     return (nch * 32 * 2 + (size_t)M * nch * 2 + (size_t)M * 4 + nch + C * 2 + kChunkCap * 3 + kRowCap * 2 +
-            kQueue * 2 * (kScrThreads / 32)) * 4 + 16;
+            kQueue * 2 * (size_t)(threads / 32)) * 4 + 16;
 }
 
 // Bound of |estimate - reference float value| of every item (a, t, b) of a window
@@ -556,13 +565,14 @@ __device__ __forceinline__ float pair_margin(const Dims& d, MarginPart f, Margin
 // 31.9 -> 14.5 ms, 20 s of 64 channels 37.4 -> 14.3 ms (and 8.5 M -> 0.16 M items
 // scored exactly there, by the margin's count of non-zero channels).  Bounded by
 // instruction issue and latency together: 49 % of the issue slots, 28 warps per SM.
-__global__ void __launch_bounds__(kScrThreads, kScrPerSm) screen_kernel(const __grid_constant__ ScreenArgs P)
+template <int THREADS, int PER_SM>
+__global__ void __launch_bounds__(THREADS, PER_SM) screen_kernel(const __grid_constant__ ScreenArgs P)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ ScreenShared sh;
     const Dims& d = P.d;
     const uint32_t S = d.S, W = d.W, M = d.M, C = d.C, S2 = 2 * S + 1, nch = scr_chunks(S2);
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = kScrThreads / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = THREADS / 32;
     const uint32_t full = 0xffffffffu, below = (1u << lane) - 1u;
     float* Gf = reinterpret_cast<float*>(smraw);                       // [nch * 32] G_f, -inf out of bounds
     uint32_t* alist = reinterpret_cast<uint32_t*>(Gf + nch * 32);      // [nch * 32] A+ in ascending order
@@ -1006,11 +1016,17 @@ __global__ void __launch_bounds__(kScoreThreads) score_kernel(
         }
         uint32_t next = 0;                // channel (C > 64: all of them)
         if (lane < kScoreMany) shift[warp][e] = make_int2((int)d.S - (int)a, (int)d.S - (int)b);
-        float acc = 0.f;                  // lanes < 16
-        for (;;) {
-            const bool on = ok && (C > 64 ? next < C : left != 0ull);
-            const uint32_t act = __ballot_sync(full, on) & 0xFFFFu;
-            if (act == 0u) break;
+        // blocks of 32 taps of a channel, eight candidates at a time
+        bool on = false;                  // this candidate takes part in the channel
+        uint32_t act = 0, j0 = W, g0 = 0;
+        auto advance = [&]() {            // to the next eight, block or channel; act == 0: done
+            g0 += 8;
+            if (g0 < G && ((act >> g0) & 0xFFu)) return;
+            g0 = 0;
+            j0 += 32;
+            if (j0 < W) return;
+            on = ok && (C > 64 ? next < C : left != 0ull);
+            act = __ballot_sync(full, on) & 0xFFFFu;
             const uint32_t c = C > 64 ? next : (uint32_t)__ffsll((long long)left) - 1u;
             if (on) {
                 left &= left - 1;
@@ -1021,48 +1037,58 @@ __global__ void __launch_bounds__(kScoreThreads) score_kernel(
                 }
             }
             __syncwarp();
-            float sum = lane < kScoreMany ? acc : 0.f;
-            for (uint32_t j0 = 0; j0 < W; j0 += 32) {
-                const uint32_t j = j0 + lane;
-                for (uint32_t g0 = 0; g0 < G; g0 += 8) {
-                    if (((act >> g0) & 0xFFu) == 0u) continue;
-                    float fv[8], tv[8], vv[8];
+            j0 = 0;
+        };
+        float fv[8], tv[8], vv[8];
+        auto fetch = [&]() {
+            const uint32_t j = j0 + lane;
 #pragma unroll
-                    for (uint32_t q = 0; q < 8; ++q) {
-                        fv[q] = tv[q] = vv[q] = 0.f;
-                        if (!((act >> (g0 + q)) & 1u)) continue;   // the same for the whole warp
-                        const uint4 r = rows[warp][g0 + q];
-                        const int2 s = shift[warp][g0 + q];
-                        const int jf = (int)j + s.x, jt = (int)j + s.y;
-                        if (j < W) {
-                            vv[q] = __ldg(V + (((uint64_t)r.w << 32) | r.z) + j);
-                            if (jf >= 0 && jf < (int)W) fv[q] = __ldg(T + r.x + jf);
-                            if (jt >= 0 && jt < (int)W) tv[q] = __ldg(T + r.y + jt);
-                        }
-                    }
-#pragma unroll
-                    for (uint32_t q = 0; q < 8; ++q) {
-                        if (!((act >> (g0 + q)) & 1u)) continue;
-                        const float sv = fadd(fv[q], tv[q]);
-                        prod[warp][(g0 + q) * 33 + lane] = fmul(sv, vv[q]);
-                        prod[warp][(kScoreMany + g0 + q) * 33 + lane] = fmul(sv, sv);
-                    }
+            for (uint32_t q = 0; q < 8; ++q) {
+                fv[q] = tv[q] = vv[q] = 0.f;
+                if (!((act >> (g0 + q)) & 1u)) continue;   // the same for the whole warp
+                const uint4 r = rows[warp][g0 + q];
+                const int2 s = shift[warp][g0 + q];
+                const int jf = (int)j + s.x, jt = (int)j + s.y;
+                if (j < W) {
+                    vv[q] = __ldg(V + (((uint64_t)r.w << 32) | r.z) + j);
+                    if (jf >= 0 && jf < (int)W) fv[q] = __ldg(T + r.x + jf);
+                    if (jt >= 0 && jt < (int)W) tv[q] = __ldg(T + r.y + jt);
                 }
-                __syncwarp();
-                if (on) {
-                    const uint32_t m = min(32u, W - j0);
-                    if (m == 32u) {
-#pragma unroll
-                        for (uint32_t k = 0; k < 32; ++k) sum = fadd(sum, mine[k]);
-                    } else {
-#pragma unroll 4
-                        for (uint32_t k = 0; k < m; ++k) sum = fadd(sum, mine[k]);
-                    }
-                }
-                __syncwarp();
             }
-            const float ss = __shfl_sync(full, sum, lane | 16u);
-            if (on && lane < kScoreMany) acc = ss > 0.f ? fsub(sum, fmul(0.5f, ss)) : sum;
+        };
+        float acc = 0.f, sum = 0.f;       // acc: lanes < 16
+        advance();
+        fetch();
+        while (act) {
+            const uint32_t cact = act, cj0 = j0, cg0 = g0;
+            const bool con = on, last = cg0 + 8 >= G || ((cact >> (cg0 + 8)) & 0xFFu) == 0u;
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q) {
+                if (!((cact >> (cg0 + q)) & 1u)) continue;
+                const float sv = fadd(fv[q], tv[q]);
+                prod[warp][(cg0 + q) * 33 + lane] = fmul(sv, vv[q]);
+                prod[warp][(kScoreMany + cg0 + q) * 33 + lane] = fmul(sv, sv);
+            }
+            __syncwarp();
+            advance();
+            fetch();   // on its way during the sums
+            if (!last) continue;
+            if (cj0 == 0) sum = lane < kScoreMany ? acc : 0.f;
+            if (con) {
+                const uint32_t m = min(32u, W - cj0);
+                if (m == 32u) {
+#pragma unroll
+                    for (uint32_t k = 0; k < 32; ++k) sum = fadd(sum, mine[k]);
+                } else {
+#pragma unroll 4
+                    for (uint32_t k = 0; k < m; ++k) sum = fadd(sum, mine[k]);
+                }
+            }
+            if (cj0 + 32 >= W) {
+                const float ss = __shfl_sync(full, sum, lane | 16u);
+                if (con && lane < kScoreMany) acc = ss > 0.f ? fsub(sum, fmul(0.5f, ss)) : sum;
+            }
+            __syncwarp();
         }
         if (ok && lane < kScoreMany && acc > 0.f) {
             const uint64_t r = (uint64_t)t + (uint64_t)M * a + (uint64_t)M * S2 * b;
@@ -1187,11 +1213,15 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
     const bool fft = window_corr_by_fft(d);
     if (Q == 0 && !fft) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
     const uint32_t pc_threads = 32u * std::min<uint32_t>((S2 + 15) / 16, kPcMaxWarps);
-    const size_t smem_b = screen_smem_bytes(d.M, S2, d.C);
-    if (smem_b > 200 * 1024) return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
-    FBP_CUDA(allow_max_dyn_smem(screen_kernel));
+    if (screen_smem_bytes(d.M, S2, d.C, kScrThreads) > 200 * 1024)
+        return launch_overlap_plain(d, w, V, T, theta, nflag_max, st);
+    const bool wide = nflag_max <= kScrFewWindows && screen_smem_bytes(d.M, S2, d.C, kScrWideThreads) <= 100 * 1024;
+    const int scr_threads = wide ? kScrWideThreads : kScrThreads;
+    const size_t smem_b = screen_smem_bytes(d.M, S2, d.C, scr_threads);
+    const auto screen = wide ? screen_kernel<kScrWideThreads, kScrWidePerSm> : screen_kernel<kScrThreads, kScrPerSm>;
+    FBP_CUDA(allow_max_dyn_smem(screen));
     int scr_per_sm = 1;
-    FBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scr_per_sm, screen_kernel, kScrThreads, smem_b));
+    FBP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scr_per_sm, screen, scr_threads, smem_b));
     const uint32_t groups = Q > 0 ? (d.M + Q - 1) / Q : 0u;
     float* G = w.at<float>(L.off_g);
     const float2* Et = w.at<float2>(L.off_et);
@@ -1260,7 +1290,7 @@ int launch_overlap_fast(const Dims& d, const Work& w, const float* V, const floa
         P.k0 = k0;
         P.kc = kc;
         const uint32_t grid = std::min<uint32_t>(kc, 148u * (scr_per_sm > 0 ? scr_per_sm : 1));
-        screen_kernel<<<grid, kScrThreads, smem_b, st>>>(P);
+        screen<<<grid, scr_threads, smem_b, st>>>(P);
         }
         KScope ks(&fbp_chunk_stats::ms_score, st);
         score_kernel<<<148 * 6, kScoreThreads, 0, st>>>(d, V, T, w.flag(), k0, w.best_lab(), w.best_idx(), P.gcand,

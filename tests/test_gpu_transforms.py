@@ -98,3 +98,13 @@ def test_window_lists_over_many_tiles(windows, recheck):
     assert si["n_samples_per_chan"] == W and abs(V.shape[1] - windows * W) <= W
     si["do_overlap_recheck"] = recheck
     _same_as_oracle(V, si, sm, W - 1)
+
+
+@pytest.mark.parametrize("seconds", [0.05, 4.0, 13.0])
+def test_few_and_many_windows(seconds):
+    """Passes of fewer and of more listed windows than the recheck's screen takes 512 threads
+    for, and of fewer and more queued runs than the recomputation has warps for."""
+    V, si, sm, _ = synth.make_recording(61, n_chans=5, fs=30000, duration_s=seconds, n_units=8,
+                                        rate_model=("uniform", 40.0, 90.0), overlap_frac=0.3)
+    si["get_adjusted_clips"] = True
+    _same_as_oracle(V, si, sm, si["n_samples_per_chan"] - 1)
