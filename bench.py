@@ -47,11 +47,7 @@ METRIC = "binary-pursuit Msample·ch/s, chosen vs plain FP32 on B200, ≥99.9% s
 # DRAM bytes per unit measured by ncu (dram__bytes_read.sum + dram__bytes_write.sum of one
 # launch of the 60 s slice of the linear16 workload, divided by the windows it processed)
 DRAM_PER_UNIT = {
-    "lik_tc_kernel": (17.0e3, "listed", "profiles/lik_tc_persist_kernel_linear16_60s.md: 105.9 MB / 6,240 windows"),
-    "partial_corr_kernel": (35.8e3, "flagged", "profiles/partial_corr_kernel_linear16_60s.md: 107.3 MB / 3,001 windows"),
-    "screen_kernel": (39.1e3, "flagged", "profiles/screen_kernel_linear16_60s.md: 117.3 MB / 3,001 windows"),
-    "argmax_kernel": (18.8, "listed", "profiles/residual_accept_compact_linear16_60s.md: argmax_lazy_kernel, "
-                      "0.45 MB / 23,808 windows"),
+    "lik_fft_kernel": (20.9e3, "listed", "profiles/lik_fft_kernel_linear16_60s.md: 497.5 MB / 23,763 windows"),
 }
 
 
@@ -337,7 +333,7 @@ def main():
                                          and np.array_equal(res_fast[1], res_plain[1])),
                  "stages_ms": {k: v for k, v in st_plain.items() if k.startswith("ms_")}}
 
-    hbm, tflops, peak_kind = load_peaks()
+    hbm, _, peak_kind = load_peaks()
     # per-kernel device time of one step (separate run with FBP_TIMING) and the
     # algorithmic work each kernel family does in that step
     S2 = 2 * S + 1
@@ -345,15 +341,19 @@ def main():
     # FP32 FMA issue peak of the SIMT pipes (148 SMs x 128 lanes x 2 flop) at the
     # median SM clock of the timed region (nominal max clock if no sample)
     fma_peak = 148 * 128 * 2 * (clocks.get("sm_mhz") or 1965.0) * 1e6 / 1e12
+    # correlations by 256-point transforms, two real signals a transform: of every channel,
+    # of the products with the templates' spectra on their non-zero channels, of every template
+    nz = float(np.count_nonzero(np.abs(T.reshape(M, C, W)).max(axis=2)))
+    transforms = (C + M) * 0.5 * 5 * 256 * 8 + nz * 129 * 8
     fam = {
-        "lik_tc_kernel": (st_stage["ms_lik_tc"], "tensor", 2.0 * M * C * W * W * listed,
-                          "2*M*C*W*W flop per listed window (nominal dense product); launched as "
-                          "lik_tc_persist_kernel up to 128 template columns, lik_tc_kernel above"),
-        "fixup_kernel": (st_stage["ms_fixup"], "fp32", 2.0 * C * W * 4 * st_stage["fixup_runs_queued"],
-                         "2*C*W flop per sample recomputed"),
-        "partial_corr_kernel": (st_stage["ms_partial_corr"], "fp32", 2.0 * st_stage["pc_macs"],
-                                "2 flop per multiply-add done (device counter)"),
-        "screen_kernel": (st_stage["ms_screen"], "latency", None, "L2-latency-bound table scan"),
+        "lik_fft_kernel": (st_stage["ms_lik_tc"], "fp32", transforms * listed * W / (257.0 - W),
+                           "transforms of all channels and templates and products on non-zero channels "
+                           "per 257 - W samples of the listed windows"),
+        "fixup_kernel": (st_stage["ms_fixup"], "fp32", 2.0 * nz / M * W * 4 * st_stage["fixup_runs_queued"],
+                         "2 flop per tap of the non-zero channels and sample of the queued runs"),
+        "window_corr_kernel": (st_stage["ms_partial_corr"], "fp32", transforms * flagged,
+                               "transforms and products as above per flagged window"),
+        "screen_kernel": (st_stage["ms_screen"], "latency", None, "L2 latency and instruction issue: chunks of 32 items"),
         "score_kernel": (st_stage["ms_score"], "latency", None, "one sequential C*W chain per candidate"),
         "argmax_kernel": (st_stage["ms_argmax"], "hbm", 24.0 * listed,
                           "3 window keys (8 B) per listed window (argmax_lazy_kernel)"),
@@ -368,18 +368,13 @@ def main():
             ach = work / (ms * 1e-3) / 1e9
             kernels[name] = {"ms": ms, "bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
                              "frac": ach / hbm, "work": what}
-        elif bound == "tensor":
-            ach = work / (ms * 1e-3) / 1e12
-            kernels[name] = {"ms": ms, "bound": "tensor", "achieved": ach, "peak": tflops, "unit": "TFLOP/s",
-                             "frac": ach / tflops, "work": what}
         else:
             ach = work / (ms * 1e-3) / 1e12
             kernels[name] = {"ms": ms, "bound": "fp32-simt", "achieved": ach, "peak": fma_peak,
                              "unit": "TFLOP/s", "frac": ach / fma_peak, "work": what,
                              "peak_kind": "nominal FP32 FMA issue rate at the sampled clock"}
-    # the roofline line reports the dominant kernel among those bound by the tensor pipe
-    # or by HBM; the FP32-pipe and latency-bound kernels are in `kernels`
-    dom = max((k for k in kernels if kernels[k]["bound"] in ("tensor", "hbm")), key=lambda k: kernels[k]["ms"])
+    # the roofline line reports the slowest kernel with a rate; latency-bound ones are in `kernels`
+    dom = max((k for k in kernels if "achieved" in kernels[k]), key=lambda k: kernels[k]["ms"])
     roof = dict(kernels[dom])
     # DRAM bytes (read + write) per launch: ncu's per-unit figure from the captures in
     # profiles/ (60 s slice of this workload) times the units of an average launch here
@@ -391,9 +386,10 @@ def main():
         traffic_detail = {"bytes_per_unit": per_unit[0], "unit": per_unit[1] + " window",
                           "launches_per_step": st_stage["passes"], "source": per_unit[2]}
     slowest = max(kernels, key=lambda k: kernels[k]["ms"])
-    roof.update({"kernel": dom, "traffic": traffic, "traffic_detail": traffic_detail, "peak_kind": peak_kind,
-                 "note": ("peak = measured dense bf16 burst (the kernel computes in TF32, whose nominal rate is half)"
-                          if roof["bound"] == "tensor" else "peak = measured HBM copy bandwidth"),
+    roof.update({"kernel": dom, "traffic": traffic, "traffic_detail": traffic_detail,
+                 "peak_kind": roof.get("peak_kind", peak_kind),
+                 "note": ("peak = measured HBM copy bandwidth" if roof["bound"] == "hbm" else
+                          "peak = nominal FP32 FMA issue rate; a transform's additions are half its flop"),
                  "slowest_kernel": slowest})
     launches = int(st_fast["launches"]) * args.steps
 

@@ -111,7 +111,7 @@ struct Layout {
     // tensor-core likelihood (mode 1)
     size_t off_vt_hi, off_tt_hi, off_tpad, off_fix, off_tnorm, off_tchm;
     uint64_t Cp, Mp, n_fix_cap, vq_rows;
-    // lazy exactness of the tensor-core likelihood: per-window maximum keys and
+    // lazy exactness of the fast likelihood: per-window maximum keys and
     // positive flags, and per (window, template) "row holds estimates" flags
     size_t off_wkey, off_wpos, off_wflag;
     // transforms (corr_fft.cu): template spectra, channel lists and counts, twiddles
@@ -157,7 +157,7 @@ struct Work {
     unsigned long long* tiles() const { return reinterpret_cast<unsigned long long*>(base + lay->off_status + 256); }
 };
 
-// Where the tensor-core likelihood left estimates (lazy exactness): readers of
+// Where the fast likelihood left estimates (lazy exactness): readers of
 // a positive likelihood value recompute it exactly when its window row is flagged.
 struct LazyRef {
     const uint8_t* wflag;      // [nw][M] flags, or null: L is exact wherever read

@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kOvThreads) overlap_plain_kernel(
 // parse_overlap_recheck_indices (binary_pursuit.cl:657-815), one thread per
 // flagged window, from the winner key.
 // ---------------------------------------------------------------------------
-// L[t][s], made exact where the tensor-core likelihood may have left an estimate
+// L[t][s], made exact where the fast likelihood may have left an estimate
 // (a positive value in a flagged window row; the window's voltage is unchanged
 // since it was computed, so the current voltage gives the exact value).  Called
 // by a whole warp with the same (t, s) on every lane.

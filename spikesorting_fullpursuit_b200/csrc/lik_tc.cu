@@ -16,6 +16,9 @@
 // pre-arranged as Tq[j][Cp/8][2][Np][4] and streamed per (tap, channel pair)
 // through a ring of shared-memory stages.
 //
+// The pursuit takes these kernels where the transforms of corr_fft.cu do not apply and
+// where the caller sets their launch shapes; the stand-alone fbp_likelihood always.
+//
 // Exactness.  The pursuit reads a likelihood either for its sign or, when it is
 // positive, for its value.  The epilogue bounds |estimate - reference float
 // result| rigorously (TF32 operand truncation, FP32 accumulation, the

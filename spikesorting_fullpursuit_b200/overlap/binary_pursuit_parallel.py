@@ -26,7 +26,7 @@ Differences, all documented:
 * The reference's pass loop has no limit (binary_pursuit_parallel.py:907);
   here a chunk that still adds spikes after ``max_passes`` passes raises
   FbpError (status FBP_E_PASSES) instead of running on.
-* Keyword-only extras: ``mode`` ("fast": tensor-core likelihood and screened
+* Keyword-only extras: ``mode`` ("fast": likelihood by transforms and screened
   overlap recheck, both exact; "plain": scalar FP32 kernels), ``device``,
   ``work_group_size`` (the reference's kernel work-group size, 256, whose
   execution order the results follow), ``max_passes``,
