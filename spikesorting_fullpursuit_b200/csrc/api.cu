@@ -468,10 +468,22 @@ extern "C" int fbp_copy_rows(void* dst, size_t dst_pitch, const void* src, size_
     if (!dst || !src) return fail(FBP_E_ARG, "null pointer argument");
     if (rows > 1 && (dst_pitch < width || src_pitch < width)) return fail(FBP_E_ARG, "rows overlap");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (rows == 1 || (dst_pitch == width && src_pitch == width))
+    if (rows == 1 || (dst_pitch == width && src_pitch == width)) {
         FBP_CUDA(cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyHostToDevice, st));
-    else
+        return FBP_OK;
+    }
+    // one 2-D copy, whose pitches are limited (2^31 - 1 bytes: rows of 2^29 samples exceed
+    // it), else a copy per row
+    int dev = 0, most = 0;
+    FBP_CUDA(cudaGetDevice(&dev));
+    FBP_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxPitch, dev));
+    if (dst_pitch <= (size_t)most && src_pitch <= (size_t)most) {
         FBP_CUDA(cudaMemcpy2DAsync(dst, dst_pitch, src, src_pitch, width, rows, cudaMemcpyHostToDevice, st));
+        return FBP_OK;
+    }
+    for (uint32_t r = 0; r < rows; ++r)
+        FBP_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + r * dst_pitch, static_cast<const char*>(src) + r * src_pitch,
+                                 width, cudaMemcpyHostToDevice, st));
     return FBP_OK;
 }
 
