@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(MAXT, MINB) window_corr_kernel(
     const uint32_t S = d.S, W = d.W, M = d.M, S2 = 2 * S + 1;
     const uint32_t Sw = S < W - 1 ? S : W - 1;   // shifts beyond meet no sample
     for (uint32_t i = threadIdx.x; i < kFft; i += blockDim.x) tw[i] = F.tw[i];
-    const uint32_t nflag = status->n_flag;
+    const uint32_t nflag = flagged_windows(status);
     const uint32_t live = nflag > k0 ? min(kc, nflag - k0) : 0u;
     unsigned long long macs = 0;
     for (uint32_t u = blockIdx.x; 2 * u < live; u += gridDim.x) {

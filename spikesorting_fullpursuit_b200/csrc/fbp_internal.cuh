@@ -99,6 +99,13 @@ struct DevStatus {
 };
 static_assert(sizeof(DevStatus) <= 256, "the allocation-free residual keeps 256 bytes for it");
 
+#ifdef __CUDACC__
+// Lengths of the pass's lists as later kernels read them: none once a kernel has set the
+// error word, since a list whose compaction failed has entries that nobody wrote.
+__device__ __forceinline__ uint32_t flagged_windows(const DevStatus* s) { return s->error ? 0u : s->n_flag; }
+__device__ __forceinline__ uint32_t accepted_spikes(const DevStatus* s) { return s->error ? 0u : s->n_spikes; }
+#endif
+
 // ---------------------------------------------------------------------------
 // Workspace layout (all offsets 256-byte aligned)
 // ---------------------------------------------------------------------------

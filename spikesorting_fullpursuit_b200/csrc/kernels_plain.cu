@@ -13,6 +13,7 @@
 //   * spike output: window-list order; residual: list order for overlaps.
 #include <cub/cub.cuh>
 
+#include "compact.cuh"
 #include "lik_common.cuh"
 
 namespace fbp {
@@ -228,78 +229,6 @@ __global__ void argmax_lazy_kernel(ArgmaxLazy a, uint32_t nlist)
         argmax_window(a, a.list[k]);
 }
 
-// ---------------------------------------------------------------------------
-// Ordered stream compaction in one launch.  A functor supplies visit(i), which
-// evaluates item i once and says whether it is kept, and emit(i, pos).  Tiles are
-// numbered by a ticket, so that every tile before one that runs has started; a tile
-// publishes its count, then adds up the counts of the tiles before it, back to the
-// nearest one that knows its own position (decoupled look-back).  The wait for a
-// predecessor is limited; past it the error word is set and nothing is emitted.
-// (Count, scan and scatter as three launches took three times the launch gaps, and
-// evaluated every item twice.)
-// ---------------------------------------------------------------------------
-constexpr int kCompactThreads = 256;
-constexpr int kCompactItems = 4;
-constexpr int kCompactTile = kCompactThreads * kCompactItems;
-constexpr uint32_t kLookbackPolls = 1u << 22;
-
-constexpr unsigned long long kTileCount = 1ull << 62, kTilePlace = 2ull << 62, kTileFlags = 3ull << 62;
-
-template <class F>
-__global__ void __launch_bounds__(kCompactThreads) compact_kernel(F f, uint32_t n, unsigned long long* state,
-                                                                  uint32_t* ticket, uint32_t* total, DevStatus* status)
-{
-    typedef cub::BlockScan<uint32_t, kCompactThreads> S;
-    __shared__ typename S::TempStorage tmp;
-    __shared__ uint32_t s_tile, s_base;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const uint64_t first = (uint64_t)tile * kCompactTile + threadIdx.x * kCompactItems;
-    bool keep[kCompactItems];
-    uint32_t cnt = 0;
-#pragma unroll
-    for (int r = 0; r < kCompactItems; ++r) {
-        keep[r] = first + r < n && f.visit((uint32_t)(first + r));
-        cnt += keep[r];
-    }
-    uint32_t ex, all;
-    S(tmp).ExclusiveSum(cnt, ex, all);
-    if (threadIdx.x < 32) {
-        const uint32_t lane = threadIdx.x;
-        volatile unsigned long long* st = state;
-        if (lane == 0) st[tile] = (tile ? kTileCount : kTilePlace) | all;
-        uint32_t base = 0;
-        bool failed = false;
-        for (int64_t at = (int64_t)tile - 1; at >= 0 && !failed;) {   // 32 predecessors at a time, nearest on lane 0
-            const int64_t mine = at - lane;
-            unsigned long long v = kTilePlace;
-            if (mine >= 0) {
-                uint32_t polls = 0;
-                while (((v = st[mine]) & kTileFlags) == 0ull && ++polls < kLookbackPolls) {}
-            }
-            failed = __any_sync(0xffffffffu, (v & kTileFlags) == 0ull);
-            const uint32_t place = __ballot_sync(0xffffffffu, (v & kTileFlags) == kTilePlace);
-            const uint32_t upto = place ? (uint32_t)__ffs(place) - 1u : 31u;   // counts before it, and its position
-            base += __reduce_add_sync(0xffffffffu, lane <= upto ? (uint32_t)v : 0u);
-            if (place) break;
-            at -= 32;
-        }
-        if (lane == 0) {
-            if (failed) atomicOr(&status->error, 0x400u);
-            st[tile] = kTilePlace | (base + all);
-            s_base = failed ? 0xFFFFFFFFu : base;
-            if ((uint64_t)(tile + 1) * kCompactTile >= n) *total = base + all;
-        }
-    }
-    __syncthreads();
-    if (s_base == 0xFFFFFFFFu) return;
-    uint32_t pos = s_base + ex;
-#pragma unroll
-    for (int r = 0; r < kCompactItems; ++r)
-        if (keep[r]) f.emit((uint32_t)(first + r), pos++);
-}
-
 // `which` (0..2): the call's look-back state of the pass (zeroed at its start)
 template <class F>
 int compact(F f, const Work& w, int which, uint32_t n, uint32_t* total, cudaStream_t st)
@@ -308,7 +237,7 @@ int compact(F f, const Work& w, int which, uint32_t n, uint32_t* total, cudaStre
     if (nb == 0) return FBP_OK;   // the pass starts with zero totals
     count_launch();
     compact_kernel<F><<<nb, kCompactThreads, 0, st>>>(f, n, w.tiles() + (size_t)which * w.lay->nblk,
-                                                      &w.status()->ticket[which], total, w.status());
+                                                      &w.status()->ticket[which], total, w.status(), kLookbackPolls);
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -417,7 +346,7 @@ __global__ void __launch_bounds__(kOvThreads) overlap_plain_kernel(
     const uint64_t slots = nloc * d.WG;
     uint32_t lbits = 0;
     while ((1u << lbits) < d.WG) ++lbits;
-    const uint32_t nflag = status->n_flag;
+    const uint32_t nflag = flagged_windows(status);
     const uint64_t ntask = (uint64_t)nflag * d.M;
     unsigned long long my_items = 0;
     for (uint64_t task = blockIdx.x; task < ntask; task += gridDim.x) {
@@ -562,7 +491,7 @@ __global__ void __launch_bounds__(kParseThreads) parse_kernel(
 {
     __shared__ float buf[kParseThreads / 32][32 * kExactBlocks];
     __shared__ float value[kParseThreads / 32];
-    const uint32_t nflag = status->n_flag;
+    const uint32_t nflag = flagged_windows(status);
     const uint64_t S2 = 2ull * d.S + 1;
     const uint64_t items = S2 * S2 * d.M;
     uint32_t lbits = 0;
@@ -665,7 +594,7 @@ __global__ void reassign_kernel(Dims d, const uint32_t* __restrict__ flag, DevSt
                                 uint32_t* best_lab, uint8_t* check, const uint32_t* __restrict__ ov_idx,
                                 const uint32_t* __restrict__ ov_lab)
 {
-    const uint32_t nflag = status->n_flag;
+    const uint32_t nflag = flagged_windows(status);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nflag; k += gridDim.x * blockDim.x) {
         const uint32_t id = flag[k];
         if (!orech[id]) { orech_fin[id] = 0; continue; }
@@ -685,7 +614,7 @@ __global__ void reassign_commit_kernel(Dims d, const uint32_t* __restrict__ flag
                                        uint32_t* best_lab, uint8_t* check, const uint32_t* __restrict__ ov_idx,
                                        const uint32_t* __restrict__ ov_lab)
 {
-    const uint32_t nflag = status->n_flag;
+    const uint32_t nflag = flagged_windows(status);
     if (!(status->chain_overflow & 1u)) {
         for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nflag; k += gridDim.x * blockDim.x) {
             const uint32_t id = flag[k];

@@ -1215,7 +1215,7 @@ __global__ void lazy_fix_kernel(Dims d, const float* __restrict__ V, const float
                                 const DevStatus* status, const uint8_t* __restrict__ check, float* L,
                                 uint8_t* wflag, const float* __restrict__ tnorm)
 {
-    const uint32_t n = status->n_spikes;
+    const uint32_t n = accepted_spikes(status);
     for (uint32_t k = blockIdx.x; k < n; k += gridDim.x) {
         const uint64_t s = pidx[k];
         const uint64_t lo = s + 1 >= d.W ? s + 1 - d.W : 0;

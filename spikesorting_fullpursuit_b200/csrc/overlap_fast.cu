@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kPcMaxWarps * 32, 2) partial_corr_kernel(
         Ts[e] = (g0 + q < M && j < W) ? T[((uint64_t)perm[g0 + q] * d.C + chans[ci]) * W + j] : 0.f;
     }
     for (uint32_t e = threadIdx.x; e < kPcWin * gm.WS; e += blockDim.x) Vs[e] = 0.f;
-    const uint32_t nflag = status->n_flag;
+    const uint32_t nflag = flagged_windows(status);
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const uint32_t wi = lane >> 2, bs = lane & 3;
     unsigned long long macs = 0;   // multiply-adds this thread does
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM) screen_kernel(const __grid_co
     const uint64_t slots = ((items - 1) / d.WG + 1) * d.WG;
     uint32_t lbits = 0;
     while ((1u << lbits) < d.WG) ++lbits;
-    const uint32_t nflag = P.status->n_flag;
+    const uint32_t nflag = flagged_windows(P.status);
     const uint32_t live = nflag > P.k0 ? min(P.kc, nflag - P.k0) : 0u;
     uint32_t evals = 0;   // chunks evaluated by this warp
     for (uint32_t jo = blockIdx.x; jo < live; jo += gridDim.x) {
@@ -943,7 +943,7 @@ __global__ void __launch_bounds__(1024) label_order_kernel(Dims d, const uint32_
                                                            uint32_t kc, uint32_t* order)
 {
     extern __shared__ uint32_t hist[];   // [M + 1]
-    const uint32_t nflag = status->n_flag, M = d.M;
+    const uint32_t nflag = flagged_windows(status), M = d.M;
     for (uint32_t i = threadIdx.x; i <= M; i += blockDim.x) hist[i] = 0;
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < kc; j += blockDim.x) {
@@ -1005,7 +1005,7 @@ __global__ void __launch_bounds__(kScoreThreads) score_kernel(
         const unsigned long long code = e < have ? gcand[i0 + e] : ~0ull;
         const uint32_t kk = (uint32_t)(code >> 32);
         const uint32_t t = (uint32_t)(code >> 20) & 0xFFFu, a = (uint32_t)(code >> 10) & 0x3FFu, b = (uint32_t)code & 0x3FFu;
-        const bool ok = code != ~0ull && (uint64_t)k0 + kk < status->n_flag && t < M && a < S2 && b < S2;
+        const bool ok = code != ~0ull && (uint64_t)k0 + kk < flagged_windows(status) && t < M && a < S2 && b < S2;
         uint32_t f = 0, p = 0;
         unsigned long long left = 0ull;   // channels still to sum (C <= 64)
         if (ok) {
