@@ -472,8 +472,9 @@ extern "C" int fbp_copy_rows(void* dst, size_t dst_pitch, const void* src, size_
         FBP_CUDA(cudaMemcpyAsync(dst, src, width * rows, cudaMemcpyHostToDevice, st));
         return FBP_OK;
     }
-    // one 2-D copy, whose pitches are limited (2^31 - 1 bytes: rows of 2^29 samples exceed
-    // it), else a copy per row
+    // One 2-D copy up to the device's pitch limit, else a copy per row: CUDA documents an
+    // error past it (2^31 - 1 bytes, rows of 2^29 samples).  Driver 580.159 copies such
+    // rows all the same; nothing here relies on that.
     int dev = 0, most = 0;
     FBP_CUDA(cudaGetDevice(&dev));
     FBP_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxPitch, dev));

@@ -1,5 +1,5 @@
 """Voltage uploads whose rows lie far apart: recordings of hours, where a row's pitch
-exceeds what a 2-D copy takes (2^31 - 1 bytes)."""
+exceeds the documented limit of a 2-D copy (2^31 - 1 bytes)."""
 import ctypes
 
 import numpy as np
