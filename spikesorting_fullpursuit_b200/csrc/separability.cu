@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "fbp_internal.cuh"
+#include "pair_rule.cuh"
 #include "pairwise.cuh"
 
 namespace fbp {
@@ -273,28 +274,7 @@ __global__ void __launch_bounds__(kPairThreads) pair_separability_kernel(
 // pair: 200 templates of 64 x 76 samples 10.5 -> 3.7 ms (4.7 ms with 32 pairs a CTA
 // and the covariances not fetched ahead).  Bounded by latency: where n1 is zero on a
 // channel, only the few pairs whose n2 is not have work between two barriers.
-constexpr uint32_t kTilePairs = 64;
 constexpr int kTileThreads = 8 * kTilePairs;
-
-struct PairTileSmem {
-    size_t k, d, t1, nz, total;   // byte offsets; total
-};
-
-// zeros before and after template n1: the lags, in whole groups of 16, and a channel's
-// last 32 lanes reach past it (by at most max_shift + 15 + 31, max_shift < W)
-__host__ __device__ inline uint32_t pair_pad(uint32_t W) { return W + 48; }
-
-template <int NJ>
-__host__ __device__ inline PairTileSmem pair_tile_smem(uint32_t C, uint32_t W)
-{
-    PairTileSmem s;
-    s.k = 0;                                                     // [2][W][8 NJ] covariances, zero columns past W
-    s.d = s.k + (size_t)2 * W * 8 * NJ * 8;                      // [64][8 NJ] aligned differences
-    s.t1 = s.d + (size_t)kTilePairs * 8 * NJ * 8;                // [C W] template n1 between zeros
-    s.nz = s.t1 + ((size_t)C * W + 2 * pair_pad(W)) * 8;          // [65][C] non-zero channels of the n2, then of n1
-    s.total = s.nz + (size_t)(kTilePairs + 1) * C;
-    return s;
-}
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src)
 {
@@ -310,7 +290,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) pair_tile_kernel(
 {
     extern __shared__ __align__(16) unsigned char sraw[];
     __shared__ int s_shift[kTilePairs];
-    const PairTileSmem lay = pair_tile_smem<NJ>(C, W);
+    const PairTileSmem lay = pair_tile_smem(NJ, C, W);
     double* K = reinterpret_cast<double*>(sraw + lay.k);
     double* D = reinterpret_cast<double*>(sraw + lay.d);
     double* t1 = reinterpret_cast<double*>(sraw + lay.t1) + pair_pad(W);   // t1[-pad, C W + pad)
@@ -527,13 +507,12 @@ extern "C" int fbp_pair_separability(const void* templates, int templates_f64, c
     auto run = [&](auto* t) -> int {
         using F = std::remove_const_t<std::remove_pointer_t<decltype(t)>>;
         const F* energy = static_cast<const F*>(template_ss);
-        // tiles of pairs up to 128 samples per channel where a template and a covariance fit
-        // shared memory together; any other size a CTA per pair
         const dim3 tiles((n_templates + kTilePairs - 1) / kTilePairs, n_templates);
+        const uint32_t nj = pair_tile_columns(n_templates, n_chans, template_len, (size_t)optin);
 #define FBP_PAIR(NJ)                                                                                              \
-    if (template_len <= 8 * NJ && pair_tile_smem<NJ>(n_chans, template_len).total + 2048 <= (size_t)optin) {      \
+    if (nj == NJ) {                                                                                               \
         FBP_CUDA(allow_max_dyn_smem(pair_tile_kernel<F, NJ>));                                                     \
-        pair_tile_kernel<F, NJ><<<tiles, kTileThreads, pair_tile_smem<NJ>(n_chans, template_len).total, st>>>(    \
+        pair_tile_kernel<F, NJ><<<tiles, kTileThreads, pair_tile_smem(NJ, n_chans, template_len).total, st>>>(    \
             t, energy, channel_cov, variance, threshold, n_templates, n_chans, template_len, max_shift,           \
             pair_matrix, noise_contamination, noise_misses, optimal_shift);                                        \
         return FBP_OK;                                                                                             \
