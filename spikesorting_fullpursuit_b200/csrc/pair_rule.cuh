@@ -52,12 +52,14 @@ __host__ __device__ inline bool pair_tiles_pay(uint32_t M, uint32_t C, uint32_t 
     return M >= (C >= 8 && C <= 24 && W >= 70 ? 48u : kTilePairs);
 }
 
-// Columns a lane of the tile kernel takes (W <= 8 of them), or 0: a CTA per pair, also
-// where a template and two covariances do not fit `most` bytes of shared memory.
+// Columns a lane of the tile kernel takes (8 lanes hold a row: W <= 8 of them), or 0: a CTA
+// per pair, also where a template and two covariances do not fit `most` bytes of shared
+// memory.  In 227 KB they fit up to 225 channels at W = 64, 133 at 76, 120 at 80, 18 at 96,
+// 7 at 101 and 1 at 104, and from 105 on (14 columns or more) never.
 __host__ __device__ inline uint32_t pair_tile_columns(uint32_t M, uint32_t C, uint32_t W, size_t most)
 {
     if (!pair_tiles_pay(M, C, W)) return 0;
-    const uint32_t cols[] = {8, 10, 13, 16};
+    const uint32_t cols[] = {8, 10, 13};
     for (uint32_t nj : cols)
         if (W <= 8 * nj && pair_tile_smem(nj, C, W).total + 2048 <= most) return nj;
     return 0;

@@ -265,7 +265,8 @@ __global__ void __launch_bounds__(kPairThreads) pair_separability_kernel(
                     shift_out);
 }
 
-// The same for a tile of 64 units n2 against one n1 per CTA, W <= 8 NJ: a channel's
+// The same for a tile of 64 units n2 against one n1 per CTA, W <= 8 NJ, for the sets of
+// pair_rule.cuh (many units, windows up to about 100 samples): a channel's
 // covariance is read into shared memory once for the tile, the next one's while it is
 // used, and channels where neither template is non-zero are skipped, as are the zero
 // channels of T2 in the cross-correlation.  8 lanes take a pair's quadratic form: NJ
@@ -520,7 +521,6 @@ extern "C" int fbp_pair_separability(const void* templates, int templates_f64, c
         FBP_PAIR(8)
         FBP_PAIR(10)
         FBP_PAIR(13)
-        FBP_PAIR(16)
 #undef FBP_PAIR
         FBP_CUDA(allow_max_dyn_smem(pair_separability_kernel<F>));
         pair_separability_kernel<F><<<grid, kPairThreads, smem, st>>>(

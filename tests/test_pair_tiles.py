@@ -1,6 +1,7 @@
 """Pairwise separability: which of its two kernels a call takes (csrc/pair_rule.cuh, on the
 CPU), and the tile kernel at its edges against the oracle (on the GPU)."""
 import os
+import re
 import subprocess
 
 import numpy as np
@@ -47,6 +48,18 @@ def test_rule_over_its_ranges(rule):
         for C in (4, 16, 33, 64):
             for W in (20, 61, 76, 101):
                 assert rule(M, C, W) == 0
+
+
+@pytest.mark.parametrize("W,channels", [(64, 225), (76, 133), (80, 120), (96, 18), (101, 7), (104, 1)])
+def test_largest_templates_of_the_tiles(rule, W, channels):
+    assert rule(200, channels, W) > 0
+    assert rule(200, channels + 1, W) == 0
+
+
+def test_every_instance_of_the_tile_kernel_is_reached(rule):
+    with open(os.path.join(build.CSRC, "separability.cu")) as fp:
+        built = {int(n) for n in re.findall(r"^ +FBP_PAIR\((\d+)\)", fp.read(), re.M)}
+    assert built == {rule(200, 1, W) for W in range(1, 130)} - {0}
 
 
 # Tolerances: a tail probability's relative error is about z times the error of its argument
