@@ -10,7 +10,7 @@ with the real templates -- and keeps the fastest: first the likelihood, by its
 stage's device time within whole pursuits of the slice (the pass-by-pass window
 lists of a real pursuit), then the partial-correlation group, by whole pursuits.  Results are cached in a JSON file
 (``FBP_TUNE_CACHE``, else ~/.cache/spikesorting_fullpursuit_b200/tuning.json)
-keyed by (channels, templates, window, shift, device name), so each shape is
+keyed by (candidate set, channels, templates, window, shift, device name), so each shape is
 measured once.  Launch shapes change speed only: every candidate gives the
 same spikes.
 """
@@ -27,6 +27,11 @@ from . import _native
 
 _LOCK = threading.Lock()
 FIELDS = ("lik_tiles", "lik_group", "lik_stages", "pc_group", "lik_epi")
+# Part of every cache key, raised when the candidates or the meaning of their values change.
+# 2: all zeros, the library's choice, is a candidate.  Entries without a version come from
+# tensor-core shapes alone, which now ask for the slower kernels instead of the transforms
+# (twice to four times the time of a pursuit).
+CANDIDATES = 2
 
 
 def cache_path():
@@ -57,7 +62,12 @@ def _store(key, value):
 
 
 def key_of(C, M, W, S, device_name):
-    return "C%d-M%d-W%d-S%d-%s" % (C, M, W, S, device_name)
+    return "v%d-C%d-M%d-W%d-S%d-%s" % (CANDIDATES, C, M, W, S, device_name)
+
+
+def cached(C, M, W, S, device_name):
+    """The stored launch shapes for these sizes, or None."""
+    return _load().get(key_of(C, M, W, S, device_name))
 
 
 def apply(tuning):
@@ -114,9 +124,9 @@ def tune(voltage, templates, bias, theta, W, S, overlap=True, sample_s=None, sam
         "cuda", torch.cuda.current_device() if device is None else int(device))
     C = int(voltage.shape[0])
     M = int(np.asarray(templates).shape[0])
-    key = key_of(C, M, W, S, torch.cuda.get_device_name(dev))
+    name = torch.cuda.get_device_name(dev)
     if use_cache:
-        hit = _load().get(key)
+        hit = cached(C, M, W, S, name)
         if hit is not None:
             return hit
     n = int(voltage.shape[1])
@@ -169,5 +179,5 @@ def tune(voltage, templates, bias, theta, W, S, overlap=True, sample_s=None, sam
     finally:
         apply(None)
     if use_cache:
-        _store(key, best)
+        _store(key_of(C, M, W, S, name), best)
     return best
