@@ -172,7 +172,8 @@ class _Uploader:
         Returns (events, upto, flags, finish): events[k] completes once samples
         [0, upto[k]) of every channel are in ``dst``; flags[k] turns 1 once events[k]
         is recorded (the library waits for it before waiting on the event);
-        ``finish()`` joins the thread and re-raises its error, if any."""
+        ``finish()`` joins the thread and re-raises its error, if any.  After an error the
+        rest of ``dst`` is zero: a pursuit already behind the upload finds nothing there."""
         torch = self.torch
         C, N = host.shape
         slab = min(self.SLAB_FLOATS, max(self.LEAST_FLOATS, -(-C * N // 16)))
@@ -214,9 +215,13 @@ class _Uploader:
                             filled.append(pool.submit(fill, k + n_slabs))
             except BaseException as e:   # the library must not wait for ranges that never come
                 failure.append(e)
-                with torch.cuda.device(self.dev):
-                    for k in range(len(ranges)):
-                        if not flags[k]:
+                with torch.cuda.device(self.dev), torch.cuda.stream(stream):
+                    k0 = int(np.count_nonzero(flags))   # flags turn 1 in order
+                    try:
+                        if k0 < len(ranges):
+                            dst[:, ranges[k0][0]:].zero_()
+                    finally:
+                        for k in range(k0, len(ranges)):
                             events[k].record(stream)
                             flags[k] = 1
             finally:   # the slabs go back to torch's pinned cache: their last copies must be done

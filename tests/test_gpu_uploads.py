@@ -1,5 +1,6 @@
-"""Voltage uploads whose rows lie far apart: recordings of hours, where a row's pitch
-exceeds the documented limit of a 2-D copy (2^31 - 1 bytes)."""
+"""Voltage uploads whose rows lie far apart -- recordings of hours, where a row's pitch
+exceeds the documented limit of a 2-D copy (2^31 - 1 bytes) -- and uploads whose source
+fails on the way."""
 import ctypes
 
 import numpy as np
@@ -59,5 +60,40 @@ def test_upload_of_a_part_of_a_long_recording(direct, monkeypatch):
     try:
         up.upload(host, dst)
         assert np.array_equal(dst.cpu().numpy(), host)
+    finally:
+        up.close()
+
+
+class _FailingSource:
+    """A voltage that cannot be read from sample `at` on, as a truncated file."""
+
+    def __init__(self, data, at):
+        self.data, self.at, self.shape = data, at, data.shape
+
+    def __getitem__(self, key):
+        if key[1].stop > self.at:
+            raise OSError("read error")
+        return self.data[key]
+
+
+@pytest.mark.parametrize("at", [0, 499, 500, 30000, 30010])
+def test_a_failed_upload_leaves_zeros(at, monkeypatch):
+    """A pursuit that runs behind the upload must not see memory that was never written."""
+    monkeypatch.setattr(bpp._Uploader, "SLAB_FLOATS", 1000)
+    monkeypatch.setattr(bpp._Uploader, "LEAST_FLOATS", 1000)
+    n, span = 30011, 500   # two channels: 500 samples a range
+    data = np.random.default_rng(3).standard_normal((2, n))
+    dev = torch.device("cuda", torch.cuda.current_device())
+    dst = torch.full((2, n), float("nan"), dtype=torch.float32, device=dev)
+    up = bpp._Uploader(torch, dev)
+    try:
+        _, upto, flags, finish = up.start_staged(_FailingSource(data, at), dst)
+        with pytest.raises(OSError, match="read error"):
+            finish()
+        assert np.all(flags == 1) and upto[-1] == n
+        done = at // span * span
+        got = dst.cpu().numpy()
+        assert np.array_equal(got[:, :done], data[:, :done].astype(np.float32))
+        assert np.all(got[:, done:] == 0)
     finally:
         up.close()
