@@ -67,11 +67,12 @@ __global__ void __launch_bounds__(128) energy_table_kernel(Dims d, const float* 
     }
 }
 
-// largest value of the warp's lanes, NaN ignored
+// largest value of the warp's lanes, NaN ignored; volatile, since all lanes have to reach it
+// and some uses are by one lane only: plain asm may be moved into such a branch
 __device__ __forceinline__ float warp_max(float v)
 {
     float r;
-    asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
 }
 
