@@ -304,7 +304,7 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
     }
     // per-window state starts at zero (binary_pursuit_parallel.py:595-654)
     FBP_CUDA(cudaMemsetAsync(w.base + lay.off_best_lik, 0, lay.off_list - lay.off_best_lik, st));
-    const size_t all_bytes = 256 + 3 * lay.nblk * 8, pass_bytes = all_bytes - offsetof(DevStatus, n_flag);
+    const size_t all_bytes = 256 + 3 * lay.nblk * 8, pass_bytes = all_bytes - offsetof(DevStatus, error);
     FBP_CUDA(cudaMemsetAsync(w.status(), 0, all_bytes, st));
     FBP_TRY(launch_iota(w.list(), d.nw, st));
     if (!plain) FBP_TRY(launch_template_info(d, w, templates, st));
@@ -327,7 +327,7 @@ int pursue_chunk(const fbp_dims* dims, uint32_t flags, float* voltage, const flo
         S.passes = pass;
         S.listed += nlist;
         if (pass > 1)   // the pass's counters and look-back states
-            FBP_CUDA(cudaMemsetAsync(&w.status()->n_flag, 0, pass_bytes, st));
+            FBP_CUDA(cudaMemsetAsync(&w.status()->error, 0, pass_bytes, st));
         tm.start(timing, st, &S.ms_likelihood);
         if (pass == 1 && ready.n > 0) {
             // first pass behind the upload: of each arrived range, the spans (or

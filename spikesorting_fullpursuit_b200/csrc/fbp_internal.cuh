@@ -79,13 +79,13 @@ class KScope {
 // ---------------------------------------------------------------------------
 struct DevStatus {
     // of the whole call
-    uint32_t error;         // nonzero: a kernel detected an inconsistent state
     uint32_t n_pair_exact;  // overlap items recomputed exactly
+    uint32_t n_fix_local;   // runs recomputed inside the likelihood kernel
     unsigned long long pair_items;  // items evaluated by the overlap recheck
     unsigned long long pc_macs;     // multiply-adds done by the partial correlations
-    uint32_t n_fix_local;   // runs recomputed inside the likelihood kernel
-    uint32_t reserved;
+    uint32_t reserved[2];
     // of one pass: from here to the end, and the look-back states behind it, zeroed at its start
+    uint32_t error;         // nonzero: a kernel detected an inconsistent state (read with n_flag)
     uint32_t n_flag;        // windows flagged for the overlap recheck this pass
     uint32_t n_spikes;      // spikes accepted this pass
     uint32_t n_next;        // windows listed for the next pass
@@ -94,6 +94,7 @@ struct DevStatus {
     uint32_t n_units;       // spans of listed windows the transform likelihood takes this pass
     uint32_t cand_count;    // candidates appended to the exact-scoring list (per batch)
     uint32_t ticket[3];     // next tile of the pass's three compactions
+    uint32_t reserved2;
     uint32_t n_conf;        // spikes of a residual overlapping an earlier one
     uint32_t residual_done; // CTAs of a residual that are done
 };
@@ -102,7 +103,15 @@ static_assert(sizeof(DevStatus) <= 256, "the allocation-free residual keeps 256 
 #ifdef __CUDACC__
 // Lengths of the pass's lists as later kernels read them: none once a kernel has set the
 // error word, since a list whose compaction failed has entries that nobody wrote.
-__device__ __forceinline__ uint32_t flagged_windows(const DevStatus* s) { return s->error ? 0u : s->n_flag; }
+// (One load: two in turn made a pass of a small pursuit 2 us longer.)
+static_assert(offsetof(DevStatus, error) % 16 == 0 && offsetof(DevStatus, n_flag) == offsetof(DevStatus, error) + 4 &&
+                  offsetof(DevStatus, n_conf) % 8 == 0,
+              "read as a pair; zeroed from aligned addresses on");
+__device__ __forceinline__ uint32_t flagged_windows(const DevStatus* s)
+{
+    const uint2 v = *reinterpret_cast<const uint2*>(&s->error);
+    return v.x ? 0u : v.y;
+}
 __device__ __forceinline__ uint32_t accepted_spikes(const DevStatus* s) { return s->error ? 0u : s->n_spikes; }
 #endif
 
