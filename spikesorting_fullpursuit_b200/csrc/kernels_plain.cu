@@ -1123,7 +1123,10 @@ int launch_residual(const Dims& d, const Work& w, float* V, const float* T, cons
     const uint32_t back = 4 + 2 * ((d.S + d.W - 1) / d.W);
     FBP_CUDA(cudaMemsetAsync(&w.status()->n_conf, 0, 8, st));   // and residual_done
     count_launch();
-    const uint32_t grid = std::min<uint32_t>(n, 148u * kResPerSm), batch = std::min((n + grid - 1) / grid, kResBatch);
+    // spikes a CTA: enough for a row a warp, and for the spikes to fit the resident CTAs
+    const uint32_t rows = std::max(1u, kResThreads / 32 / d.C), most = 148u * kResPerSm;
+    const uint32_t batch = std::min(std::max(rows, (n + most - 1) / most), kResBatch);
+    const uint32_t grid = std::min((n + batch - 1) / batch, most);
     residual_kernel<<<grid, kResThreads, 0, st>>>(d, V, T, idx, lab, win, n, batch, back, w.pconf(), w.status(), out_idx,
                                                   out_lab);
     FBP_CUDA(cudaGetLastError());
