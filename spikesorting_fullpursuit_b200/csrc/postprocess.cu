@@ -58,58 +58,10 @@ __device__ __forceinline__ float sq_diff(const float* __restrict__ a, const floa
     return __fmul_rn(d, d);
 }
 
-// Sum of (a - b)^2 over [0, n <= 128) in numpy's order by 8 lanes (lane j of the group:
-// the values j, j + 8, ... of the whole eights, combined as a tree, then the rest in
-// order); n < 8: in order.  The sum on every lane of the group.
-__device__ __forceinline__ float piece_sum(const float* __restrict__ a, const float* __restrict__ b, uint32_t n,
-                                           uint32_t j, uint32_t mask)
-{
-    const uint32_t n8 = n - n % 8;
-    float r = 0.f;
-    if (n8) {
-        r = sq_diff(a, b, j);
-#pragma unroll 8
-        for (uint32_t i = 8 + j; i < n8; i += 8) r = __fadd_rn(r, sq_diff(a, b, i));
-        r = __fadd_rn(r, __shfl_xor_sync(mask, r, 1));
-        r = __fadd_rn(r, __shfl_xor_sync(mask, r, 2));
-        r = __fadd_rn(r, __shfl_xor_sync(mask, r, 4));
-    }
-    for (uint32_t i = n8; i < n; ++i) r = __fadd_rn(r, sq_diff(a, b, i));
-    return r;
-}
-
-// The pieces of clips of one length and the additions of their sums, in order: step k
-// adds the sum at right[k] to the one at left[k] (made on the host, passed by value).
-constexpr uint32_t kPieces = 256;   // pieces of 64 values at least: clips of 16,384 samples fit
-struct PieceList {
-    uint16_t count;
-    uint16_t first[kPieces + 1];
-    uint8_t left[kPieces], right[kPieces];
-};
-
-PieceList make_pieces(uint32_t len)
-{
-    PieceList l{};
-    uint32_t adds = 0;
-    pairwise_sum<uint32_t>(   // a sum is the place of its leftmost piece
-        len,
-        [&](uint32_t at, uint32_t) {
-            l.first[l.count] = (uint16_t)at;
-            return (uint32_t)l.count++;
-        },
-        [&](uint32_t a, uint32_t b) {
-            l.left[adds] = (uint8_t)a;
-            l.right[adds++] = (uint8_t)b;
-            return a;
-        });
-    l.first[l.count] = (uint16_t)len;
-    return l;
-}
-
 // A warp per clip: its pieces by groups of 8 lanes, their sums added by one lane.
 // (A thread per clip read its clip alone, 4 bytes of every 32-byte sector at a time:
-// 188 us for a unit of 300 clips x 1616 samples, now 20.)  Longer clips than
-// kPieces allows by a thread each.
+// 188 us for a unit of 300 clips x 1616 samples, now 20.)  Longer clips than kPieces
+// allows by a thread each.
 constexpr int kSseThreads = 128;
 
 __global__ void __launch_bounds__(kSseThreads) sse_kernel(const float* __restrict__ clips,
@@ -118,11 +70,14 @@ __global__ void __launch_bounds__(kSseThreads) sse_kernel(const float* __restric
 {
     __shared__ float sums[kSseThreads / 32][kPieces];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 3, j = lane & 7u;
-    const uint32_t count = P.count, nwarps = gridDim.x * (kSseThreads / 32);
-    for (uint32_t i = blockIdx.x * (kSseThreads / 32) + warp; i < n; i += nwarps) {
+    const uint32_t count = P.count, nwarps = gridDim.x * (kSseThreads / 32), group = 0xFFu << (8 * g);
+    const uint32_t w = blockIdx.x * (kSseThreads / 32) + warp;
+    for (uint32_t i = w; i < n; i += nwarps) {
         const float* c = clips + (uint64_t)i * len;
         for (uint32_t k = g; k < count; k += 4) {
-            const float s = piece_sum(c + P.first[k], tmpl + P.first[k], P.first[k + 1] - P.first[k], j, 0xFFu << (8 * g));
+            const float *x = c + P.first[k], *y = tmpl + P.first[k];
+            const float s = piece_sum<float>([=](uint32_t q) { return sq_diff(x, y, q); },
+                                             P.first[k + 1] - P.first[k], j, group);
             if (j == 0) sums[warp][k] = s;
         }
         __syncwarp();
@@ -132,6 +87,22 @@ __global__ void __launch_bounds__(kSseThreads) sse_kernel(const float* __restric
             sse[i] = sums[warp][0];
         }
         __syncwarp();
+    }
+}
+
+// Clips of one piece (at most 128 values): a clip by 8 lanes.  (A warp each left 24 lanes
+// idle: duplicate removal of 200,000 clips of 76 samples 395 us, by a thread each 370, now
+// 340; of 20 samples 380, 334 and 336.)
+__global__ void __launch_bounds__(kSseThreads) sse_short_kernel(const float* __restrict__ clips,
+                                                                const float* __restrict__ tmpl, uint32_t n,
+                                                                uint32_t len, float* sse)
+{
+    const uint32_t j = threadIdx.x & 7u, group = 0xFFu << (threadIdx.x & 24u);
+    const uint64_t step = (uint64_t)gridDim.x * (kSseThreads / 8);
+    for (uint64_t i = (uint64_t)blockIdx.x * (kSseThreads / 8) + (threadIdx.x >> 3); i < n; i += step) {
+        const float* c = clips + i * len;
+        const float s = piece_sum<float>([=](uint32_t x) { return sq_diff(c, tmpl, x); }, len, j, group);
+        if (j == 0) sse[i] = s;
     }
 }
 
@@ -268,7 +239,10 @@ extern "C" int fbp_bp_duplicates(const int64_t* event_indices, const float* clip
     float* sse = reinterpret_cast<float*>(ws);
     uint8_t* start = ws + ((size_t)n * 4 + 255) / 256 * 256;
     const uint32_t g = (n + 255) / 256 < 148u * 16 ? (n + 255) / 256 : 148u * 16;
-    if (clip_len <= 64 * kPieces)   // a piece has at least 64 values once there are two
+    if (clip_len <= kPairwisePiece)
+        sse_short_kernel<<<std::min<uint32_t>((n + kSseThreads / 8 - 1) / (kSseThreads / 8), 148u * 16), kSseThreads, 0,
+                           st>>>(clips, unit_template, n, clip_len, sse);
+    else if (clip_len <= 64 * kPieces)   // a piece has at least 64 values once there are two
         sse_kernel<<<std::min<uint32_t>((n + kSseThreads / 32 - 1) / (kSseThreads / 32), 148u * 16), kSseThreads, 0, st>>>(
             clips, unit_template, n, clip_len, make_pieces(clip_len), sse);
     else
