@@ -80,7 +80,8 @@ template <class F>
 __global__ void __launch_bounds__(kSepThreads) separability_kernel(const F* __restrict__ T,
                                                                    const double* __restrict__ cov, uint32_t C,
                                                                    uint32_t W, double sigma_noise, double sigma_ci,
-                                                                   int apply_bp_threshold, SepOut out, bool staged)
+                                                                   int apply_bp_threshold, SepOut out,
+                                                                   const __grid_constant__ PieceList P)
 {
     typedef cub::BlockReduce<double, kSepThreads> RD;
     __shared__ typename RD::TempStorage rd;
@@ -88,24 +89,28 @@ __global__ void __launch_bounds__(kSepThreads) separability_kernel(const F* __re
     __shared__ uint32_t s_idx;
     const uint32_t n = blockIdx.x;
     const F* t = T + (uint64_t)n * C * W;
-    // staged where it fits: the energy's summation is one thread's chain (273 -> 252 us
-    // for 200 templates of 64 x 76 samples)
-    extern __shared__ __align__(16) unsigned char sep_smem[];
-    if (staged) {
-        F* ts = reinterpret_cast<F*>(sep_smem);
-        for (uint32_t e = threadIdx.x; e < C * W; e += blockDim.x) ts[e] = t[e];
-        __syncthreads();
-        t = ts;
-    }
-    // FP64 quadratic forms: thread-strided partial sums over (c, i), each a row
-    // of Cov_c against the template, then one block reduction
+    // FP64 quadratic forms: thread-strided partial sums over (c, i), each a row of Cov_c
+    // against the template, eight elements in flight (200 templates of 64 x 76: 288 -> 213 us),
+    // then one block reduction
     double part = 0.0;
     for (uint64_t e = threadIdx.x; e < (uint64_t)C * W; e += blockDim.x) {
         const uint32_t c = (uint32_t)(e / W), i = (uint32_t)(e % W);
         const double* row = cov + ((uint64_t)c * W + i) * W;
         const F* tc = t + (uint64_t)c * W;
         double r = 0.0;
-        for (uint32_t j = 0; j < W; ++j) r = fma(row[j], (double)tc[j], r);
+        uint32_t j = 0;
+        for (; j + 8 <= W; j += 8) {
+            double k[8];
+            F x[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                k[q] = __ldg(row + j + q);
+                x[q] = tc[j + q];
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) r = fma(k[q], (double)x[q], r);
+        }
+        for (; j < W; ++j) r = fma(row[j], (double)tc[j], r);
         part = fma((double)tc[i], r, part);
     }
     const double var = RD(rd).Sum(part);
@@ -122,8 +127,23 @@ __global__ void __launch_bounds__(kSepThreads) separability_kernel(const F* __re
     __syncthreads();
     if (bi != 0xFFFFFFFFu && bb == s_bits) atomicMin(&s_idx, bi);
     __syncthreads();
+    // the energy in numpy's order: a warp's groups of 8 lanes take the pieces (by one thread,
+    // C W / 8 additions one after the other, 40 templates of 16 x 101 float64 samples took
+    // 72 us, so 57)
+    __shared__ F sums[kPieces];
+    if (P.count > 0 && threadIdx.x < 32) {
+        const uint32_t g = threadIdx.x >> 3, j = threadIdx.x & 7u;
+        for (uint32_t k = g; k < P.count; k += 4) {
+            const F* x = t + P.first[k];
+            const F s = piece_sum<F>([=](uint32_t i) { return sq(x, i); }, P.first[k + 1] - P.first[k], j, 0xFFu << (8 * g));
+            if (j == 0) sums[k] = s;
+        }
+        __syncwarp();
+        if (threadIdx.x == 0)
+            for (uint32_t k = 0; k + 1 < P.count; ++k) sums[P.left[k]] = add_rn(sums[P.left[k]], sums[P.right[k]]);
+    }
     if (threadIdx.x == 0) {
-        const F ss = pairwise_sq_sum(t, C * W);
+        const F ss = P.count > 0 ? sums[0] : pairwise_sq_sum(t, C * W);
         const F expectation = (F)0.5 * ss;   // exact (a power of two)
         const double sd = sqrt(var);
         const double lower_ci = (double)expectation - sigma_ci * sd;
@@ -463,19 +483,16 @@ extern "C" int fbp_separability(const void* templates, int templates_f64, const 
         return fail(FBP_E_ARG, "null pointer argument");
     SepOut out{template_ss, variance, lower_ci, threshold, contamination, peak_channel};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const size_t bytes = (size_t)n_chans * template_len * (templates_f64 ? 8 : 4);
-    const bool staged = bytes <= 160 * 1024;
-    const size_t smem = staged ? bytes : 0;
+    // longer templates than the list of pieces holds: one thread sums
+    const PieceList pieces = n_chans * template_len <= 64 * kPieces ? make_pieces(n_chans * template_len) : PieceList{};
     if (templates_f64) {
-        FBP_CUDA(allow_max_dyn_smem(separability_kernel<double>));
-        separability_kernel<double><<<n_templates, kSepThreads, smem, st>>>(
+        separability_kernel<double><<<n_templates, kSepThreads, 0, st>>>(
             static_cast<const double*>(templates), channel_cov, n_chans, template_len, sigma_bp_noise, sigma_bp_ci,
-            apply_bp_threshold, out, staged);
+            apply_bp_threshold, out, pieces);
     } else {
-        FBP_CUDA(allow_max_dyn_smem(separability_kernel<float>));
-        separability_kernel<float><<<n_templates, kSepThreads, smem, st>>>(
+        separability_kernel<float><<<n_templates, kSepThreads, 0, st>>>(
             static_cast<const float*>(templates), channel_cov, n_chans, template_len, sigma_bp_noise, sigma_bp_ci,
-            apply_bp_threshold, out, staged);
+            apply_bp_threshold, out, pieces);
     }
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
