@@ -25,6 +25,8 @@
 // for the sum of v^2) and 521 us for the gradient at 16 channels x 60 s, 19200 spikes of
 // 101 samples, with the FP64 pipe 6-9% and the L2's atomics 9% busy; as here: 137 us and
 // 242 us.
+#include <algorithm>
+
 #include <cub/cub.cuh>
 
 #include "fbp_internal.cuh"
@@ -142,17 +144,22 @@ __device__ __forceinline__ void residual_row(const AdjArgs& A, uint32_t c, int64
     }
 }
 
-// E: a warp takes 128 samples of all channels at a time.
-__global__ void __launch_bounds__(kAdjThreads) adjoint_loss_kernel(AdjArgs A, double* loss)
+// E: a warp takes 128 samples of every slices-th channel at a time: of all channels where
+// the recording has samples enough to fill the SMs, else of a share of them (64 channels x
+// 100,000 samples, 300 spikes, 89 us by all channels a warp, now 24).
+template <bool SLICED>
+__global__ void __launch_bounds__(kAdjThreads) adjoint_loss_kernel(AdjArgs A, uint32_t slices, double* loss)
 {
     typedef cub::BlockReduce<double, kAdjThreads> R;
     __shared__ typename R::TempStorage tmp;
     __shared__ AdjSpike box[kAdjWarps][32];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t nseg = ((uint64_t)A.N + kAdjSpan - 1) / kAdjSpan;
+    if (!SLICED) slices = 1;
     double acc = 0.0;
-    for (uint64_t g = (uint64_t)blockIdx.x * kAdjWarps + warp; g < nseg; g += (uint64_t)gridDim.x * kAdjWarps) {
-        const int64_t x0 = (int64_t)(g * kAdjSpan);
+    for (uint64_t g = (uint64_t)blockIdx.x * kAdjWarps + warp; g < nseg * slices; g += (uint64_t)gridDim.x * kAdjWarps) {
+        const uint64_t seg = SLICED ? g / slices : g;
+        const int64_t x0 = (int64_t)(seg * kAdjSpan);
         const uint32_t k0 = first_onset(A, x0 - (int64_t)A.W);
         uint32_t k1 = k0;   // past the last spike with onset <= x0 + 128
         for (;;) {
@@ -167,7 +174,7 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_loss_kernel(AdjArgs A, do
             if (lane < k1 - k0) box[warp][lane] = adj_spike(A, k0 + lane, x0);
             __syncwarp();
         }
-        for (uint32_t c = 0; c < A.C; ++c) {
+        for (uint32_t c = (uint32_t)(g - seg * slices); c < A.C; c += slices) {
             double r[kAdjCols];
             residual_row(A, c, x0, k0, k1, box[warp], one, r);
 #pragma unroll
@@ -178,13 +185,16 @@ __global__ void __launch_bounds__(kAdjThreads) adjoint_loss_kernel(AdjArgs A, do
     if (threadIdx.x == 0) atomicAdd(loss, s);
 }
 
-// A CTA takes a spike, a warp every fourth channel; a row's W + 2 columns are taken 126
-// at a time, with one more on either side for the shifted residual.
-__global__ void __launch_bounds__(kAdjThreads, 8) adjoint_grad_kernel(AdjArgs A, double scale, double* gT, float* g_amp,
-                                                                  float* g_tau)
+// A CTA takes a spike, a warp every WARPS-th channel; a row's W + 2 columns are taken 126
+// at a time, with one more on either side for the shifted residual.  Four warps, or 16
+// where few spikes of many channels leave the SMs idle (300 spikes of 64 channels x 20
+// samples 45 us, now 29; 60 of 128 x 76 85 us, now 33).
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 32 / WARPS) adjoint_grad_kernel(AdjArgs A, double scale, double* gT,
+                                                                              float* g_amp, float* g_tau)
 {
-    __shared__ AdjSpike box[kAdjWarps][32];
-    __shared__ double part[2][kAdjWarps];
+    __shared__ AdjSpike box[WARPS][32];
+    __shared__ double part[2][WARPS];
     const int W = (int)A.W, TL = W + 2;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (uint32_t k = blockIdx.x; k < A.n; k += gridDim.x) {
@@ -214,7 +224,7 @@ __global__ void __launch_bounds__(kAdjThreads, 8) adjoint_grad_kernel(AdjArgs A,
                     if (lane < k1 - k0) box[warp][lane] = adj_spike(A, k0 + lane, x0);
                     __syncwarp();
                 }
-                for (uint32_t c = warp; c < A.C; c += kAdjWarps) {
+                for (uint32_t c = warp; c < A.C; c += WARPS) {
                     double r[kAdjCols];
                     residual_row(A, c, x0, k0, k1, box[warp], one, r);
                     const int j0 = q0 + (int)lane - 2;   // template sample of column `lane`
@@ -274,7 +284,7 @@ __global__ void __launch_bounds__(kAdjThreads, 8) adjoint_grad_kernel(AdjArgs A,
         __syncthreads();
         if (threadIdx.x == 0) {
             double sa = 0.0, st = 0.0;
-            for (int w = 0; w < kAdjWarps; ++w) {
+            for (int w = 0; w < WARPS; ++w) {
                 sa += part[0][w];
                 st += part[1][w];
             }
@@ -338,8 +348,13 @@ extern "C" int fbp_adjoint_loss(const fbp_dims* dims, const float* voltage, cons
     const AdjArgs A = adj_args(dims, voltage, templates, spike_idx, spike_lab, amplitude, shift, n_spikes);
     FBP_CUDA(cudaMemsetAsync(loss, 0, sizeof(double), st));
     count_launch();
-    const uint64_t blocks = ((uint64_t)A.N + kAdjSpan * kAdjWarps - 1) / (kAdjSpan * kAdjWarps);
-    adjoint_loss_kernel<<<blocks < 148u * 16 ? (uint32_t)blocks : 148u * 16, kAdjThreads, 0, st>>>(A, loss);
+    const uint64_t nseg = ((uint64_t)A.N + kAdjSpan - 1) / kAdjSpan, most = 148ull * 16 * kAdjWarps;
+    const uint32_t slices = (uint32_t)std::min<uint64_t>(A.C, std::max<uint64_t>(1, most / nseg));
+    const uint32_t blocks = (uint32_t)((std::min<uint64_t>(nseg * slices, most) + kAdjWarps - 1) / kAdjWarps);
+    if (slices > 1)
+        adjoint_loss_kernel<true><<<blocks, kAdjThreads, 0, st>>>(A, slices, loss);
+    else
+        adjoint_loss_kernel<false><<<blocks, kAdjThreads, 0, st>>>(A, 1, loss);
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
@@ -360,8 +375,11 @@ extern "C" int fbp_adjoint_grad(const fbp_dims* dims, const float* voltage, cons
     FBP_CUDA(cudaMemsetAsync(grad_templates64, 0, nt * sizeof(double), st));
     if (n_spikes) {
         count_launch();
-        adjoint_grad_kernel<<<n_spikes < 148u * 16 ? n_spikes : 148u * 16, kAdjThreads, 0, st>>>(
-            A, scale, grad_templates64, grad_amplitude, grad_shift);
+        const uint32_t blocks = std::min(n_spikes, 148u * 16);
+        if (A.C > 8 && n_spikes <= 148u * 4)
+            adjoint_grad_kernel<16><<<blocks, 32 * 16, 0, st>>>(A, scale, grad_templates64, grad_amplitude, grad_shift);
+        else
+            adjoint_grad_kernel<4><<<blocks, 32 * 4, 0, st>>>(A, scale, grad_templates64, grad_amplitude, grad_shift);
     }
     count_launch();
     f64_to_f32_kernel<<<148 * 4, 256, 0, st>>>(grad_templates64, grad_templates, nt);
