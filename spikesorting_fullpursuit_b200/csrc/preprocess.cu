@@ -265,11 +265,12 @@ __global__ void __launch_bounds__(kRtThreads) robust_template_kernel(const float
 // rank order through shared memory.  16 channels x 101 samples x 10,000 rows: 7.5 ms
 // with the means summed by every output row's CTA, one scattered load at a time,
 // 1.9 ms with a pass of its own for them, 0.5 ms now.
-constexpr uint32_t kCovTile = 112, kCovRows = 16, kCovCluster = 8, kCovThreads = 256, kCovProbe = 32;
+constexpr uint32_t kCovTile = 112, kCovRows = 16, kCovCluster = 8, kCovThreads = 256, kCovProbe = 32,
+                   kCovFewRows = 64;
 constexpr uint32_t kCovLoads = kCovRows * kCovTile / kCovThreads;   // elements of a step a thread loads
 
 template <bool DIAG>
-__global__ void __cluster_dims__(kCovCluster, 1, 1) __launch_bounds__(kCovThreads, 1)
+__global__ void __launch_bounds__(kCovThreads, 1)
     covariance_kernel(const float* __restrict__ clips, const float* __restrict__ tmpls,
                       const uint32_t* __restrict__ unit_of, const int64_t* __restrict__ rows, uint32_t n_rows,
                       uint32_t len, uint32_t wc, double* cov)
@@ -284,27 +285,34 @@ __global__ void __cluster_dims__(kCovCluster, 1, 1) __launch_bounds__(kCovThread
     double* shift = sums + 2 * kCovTile;             // [2][kCovTile] s
     double* total = shift + 2 * kCovTile;            // [2][kCovTile] the cluster's sums
     __shared__ uint64_t s_clip[2][kCovRows], s_tmpl[2][kCovRows];   // row offsets of two steps
-    const uint32_t nt = (wc + kCovTile - 1) / kCovTile, c = blockIdx.z, rank = cluster.block_rank();
+    const uint32_t nt = (wc + kCovTile - 1) / kCovTile, c = blockIdx.z, rank = cluster.block_rank(),
+                   ctas = cluster.num_blocks();
     // tile pair: the diagonal launch numbers the tiles, the other one the ordered pairs
     const uint32_t it = DIAG ? blockIdx.y : blockIdx.y / (nt - 1);
     uint32_t jt = DIAG ? it : blockIdx.y % (nt - 1);
     if (!DIAG && jt >= it) ++jt;
     const uint32_t base[2] = {it * kCovTile, jt * kCovTile};
     const uint32_t cols[2] = {min(kCovTile, wc - base[0]), min(kCovTile, wc - base[1])};
-    const uint32_t share = (n_rows + kCovCluster - 1) / kCovCluster;
+    // whole steps a CTA; the last ones of a cluster have no rows if there are few
+    const uint32_t share = max((n_rows + ctas - 1) / ctas, kCovRows), parts = (n_rows + share - 1) / share;
     const uint32_t r0 = min(n_rows, rank * share), r1 = min(n_rows, r0 + share);
     const int64_t* mine = rows + (uint64_t)c * n_rows;
     // provisional means
     const uint32_t probe = min(n_rows, kCovProbe);
+    __shared__ uint64_t s_probe[2][kCovProbe];   // offsets of their clip and template
+    if (threadIdx.x < probe) {
+        const uint64_t row = (uint64_t)__ldg(mine + threadIdx.x);
+        s_probe[0][threadIdx.x] = row * len + (uint64_t)c * wc;
+        s_probe[1][threadIdx.x] = (uint64_t)__ldg(unit_of + row) * len + (uint64_t)c * wc;
+    }
+    __syncthreads();
     for (uint32_t k = threadIdx.x; k < kTiles * kCovTile; k += kCovThreads) {
         const uint32_t w = k / kCovTile, j = k - w * kCovTile;
         double s = 0.0;
         if (j < cols[w])
-#pragma unroll 8
-            for (uint32_t r = 0; r < probe; ++r) {
-                const uint64_t row = (uint64_t)__ldg(mine + r), at = (uint64_t)c * wc + base[w] + j;
-                s += (double)__fsub_rn(__ldg(clips + row * len + at), __ldg(tmpls + (uint64_t)__ldg(unit_of + row) * len + at));
-            }
+#pragma unroll 16
+            for (uint32_t r = 0; r < probe; ++r)
+                s += (double)__fsub_rn(__ldg(clips + s_probe[0][r] + base[w] + j), __ldg(tmpls + s_probe[1][r] + base[w] + j));
         shift[k] = s / (double)probe;
     }
     auto offsets = [&](uint32_t step) {   // row offsets of a step, by its first threads
@@ -371,21 +379,23 @@ __global__ void __cluster_dims__(kCovCluster, 1, 1) __launch_bounds__(kCovThread
         __syncthreads();
     }
     if (threadIdx.x < kTiles * kCovTile) sums[threadIdx.x] = sum;
+    if (steps > 0) {
 #pragma unroll
-    for (int a = 0; a < 7; ++a)
+        for (int a = 0; a < 7; ++a)
 #pragma unroll
-        for (int b = 0; b < 7; ++b)
-            if (!DIAG || b >= a) part[(ty + 16 * a) * kCovTile + tx + 16 * b] = acc[a][b];
+            for (int b = 0; b < 7; ++b)
+                if (!DIAG || b >= a) part[(ty + 16 * a) * kCovTile + tx + 16 * b] = acc[a][b];
+    }
     cluster.sync();
     for (uint32_t k = threadIdx.x; k < kTiles * kCovTile; k += kCovThreads) {
         double s = 0.0;
-        for (uint32_t b = 0; b < kCovCluster; ++b) s += cluster.map_shared_rank(sums, b)[k];
+        for (uint32_t b = 0; b < parts; ++b) s += cluster.map_shared_rank(sums, b)[k];
         total[k] = s;
     }
     __syncthreads();
     // this CTA's share of the tile, parts added in rank order
     const double inv = 1.0 / (double)n_rows;   // np.cov scales by 1 / fact
-    for (uint32_t e = rank * kCovThreads + threadIdx.x; e < cols[0] * cols[1]; e += kCovCluster * kCovThreads) {
+    for (uint32_t e = rank * kCovThreads + threadIdx.x; e < cols[0] * cols[1]; e += ctas * kCovThreads) {
         uint32_t i = e / cols[1], j = e - i * cols[1];
         const uint32_t oi = i, oj = j;
         if (DIAG && j < i) {   // the covariance is symmetric: only its upper 16-blocks are there
@@ -393,7 +403,7 @@ __global__ void __cluster_dims__(kCovCluster, 1, 1) __launch_bounds__(kCovThread
             j = oi;
         }
         double s = 0.0;
-        for (uint32_t b = 0; b < kCovCluster; ++b) s += cluster.map_shared_rank(part, b)[i * kCovTile + j];
+        for (uint32_t b = 0; b < parts; ++b) s += cluster.map_shared_rank(part, b)[i * kCovTile + j];
         s -= (total[i] * total[(DIAG ? 0 : kCovTile) + j]) * inv;   // the same for (j, i)
         cov[((uint64_t)c * wc + base[0] + oi) * wc + base[1] + oj] = s * inv;
     }
@@ -454,14 +464,27 @@ extern "C" int fbp_residual_covariance(const float* clips, const float* template
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t smem = (kCovTile * kCovTile + 2 * kCovRows * kCovTile + 6 * kCovTile) * sizeof(double);
     const uint32_t nt = (n_samples_per_chan + kCovTile - 1) / kCovTile;
-    FBP_CUDA(allow_max_dyn_smem(covariance_kernel<true>));
-    covariance_kernel<true><<<dim3(kCovCluster, nt, n_chans), kCovThreads, smem, st>>>(
-        clips, templates, unit_of, rows, n_rows, clip_len, n_samples_per_chan, cov);
-    if (nt > 1) {
-        FBP_CUDA(allow_max_dyn_smem(covariance_kernel<false>));
-        covariance_kernel<false><<<dim3(kCovCluster, nt * (nt - 1), n_chans), kCovThreads, smem, st>>>(
-            clips, templates, unit_of, rows, n_rows, clip_len, n_samples_per_chan, cov);
-    }
+    // few rows of many channels: a cluster a channel would be several waves of CTAs with a
+    // step or none each (256 channels x 61 samples x 50 rows 186 us, by a CTA a channel 38)
+    const uint32_t ctas = n_rows <= kCovFewRows && (uint64_t)n_chans * nt * kCovCluster > 148 ? 1 : kCovCluster;
+    auto launch = [&](auto kernel, uint32_t tiles) -> cudaError_t {
+        cudaError_t e = allow_max_dyn_smem(kernel);
+        if (e != cudaSuccess) return e;
+        cudaLaunchAttribute shape;
+        shape.id = cudaLaunchAttributeClusterDimension;
+        shape.val.clusterDim.x = ctas;
+        shape.val.clusterDim.y = shape.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ctas, tiles, n_chans);
+        cfg.blockDim = dim3(kCovThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = &shape;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, kernel, clips, templates, unit_of, rows, n_rows, clip_len, n_samples_per_chan, cov);
+    };
+    FBP_CUDA(launch(covariance_kernel<true>, nt));
+    if (nt > 1) FBP_CUDA(launch(covariance_kernel<false>, nt * (nt - 1)));
     FBP_CUDA(cudaGetLastError());
     return FBP_OK;
 }
